@@ -185,6 +185,38 @@ __device__ __forceinline__ void add_emission_grad(double *g, float v) {
   if ((threadIdx.x & 31) == 0 && v != 0.0f) atomicAdd(g, (double)v);
 }
 
+// Whether the ray (o, d) can hit an area light, and then a tmax that lies
+// behind every light it can hit.  A BSDF sample's ray counts only if its
+// closest hit is an area light, so one that misses all the lights' boxes is
+// never queued (its contribution is zero, as when it is traced), and the
+// others are traced no farther than the boxes reach.  The slabs are widened
+// by the traversal's own bound on their float error (make_slab_ray), NaN
+// operands are dropped by fmaxf / fminf, and tmax is pushed 1 % out so that
+// no light hit is near it.
+// What it saves is traversal, which bounds every frame: in a box lit by one
+// quad about nine BSDF rays in ten miss the light's box (256^2 x 4 samples,
+// 20,494 triangles: 616 -> 463 us; 16 views of 201,742 triangles, 8 samples:
+// 32.9 -> 20.2 ms).
+__device__ __forceinline__ bool lights_in_reach(const SceneDev &S, V3 o, V3 d, float &tmax) {
+  const float oo[3] = {o.x, o.y, o.z}, dd[3] = {d.x, d.y, d.z};
+  tmax = -1.0f;
+  for (int li = 0; li < S.n_area_lights; ++li) {
+    const AreaLight &L = S.area_lights[li];
+    float tn = 0.0f, tf = __int_as_float(0x7f800000);
+    for (int a = 0; a < 3; ++a) {
+      const float inv = 1.0f / dd[a];
+      const float w = 6.0f * 5.9604645e-8f * (S.scene_abs + fabsf(oo[a])) * fabsf(inv), off = -oo[a] * inv;
+      const bool neg = signbit(inv);
+      tn = fmaxf(tn, fmaf(neg ? L.hi[a] : L.lo[a], inv, off - w));
+      tf = fminf(tf, fmaf(neg ? L.lo[a] : L.hi[a], inv, off + w));
+    }
+    if (!(tn > tf)) tmax = fmaxf(tmax, tf);
+  }
+  if (!(tmax >= 0.0f)) return false;
+  tmax = 1.01f * tmax + 1e-4f * S.scene_abs;
+  return true;
+}
+
 // Per camera hit: emission, light samples, point lights and BSDF samples
 // (DirectLightingLTEIntegrator::_SurfaceRadiance with
 // DirectLightingIntegrator::ComputeDirectLighting).
@@ -363,12 +395,12 @@ __global__ void __launch_bounds__(128) k_shade(SceneDev S, ShadeArgs A, AdjointA
   for (int k = 0; k < nl; ++k) {
     bool want = false;
     V3 val = v3(0, 0, 0), dir = v3(0, 0, 0), dkd = v3(0, 0, 0);
-    float pdf = 0.0f, tmin = 0.0f;
+    float pdf = 0.0f, tmin = 0.0f, tmax = 0.0f;
     if (surface && S.n_area_lights > 0) {
       float uc, u0, u1;
       direct_sample(A, !SPEC && A.ld, seed, gid, true, k, uc, u0, u1);
       const V3 f = bsdf_sample(b, wo, uc, u0, u1, dir, pdf);
-      if (pdf > 0.0f && !black(f)) {
+      if (pdf > 0.0f && !black(f) && lights_in_reach(S, h.p, dir, tmax)) {
         val = f * (fabsf(dot(dir, shading_n)) / (pdf * nl));
         if (ADJ) {
           dkd = mul(dI, bsdf_eval_dkd(b, wo, dir)) * (fabsf(dot(dir, shading_n)) / (pdf * nl));
@@ -380,7 +412,7 @@ __global__ void __launch_bounds__(128) k_shade(SceneDev S, ShadeArgs A, AdjointA
     }
     const int q = queue_append(want, bcount);
     if (want) {
-      store_ray(brays, q, h.p, dir, tmin, __int_as_float(0x7f800000));
+      store_ray(brays, q, h.p, dir, tmin, tmax);
       btarget[q] = ADJ ? h.g : (int)(SPEC ? tslot : slot0 + 1 + nl + S.n_point_lights + k);
       if (ADJ) store_rgb(J.b_dkd, q, dkd);
       if (SPEC) val = mul(val, wt);
