@@ -26,14 +26,13 @@ int traversal_stack_capacity(int max_depth);
 // of the reference's GetNextMinT); a triangle whose t cannot be told apart
 // from tmin in float is then skipped (it lies on the ray's own plane
 // crossing) instead of being decided in double.
+// work: a device int of the caller's, not used by any launch that may run at
+// the same time; it is zeroed on `stream` and the warps take groups of rays
+// from it as they finish.
 cudaError_t launch_traversal(bool closest, int stack_cap, const void *nodes, const void *tris, const void *rays,
                              int64_t n, const int *n_dev, float scene_abs, const int32_t *out_index, void *out,
-                             unsigned *status, cudaStream_t stream, int ctas_per_sm = 0, int *work = nullptr,
+                             unsigned *status, cudaStream_t stream, int ctas_per_sm, int *work,
                              bool surface = false);
-// work (may be null): a device int of the caller's, not used by any launch
-// that may run at the same time; it is zeroed on `stream` and the warps
-// then take groups of 32 rays from it as they finish (no idle tail).  Null:
-// each warp traces a fixed share of the rays.
 cudaError_t prepare_traversal(int stack_cap);
 // Resident CTAs per SM of the closest-hit kernel at this capacity.
 int traversal_max_ctas_per_sm(int stack_cap);

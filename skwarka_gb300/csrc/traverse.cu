@@ -23,7 +23,7 @@
 // intrinsics, no fused multiply-add).  Such hits are flagged
 // SKW_HIT_FP64_DECIDED.
 //
-// Layout: nodes are 32-byte DevNode records read as two 16-byte loads; each
+// Layout: nodes are 32-byte DevNode records, one 32-byte load each; a
 // triangle slot is 3 x float4 (v0|prim, v1|tri, v2|slot); rays are 2 x float4.
 // The traversal stack holds 12-byte entries (node words 6-7 and the widened
 // entry distance): the first SKW_TRAV_SCAP (8) of each thread in shared
@@ -43,23 +43,28 @@
 namespace skw {
 namespace {
 
-constexpr float kWiden = 8.0f * 5.9604645e-8f;  // 8 * 2^-24: slab interval widening
 // Forward error bound of the float triangle test: with u = 2^-24, the edge
 // and offset vectors carry <= u relative error, the cross products <= 4u of
 // their magnitude sums, and det, n1, n2, nt <= 8u of the matching
 // magnitude dot products (first order); 10u leaves room for the second-order
-// terms and for the bounds being evaluated in float.
-constexpr float kTriErr = 10.0f * 5.9604645e-8f;
+// terms and for the bounds being evaluated in float.  A double ray rounded
+// to float (d by u relative, o by u |o|) moves the cross product with d by
+// another u of its magnitude sum and the offset o - v0 by u (|o| + |o - v0|)
+// instead of u |o - v0|: with |o - v0| + |o| in the magnitude sums 12u covers
+// every term (9u to first order).
+constexpr float kTriErr = 10.0f * 5.9604645e-8f, kTriErrD = 12.0f * 5.9604645e-8f;
 constexpr double kDblEps = 2.220446049250313e-16;
 
 // Launch shape: threads per block and the minimum resident blocks per SM
-// that bounds the register budget (set by measurement; overridable at
-// build time for sweeps).
+// that bounds the register budget.  Six blocks (80 registers) leave the node
+// step without spills: measured on 4,194,304 closest hits over 1.1M triangles
+// with 10 / 8 / 7 / 6 / 5 / 4 blocks per SM: 4.00 / 3.85 / 3.82 / 3.69 / 3.77
+// / 4.42 ms, on 1,000 rays: 98 / 88 / 79 / 77 / 73 / 77 us.
 #ifndef SKW_TRAV_BLOCK
 #define SKW_TRAV_BLOCK 128
 #endif
 #ifndef SKW_TRAV_MINB
-#define SKW_TRAV_MINB 10
+#define SKW_TRAV_MINB 6
 #endif
 
 enum : int { kMiss = 0, kHit = 1, kAmbiguous = 2 };
@@ -71,16 +76,6 @@ struct RayF {
 // Rays and results stream through once: with SKW_TRAV_STREAMING they are
 // loaded and stored with the evict-first policy so that they do not push the
 // tree out of L2.
-// Measured slower (shared-memory latency on every triangle test outweighs
-// the registers it frees): off by default.
-#ifndef SKW_TRAV_RAYSMEM
-#define SKW_TRAV_RAYSMEM 0
-#endif
-// Preferred shared-memory carveout in percent (cudaFuncAttribute
-// PreferredSharedMemoryCarveout); negative leaves the driver's choice.
-#ifndef SKW_TRAV_CARVEOUT
-#define SKW_TRAV_CARVEOUT -1
-#endif
 #ifndef SKW_TRAV_STREAMING
 #define SKW_TRAV_STREAMING 1
 #endif
@@ -101,7 +96,9 @@ __device__ __forceinline__ RayF load_ray(const float4 *__restrict__ rays, int64_
 // Float triangle test with a forward error bound.  Returns kMiss when the
 // reference's double test certainly rejects (barycentrics or t < tmin),
 // kHit when its barycentric tests and t >= tmin certainly pass (t and a bound
-// et on |t - t_exact| are returned), else kAmbiguous.
+// et on |t - t_exact| are returned), else kAmbiguous.  ROUNDED: r is a double
+// ray rounded to float (tmin down), and the bounds cover that rounding.
+template <bool ROUNDED>
 __device__ __forceinline__ int tri_test32(const RayF &r, float3 v0, float3 v1, float3 v2, float &t, float &et) {
   t = __int_as_float(0x7fffffff);  // NaN until computed
   et = 0.0f;
@@ -122,14 +119,16 @@ __device__ __forceinline__ int tri_test32(const RayF &r, float3 v0, float3 v1, f
   const float adx = fabsf(r.dx), ady = fabsf(r.dy), adz = fabsf(r.dz);
   const float a2x = fabsf(e2x), a2y = fabsf(e2y), a2z = fabsf(e2z);
   const float a1x = fabsf(e1x), a1y = fabsf(e1y), a1z = fabsf(e1z);
-  const float aox = fabsf(ddx), aoy = fabsf(ddy), aoz = fabsf(ddz);
+  const float aox = ROUNDED ? fabsf(ddx) + fabsf(r.ox) : fabsf(ddx), aoy = ROUNDED ? fabsf(ddy) + fabsf(r.oy) : fabsf(ddy),
+              aoz = ROUNDED ? fabsf(ddz) + fabsf(r.oz) : fabsf(ddz);
+  constexpr float kErr = ROUNDED ? kTriErrD : kTriErr;
   const float A1x = ady * a2z + adz * a2y, A1y = adz * a2x + adx * a2z, A1z = adx * a2y + ady * a2x;
   const float A2x = aoy * a1z + aoz * a1y, A2y = aoz * a1x + aox * a1z, A2z = aox * a1y + aoy * a1x;
   const float D = fabsf(det);
-  const float edet = kTriErr * (a1x * A1x + a1y * A1y + a1z * A1z) + 1e-15f * D;
-  const float en1 = kTriErr * (aox * A1x + aoy * A1y + aoz * A1z) + 1e-15f * D;
-  const float en2 = kTriErr * (adx * A2x + ady * A2y + adz * A2z) + 1e-15f * D;
-  const float ent = kTriErr * (a2x * A2x + a2y * A2y + a2z * A2z);
+  const float edet = kErr * (a1x * A1x + a1y * A1y + a1z * A1z) + 1e-15f * D;
+  const float en1 = kErr * (aox * A1x + aoy * A1y + aoz * A1z) + 1e-15f * D;
+  const float en2 = kErr * (adx * A2x + ady * A2y + adz * A2z) + 1e-15f * D;
+  const float ent = kErr * (a2x * A2x + a2y * A2y + a2z * A2z);
   if (!(D > 2.0f * edet)) return kAmbiguous;  // nearly parallel (or degenerate)
   const float sgn = det < 0.0f ? -1.0f : 1.0f;
   const float N1 = sgn * n1, N2 = sgn * n2, NT = sgn * nt;
@@ -140,7 +139,9 @@ __device__ __forceinline__ int tri_test32(const RayF &r, float3 v0, float3 v1, f
   t = NT * inv;
   et = (ent + fabsf(t) * edet) * inv * 1.0001f + fabsf(t) * 2.4e-7f + 1e-30f;
   if (t + et < r.tmin) return kMiss;
-  if (N1 - en1 > 0.0f && N2 - en2 > 0.0f && (N1 + N2) + (en1 + en2) < D - edet && t - et >= r.tmin) return kHit;
+  if (N1 - en1 > 0.0f && N2 - en2 > 0.0f && (N1 + N2) + (en1 + en2) < D - edet &&
+      (ROUNDED ? t - et > r.tmin : t - et >= r.tmin))  // rounded: above tmin rounded down is above tmin
+    return kHit;
   return kAmbiguous;
 }
 
@@ -190,12 +191,6 @@ __device__ __forceinline__ bool tri_test64v(double ox, double oy, double oz, dou
     }
   }
   return false;
-}
-
-// The same test for a float ray widened exactly to double.
-__device__ __forceinline__ bool tri_test64(const RayF &r, float3 v0f, float3 v1f, float3 v2f, double tmin, double tmax,
-                                        double &t_out) {
-  return tri_test64v(r.ox, r.oy, r.oz, r.dx, r.dy, r.dz, v0f, v1f, v2f, tmin, tmax, t_out);
 }
 
 __device__ __forceinline__ void load_tri(const float4 *__restrict__ tris, uint32_t slot, float3 &v0, float3 &v1,
@@ -261,37 +256,14 @@ __device__ __forceinline__ SlabRay make_slab_ray(const RayF &r, float scene_abs,
 // entry distance max(tnear_x, tnear_y, tnear_z, tmin), all that a later
 // re-test against a smaller tmax needs.  fmaxf/fminf drop NaN operands
 // (0 * inf slabs), as the reference's comparisons are all false on NaN.
-#ifndef SKW_TRAV_MAX3
-#define SKW_TRAV_MAX3 0
-#endif
-#if SKW_TRAV_MAX3
-// Three-input max / min (sm_100+): a NaN operand is dropped, as by fmaxf /
-// fminf.
-__device__ __forceinline__ float max3f(float a, float b, float c) {
-  float d;
-  asm("max.f32 %0, %1, %2, %3;" : "=f"(d) : "f"(a), "f"(b), "f"(c));
-  return d;
-}
-__device__ __forceinline__ float min3f(float a, float b, float c) {
-  float d;
-  asm("min.f32 %0, %1, %2, %3;" : "=f"(d) : "f"(a), "f"(b), "f"(c));
-  return d;
-}
-#endif
-
 __device__ __forceinline__ bool node_visit(const float4 na, const float4 nb, const SlabRay &s, float tcull,
                                            float &lo) {
   const bool sx = s.bits & 8u, sy = s.bits & 16u, sz = s.bits & 32u;
   const float tn0 = fmaf(sx ? na.w : na.x, s.ix, s.nx), tf0 = fmaf(sx ? na.x : na.w, s.ix, s.fx);
   const float tn1 = fmaf(sy ? nb.x : na.y, s.iy, s.ny), tf1 = fmaf(sy ? na.y : nb.x, s.iy, s.fy);
   const float tn2 = fmaf(sz ? nb.y : na.z, s.iz, s.nz), tf2 = fmaf(sz ? na.z : nb.y, s.iz, s.fz);
-#if SKW_TRAV_MAX3
-  lo = max3f(tn0, tn1, fmaxf(tn2, s.tmin));
-  const float hi = min3f(tf0, tf1, fminf(tf2, tcull));
-#else
   lo = fmaxf(fmaxf(tn0, tn1), fmaxf(tn2, s.tmin));
   const float hi = fminf(fminf(tf0, tf1), fminf(tf2, tcull));
-#endif
   return !(lo > hi);
 }
 
@@ -306,253 +278,158 @@ __device__ __forceinline__ bool node_visit(const float4 na, const float4 nb, con
 #ifndef SKW_TRAV_LAG
 #define SKW_TRAV_LAG 12
 #endif
-// Postponed leaves (speculative node steps), see k_trace.
-#ifndef SKW_TRAV_POSTPONE
-#define SKW_TRAV_POSTPONE 1
-#endif
-
 // Traversal stack: the first SCAP entries of each thread live in shared
-// memory as three word arrays indexed [entry][thread] (so lanes never
-// conflict on a bank), deeper entries in local memory.  An entry holds a
-// node's words 6-7 and its widened entry distance.
-#ifndef SKW_TRAV_STACK8
-#define SKW_TRAV_STACK8 0
-#endif
-// Any-hit walks recompute the slab data (12 words) from the ray at the
-// start of every walk round instead of holding it through the triangle
-// tests (measured: 1,439 -> 1,488 Mrays/s on uniform rays over 1.1M
-// triangles); closest-hit walks keep it (there the recomputation measured
-// 2 % slower).  SKW_TRAV_SLAB_ROUND: 0 never, 1 any-hit only, 2 both.
-#ifndef SKW_TRAV_SLAB_ROUND
-#define SKW_TRAV_SLAB_ROUND 1
-#endif
-
+// memory as arrays indexed [entry][thread] (so lanes never conflict on a
+// bank), deeper entries in local memory.  An entry holds a node's words 6-7
+// and its widened entry distance.
 template <int CAP>
 struct Stack {
   static constexpr int SCAP = CAP < SKW_TRAV_SCAP ? CAP : SKW_TRAV_SCAP;
-#if SKW_TRAV_STACK8
-  // Entries are (node index, widened entry distance); a popped node's words
-  // are read back from the tree (a recent, L1-resident line).
-  uint32_t (*sa)[SKW_TRAV_BLOCK];
+  uint2 (*sw)[SKW_TRAV_BLOCK];
   float (*slo)[SKW_TRAV_BLOCK];
-  uint2 ovf[CAP - SCAP > 0 ? CAP - SCAP : 1];
-  const float4 *nodes;
+  uint4 ovf[CAP - SCAP > 0 ? CAP - SCAP : 1];
   int sp;
 
-  __device__ __forceinline__ void push(uint32_t, uint32_t, float lo, uint32_t slot) {
+  __device__ __forceinline__ void push(uint32_t a, uint32_t b, float lo, unsigned *status) {
     if (sp < SCAP) {
-      sa[sp][threadIdx.x] = slot;
+      sw[sp][threadIdx.x] = make_uint2(a, b);
       slo[sp][threadIdx.x] = lo;
+    } else if (sp < CAP) {
+      ovf[sp - SCAP] = make_uint4(a, b, __float_as_uint(lo), 0u);
     } else {
-      ovf[sp - SCAP] = make_uint2(slot, __float_as_uint(lo));
+      atomicOr(status, 1u);  // never: CAP covers the tree's depth
+      return;
     }
     ++sp;
   }
-  __device__ __forceinline__ bool pop(float tcull, uint32_t &a, uint32_t &b) {
-    float lo;
-    return pop(tcull, a, b, lo);
-  }
+  // Pops until an entry survives the re-cull against tcull (the reference
+  // culls the others when it pops them).  A ray that has just found its hit
+  // drops most of its stack here, usually on its own in the warp, so the
+  // loop over the shared entries reads nothing but their distances.
   __device__ __forceinline__ bool pop(float tcull, uint32_t &a, uint32_t &b, float &lo) {
+    while (sp > SCAP) {
+      --sp;
+      const uint4 e = ovf[sp - SCAP];
+      a = e.x;
+      b = e.y;
+      lo = __uint_as_float(e.z);
+      if (!(lo > tcull)) return true;
+    }
     while (sp > 0) {
       --sp;
-      uint32_t slot;
-      if (sp < SCAP) {
-        lo = slo[sp][threadIdx.x];
-        slot = sa[sp][threadIdx.x];
-      } else {
-        const uint2 e = ovf[sp - SCAP];
-        slot = e.x;
-        lo = __uint_as_float(e.y);
-      }
+      lo = slo[sp][threadIdx.x];
       if (!(lo > tcull)) {
-        const float4 nb = __ldg(nodes + 2 * slot + 1);
-        a = __float_as_uint(nb.z);
-        b = __float_as_uint(nb.w);
+        const uint2 e = sw[sp][threadIdx.x];
+        a = e.x;
+        b = e.y;
         return true;
       }
     }
     return false;
   }
-#else
-  uint32_t (*sa)[SKW_TRAV_BLOCK];
-  uint32_t (*sb)[SKW_TRAV_BLOCK];
-  float (*slo)[SKW_TRAV_BLOCK];
-  uint4 ovf[CAP - SCAP > 0 ? CAP - SCAP : 1];
-  int sp;
-
-  __device__ __forceinline__ void push(uint32_t a, uint32_t b, float lo, uint32_t) {
-    if (sp < SCAP) {
-      sa[sp][threadIdx.x] = a;
-      sb[sp][threadIdx.x] = b;
-      slo[sp][threadIdx.x] = lo;
-    } else {
-      ovf[sp - SCAP] = make_uint4(a, b, __float_as_uint(lo), 0u);
-    }
-    ++sp;
-  }
-  // Pops until an entry survives the re-cull against tcull (the reference
-  // culls the others when it pops them).
-  __device__ __forceinline__ bool pop(float tcull, uint32_t &a, uint32_t &b) {
-    float lo;
-    return pop(tcull, a, b, lo);
-  }
-  __device__ __forceinline__ bool pop(float tcull, uint32_t &a, uint32_t &b, float &lo) {
-    while (sp > 0) {
-      --sp;
-      if (sp < SCAP) {
-        lo = slo[sp][threadIdx.x];
-        a = sa[sp][threadIdx.x];
-        b = sb[sp][threadIdx.x];
-      } else {
-        const uint4 e = ovf[sp - SCAP];
-        a = e.x;
-        b = e.y;
-        lo = __uint_as_float(e.z);
-      }
-      if (!(lo > tcull)) return true;
-    }
-    return false;
-  }
-#endif
 };
 
-// Expands internal nodes until (cur_a, cur_b) is a leaf; false when the
-// stack runs out.
+// A 32-byte node (32-byte aligned) in one load.
+__device__ __forceinline__ void load_node(const float4 *__restrict__ nodes, uint32_t i, float4 &a, float4 &b) {
+  asm("ld.global.nc.v8.f32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
+      : "=f"(a.x), "=f"(a.y), "=f"(a.z), "=f"(a.w), "=f"(b.x), "=f"(b.y), "=f"(b.z), "=f"(b.w)
+      : "l"(nodes + 2 * (size_t)i));
+}
+
+// Expands the internal node (cur_a, cur_b): box-tests its present children,
+// makes the first passing one (in the reference's pop order) current and
+// pushes the others; false when none passes.  cur_lo is the current node's
+// widened entry distance.
 //
 // Visit order equals the reference's (TriangleAccelerator.cpp:170-211): the
 // reference pushes an internal node's children and pops the near-side one
-// first, testing each node's box when it is popped.  Here an internal node's
-// present children (contiguous, so their loads go out together) are
-// box-tested right away; the first passing one in the reference's pop order
-// becomes the current node and the rest are pushed so that they pop in that
-// order.  A pushed entry keeps its widened entry distance and is re-culled on
-// pop against the tmax of that moment -- the only part of the reference's
-// pop-time test that can change after the push, since tmax only shrinks.
+// first, testing each node's box when it is popped.  Here the present
+// children (contiguous) are box-tested right away.  A pushed entry keeps its
+// widened entry distance and is re-culled on pop against the tmax of that
+// moment -- the only part of the reference's pop-time test that can change
+// after the push, since tmax only shrinks.
 template <int CAP>
-__device__ __forceinline__ bool descend(const float4 *__restrict__ nodes, const SlabRay &s,
-                                        float tcull, Stack<CAP> &st, uint32_t &cur_a, uint32_t &cur_b,
-                                        unsigned *status) {
-  while ((cur_b & 3u) != 0u) {
-    const uint32_t type = cur_b & 3u, mask = (cur_b >> 2) & 7u;
-    const uint32_t sL = cur_a, sM = cur_a + (mask & 1u), sR = sM + ((mask >> 1) & 1u);
-    const bool near_right = (s.bits >> (type - 1u)) & 1u;  // the reference pops left first when d[axis] > 0
-    uint32_t slot[3], present[3];
-    slot[0] = near_right ? sR : sL;
-    present[0] = near_right ? (mask & 4u) : (mask & 1u);
-    slot[1] = sM;
-    present[1] = mask & 2u;
-    slot[2] = near_right ? sL : sR;
-    present[2] = near_right ? (mask & 1u) : (mask & 4u);
-    bool pass[3];
-    float lo[3];
-    uint32_t wa[3], wb[3];
-#pragma unroll
-    for (int k = 0; k < 3; ++k) {
-      pass[k] = false;
-      wa[k] = wb[k] = 0u;
-      lo[k] = 0.0f;
-      if (present[k]) {
-        const float4 ca = __ldg(nodes + 2 * slot[k]);
-        const float4 cb = __ldg(nodes + 2 * slot[k] + 1);
-        pass[k] = node_visit(ca, cb, s, tcull, lo[k]);
-        wa[k] = __float_as_uint(cb.z);
-        wb[k] = __float_as_uint(cb.w);
-      }
-    }
-    const int first = pass[0] ? 0 : (pass[1] ? 1 : (pass[2] ? 2 : -1));
-    if (st.sp + 2 > CAP) {
-      atomicOr(status, 1u);
-      return false;
-    }
-    if (pass[2] && first != 2) st.push(wa[2], wb[2], lo[2], slot[2]);
-    if (pass[1] && first != 1) st.push(wa[1], wb[1], lo[1], slot[1]);
-    if (first < 0) {
-      if (!st.pop(tcull, cur_a, cur_b)) return false;
-      continue;
-    }
-    cur_a = first == 0 ? wa[0] : (first == 1 ? wa[1] : wa[2]);
-    cur_b = first == 0 ? wb[0] : (first == 1 ? wb[1] : wb[2]);
-  }
-  return true;
-}
-
-// One internal-node step of descend(): box-tests the present children of
-// (cur_a, cur_b), makes the first passing one (in the reference's pop order)
-// current and pushes the others; pops when none passes.  cur_lo tracks the
-// current node's widened entry distance.  False when the stack runs out.
-template <int CAP>
-__device__ __forceinline__ bool step_internal(const float4 *__restrict__ nodes, const SlabRay &s,
-                                              float tcull, Stack<CAP> &st, uint32_t &cur_a, uint32_t &cur_b,
-                                              float &cur_lo, unsigned *status) {
+__device__ __forceinline__ bool expand(const float4 *__restrict__ nodes, const SlabRay &s, float tcull,
+                                       Stack<CAP> &st, uint32_t &cur_a, uint32_t &cur_b, float &cur_lo,
+                                       unsigned *status) {
   const uint32_t type = cur_b & 3u, mask = (cur_b >> 2) & 7u;
+  const bool near_right = (s.bits >> (type - 1u)) & 1u;  // the reference pops left first when d[axis] > 0
   const uint32_t sL = cur_a, sM = cur_a + (mask & 1u), sR = sM + ((mask >> 1) & 1u);
-  const bool near_right = (s.bits >> (type - 1u)) & 1u;
-  uint32_t slot[3], present[3];
-  slot[0] = near_right ? sR : sL;
-  present[0] = near_right ? (mask & 4u) : (mask & 1u);
-  slot[1] = sM;
-  present[1] = mask & 2u;
-  slot[2] = near_right ? sL : sR;
-  present[2] = near_right ? (mask & 1u) : (mask & 4u);
-  bool pass[3];
-  float lo[3];
-  uint32_t wa[3], wb[3];
+  // far, middle, near: the reverse of the pop order
+  const uint32_t slot[3] = {near_right ? sL : sR, sM, near_right ? sR : sL};
+  const bool present[3] = {(mask & (near_right ? 1u : 4u)) != 0u, (mask & 2u) != 0u,
+                           (mask & (near_right ? 4u : 1u)) != 0u};
+  bool have = false;
+  float4 ca[3], cb[3];
+#pragma unroll
+  for (int k = 0; k < 3; ++k) load_node(nodes, present[k] ? slot[k] : sL, ca[k], cb[k]);
 #pragma unroll
   for (int k = 0; k < 3; ++k) {
-    pass[k] = false;
-    wa[k] = wb[k] = 0u;
-    lo[k] = 0.0f;
-    if (present[k]) {
-      const float4 ca = __ldg(nodes + 2 * slot[k]);
-      const float4 cb = __ldg(nodes + 2 * slot[k] + 1);
-      pass[k] = node_visit(ca, cb, s, tcull, lo[k]);
-      wa[k] = __float_as_uint(cb.z);
-      wb[k] = __float_as_uint(cb.w);
+    float lo;
+    if (node_visit(ca[k], cb[k], s, tcull, lo) && present[k]) {
+      if (have) st.push(cur_a, cur_b, cur_lo, status);
+      have = true;
+      cur_a = __float_as_uint(cb[k].z);
+      cur_b = __float_as_uint(cb[k].w);
+      cur_lo = lo;
     }
   }
-  const int first = pass[0] ? 0 : (pass[1] ? 1 : (pass[2] ? 2 : -1));
-  if (st.sp + 2 > CAP) {
-    atomicOr(status, 1u);
-    return false;
-  }
-  if (pass[2] && first != 2) st.push(wa[2], wb[2], lo[2], slot[2]);
-  if (pass[1] && first != 1) st.push(wa[1], wb[1], lo[1], slot[1]);
-  if (first < 0) return st.pop(tcull, cur_a, cur_b, cur_lo);
-  cur_a = first == 0 ? wa[0] : (first == 1 ? wa[1] : wa[2]);
-  cur_b = first == 0 ? wb[0] : (first == 1 ? wb[1] : wb[2]);
-  cur_lo = first == 0 ? lo[0] : (first == 1 ? lo[1] : lo[2]);
-  return true;
+  return have;
 }
 
-// Exact double-precision t of the hit on slot `slot` (its barycentric tests
-// are known to pass).
-__device__ __forceinline__ double exact_t(const float4 *__restrict__ tris, const RayF &r, int slot, float fallback) {
+// The exact (double) decisions of a lane's ray.  They are out of line and
+// read the ray and the triangles from memory again, so that the walk's
+// registers are not laid out around their double temporaries: inline, the
+// kernel spilled in its hot loop.
+template <bool DRAY>
+__device__ __forceinline__ RayD exact_ray(const float4 *__restrict__ rays, int ray_i) {
+  if (DRAY) return load_ray_d(rays, ray_i);
+  const RayF r = load_ray(rays, ray_i);
+  return RayD{r.ox, r.oy, r.oz, r.dx, r.dy, r.dz, r.tmin, r.tmax};
+}
+
+__device__ __forceinline__ bool tri_test64(const float4 *__restrict__ tris, const RayD &r, int slot, double tmax,
+                                           double &t_out) {
   const float4 a = __ldg(tris + 3 * slot), b = __ldg(tris + 3 * slot + 1), c = __ldg(tris + 3 * slot + 2);
+  return tri_test64v(r.ox, r.oy, r.oz, r.dx, r.dy, r.dz, make_float3(a.x, a.y, a.z), make_float3(b.x, b.y, b.z),
+                     make_float3(c.x, c.y, c.z), r.tmin, tmax, t_out);
+}
+
+// t of the hit on slot `slot` (its barycentric tests are known to pass).
+template <bool DRAY>
+__device__ __noinline__ double exact_t(const float4 *__restrict__ tris, const float4 *__restrict__ rays, int ray_i,
+                                       int slot, float fallback) {
   double t;
-  return tri_test64(r, make_float3(a.x, a.y, a.z), make_float3(b.x, b.y, b.z), make_float3(c.x, c.y, c.z),
-                    (double)r.tmin, 1.0e308, t)
-             ? t
-             : (double)fallback;
+  return tri_test64(tris, exact_ray<DRAY>(rays, ray_i), slot, 1.0e308, t) ? t : (double)fallback;
 }
 
-template <bool CLOSEST>
-__device__ __forceinline__ void store_result(void *__restrict__ out, const int32_t *__restrict__ out_index, int ray_i,
-                                             int4 h, bool hit) {
-  const int o = out_index ? SKW_LD_STREAM(out_index + ray_i) : ray_i;
-  if (CLOSEST) {
-    SKW_ST_STREAM((int4 *)out + o, h);
-  } else {
-    ((uint8_t *)out)[o] = hit ? 1 : 0;
-  }
+// Whether the triangle in `slot` is hit no farther than the current tmax:
+// the ray's own (best < 0) or the t of the best hit so far.  On a hit lo / hi
+// bracket its t and `flags` has bit 0 set, and bit 1 where the two t are
+// within 1e-12 relative; no hit: flags = 0.
+struct ExactHit {
+  float lo, hi;
+  uint32_t flags;
+};
+template <bool DRAY>
+__device__ __noinline__ ExactHit exact_hit(const float4 *__restrict__ tris, const float4 *__restrict__ rays, int ray_i,
+                                           int slot, int best, float fallback) {
+  const RayD r = exact_ray<DRAY>(rays, ray_i);
+  double cur_max = r.tmax, t;
+  if (best >= 0) cur_max = tri_test64(tris, r, best, 1.0e308, t) ? t : (double)fallback;
+  if (!tri_test64(tris, r, slot, cur_max, t)) return ExactHit{0.0f, 0.0f, 0u};
+  return ExactHit{__double2float_rd(t), __double2float_ru(t),
+                  best >= 0 && fabs(t - cur_max) <= 1e-12 * fabs(t) ? 3u : 1u};
 }
 
-// Persistent traversal.  The rays form groups of 32 consecutive rays; a warp
+// Persistent traversal.  The rays form groups of consecutive rays; a warp
 // takes the launch's next group from the launch's counter (`work`, one
-// atomicAdd per group) when its current group is used up, or, without a
-// counter, warp w of W owns groups w, w + W, w + 2W, ...  A lane whose ray
-// is finished takes the next ray of the warp's group when at least
+// atomicAdd per group) when its current group is used up, and a lane whose
+// ray is finished takes the next ray of the warp's group when at least
 // SKW_TRAV_REFILL lanes are idle (or all are), so lanes rarely idle while
-// long rays finish.  No cross-warp waits.
+// long rays finish and warps that drew cheap rays take more.  A finished
+// lane keeps its result until then, so that the results of several lanes
+// are written together.  No cross-warp waits.
 //
 // Closest-hit state is kept small: the slot of the current best hit and a
 // float interval [lo_t, hi_t] that contains the reference's current tmax
@@ -562,154 +439,141 @@ __device__ __forceinline__ void store_result(void *__restrict__ out, const int32
 // surf: the rays leave surfaces with tmin from next_min_t (the renders'
 // shadow, BSDF, specular and gather rays, photon bounces).
 //
-// DRAY: the rays are skw_ray_d (double).  The walk runs on the ray rounded
-// to float (origin and direction to nearest, tmin down, tmax up) with the
-// slab widening of make_slab_ray for rounded rays, so a node is still
-// culled only if the reference culls it; every triangle of a reached leaf
-// is tested with the reference's double arithmetic on the double ray
-// (reloaded from memory for the leaf), and the current tmax is kept as the
-// exact double t of the best hit.  Closest-hit results are skw_hit_d
-// (double t, prim, tri).
+// DRAY: the rays are skw_ray_d (double).  The walk and the triangle tests
+// run on the ray rounded to float (origin and direction to nearest, tmin
+// down, tmax up) with the bounds of make_slab_ray and tri_test32 for rounded
+// rays, so a node is still culled only if the reference culls it and a
+// triangle is decided in float only where the double test decides the same;
+// the rest is decided on the double ray (read again from memory).
+// Closest-hit results are skw_hit_d (the exact double t, prim, tri).
+//
+// What bounds it: the latency of the divergent walk (ncu, 1M closest hits:
+// 0.46 instructions issued per cycle and scheduler, 57 % of the stalls on node
+// loads, L1 at 74 % of its peak, DRAM at 3 %).  What the shape of the step is
+// for, measured on 4,194,304 closest / 2,000,003 any hits over 1.1M triangles
+// (3.99 / 1.71 ms before): one place that pops, children loaded and tested
+// without branches, one 32-byte load per node and no spills in the step:
+// 3.47 / 1.33 ms.  200,001 double rays: 3.25 -> 0.53 ms with the float
+// decisions (87 % of the kernel was double triangle tests).
 template <int CAP, bool CLOSEST, bool DRAY>
 __global__ void __launch_bounds__(SKW_TRAV_BLOCK, SKW_TRAV_MINB)
     k_trace(const float4 *__restrict__ nodes, const float4 *__restrict__ tris, const float4 *__restrict__ rays,
             int n, const int *__restrict__ n_dev, float scene_abs, const int32_t *__restrict__ out_index,
-            void *__restrict__ out, unsigned *__restrict__ status, int *__restrict__ work, int surf,
+            void *__restrict__ out, unsigned *__restrict__ status, unsigned *__restrict__ work, int surf,
             unsigned long long *__restrict__ traced) {
-  static_assert(!DRAY || SKW_TRAV_POSTPONE, "double rays use the postponed-leaf walk");
   if (n_dev) n = min(n, *n_dev);  // a queue whose length lives on the device
   if (traced && blockIdx.x == 0 && threadIdx.x == 0 && n > 0) atomicAdd(traced, (unsigned long long)n);
   constexpr int SCAP = Stack<CAP>::SCAP;
-  __shared__ uint32_t s_a[SCAP][SKW_TRAV_BLOCK];
+  __shared__ uint2 s_w[SCAP][SKW_TRAV_BLOCK];
   __shared__ float s_lo[SCAP][SKW_TRAV_BLOCK];
   Stack<CAP> st;
-  st.sa = s_a;
+  st.sw = s_w;
   st.slo = s_lo;
-#if SKW_TRAV_STACK8
-  st.nodes = nodes;
-#else
-  __shared__ uint32_t s_b[SCAP][SKW_TRAV_BLOCK];
-  st.sb = s_b;
-#endif
   st.sp = 0;
 
   const unsigned lane = threadIdx.x & 31u;
-  const int warp = (int)((blockIdx.x * (unsigned)SKW_TRAV_BLOCK + threadIdx.x) >> 5);
+  // Rays per group: 32, or fewer where that leaves warps of the grid without
+  // rays (see the launch).
   const int n_warps = (int)(gridDim.x * (unsigned)(SKW_TRAV_BLOCK / 32));
-  const int groups = (n + 31) >> 5;
-  // Rays come in groups of 32.  Static (work == null): warp w takes groups
-  // w, w + W, ...; next / end are positions in that sequence.  Dynamic: a
-  // warp whose group is used up takes the launch's next group from the
-  // counter *work (zero at launch), so warps that drew cheap rays take more
-  // and the launch's tail is one group long; next / end are positions in
-  // the current group [gbase, gbase + 32), end = -1 once the rays are gone.
-  int next = 0;
-  int end = work ? 0 : (warp < groups ? ((groups - warp + n_warps - 1) / n_warps) << 5 : 0);
-  int gbase = 0;
+  const int group = (int)min(32u, max(1u, ((unsigned)n + (unsigned)n_warps - 1u) / (unsigned)n_warps));
+  // next / end are positions in the current group [gbase, gbase + group);
+  // end = -1 once the rays are gone.
+  int next = 0, end = 0;
+  unsigned gbase = 0;
 
-  int ray_i = -1;
-  // The ray itself is read only by the triangle tests: with
-  // SKW_TRAV_RAYSMEM it waits in shared memory (one word array per field,
-  // [field][thread], conflict-free) instead of holding eight registers
-  // through the node walk.
-#if SKW_TRAV_RAYSMEM
-  __shared__ float s_ray[8][SKW_TRAV_BLOCK];
-#define SKW_RAY()                                                                                          \
-  RayF {                                                                                                   \
-    s_ray[0][threadIdx.x], s_ray[1][threadIdx.x], s_ray[2][threadIdx.x], s_ray[3][threadIdx.x],            \
-        s_ray[4][threadIdx.x], s_ray[5][threadIdx.x], s_ray[6][threadIdx.x], s_ray[7][threadIdx.x]        \
-  }
-#else
-  RayF r_reg{};
-#define SKW_RAY() r_reg
-#endif
-  constexpr bool kSlabRound = SKW_TRAV_SLAB_ROUND == 2 || (SKW_TRAV_SLAB_ROUND == 1 && !CLOSEST);
-  SlabRay s_keep{};  // the walk's slab data when it is kept across rounds
+  int ray_i = -1;    // the lane's ray
+  bool fin = true;   // its walk is over; its result waits while ray_i >= 0
+  bool hit = false;  // any hit: the result
+  RayF r{};          // read only by the triangle tests
+  constexpr float kSlabWiden = DRAY ? 9.0f : 6.0f;
   uint32_t cur_a = 0, cur_b = 0;
+  float cur_lo = 0.0f;
   int best_slot = -1;
-  double best_t = 0.0;             // DRAY: the exact t of the best hit
   float lo_t = 0.0f, hi_t = 0.0f;  // bracket of the reference's current tmax
   uint32_t flags = 0;              // SKW_HIT_* bits; bit 3: [lo_t, hi_t] brackets an exact double
-#if SKW_TRAV_POSTPONE
-  bool trav = false, has_post = false;  // traversal not finished; a leaf is postponed
-  uint32_t post_a = 0, post_cnt = 0;
-  float cur_lo = 0.0f;
-#endif
 
   while (true) {
-    const unsigned idle = __ballot_sync(0xffffffffu, ray_i < 0);
-    if (idle != 0u && (__popc(idle) >= SKW_TRAV_REFILL || idle == 0xffffffffu) && work && end >= 0 && next >= end) {
-      int base = 0;
-      if (lane == 0) base = atomicAdd(work, 32);
-      base = __shfl_sync(0xffffffffu, base, 0);
-      gbase = base;
-      next = 0;
-      end = base < n ? min(32, n - base) : -1;
-    }
-    if (idle != 0u && next < end && (__popc(idle) >= SKW_TRAV_REFILL || idle == 0xffffffffu)) {
-      const int mine = next + __popc(idle & ((1u << lane) - 1u));
-      next += __popc(idle);
-      const int idx = work ? gbase + mine : ((warp + (mine >> 5) * n_warps) << 5) + (mine & 31);
-      if (ray_i < 0 && mine < end && idx < n) {
-        ray_i = idx;
-        RayF rl;
-        if (DRAY) {
-          const RayD rd = load_ray_d(rays, ray_i);
-          rl = RayF{(float)rd.ox, (float)rd.oy, (float)rd.oz, (float)rd.dx, (float)rd.dy, (float)rd.dz,
-                    __double2float_rd(rd.tmin), __double2float_ru(rd.tmax)};
+    const unsigned idle = __ballot_sync(0xffffffffu, fin);
+    if (idle != 0u && (__popc(idle) >= SKW_TRAV_REFILL || idle == 0xffffffffu)) {
+      // the finished lanes' results
+      if (fin && ray_i >= 0) {
+        const int o = out_index ? SKW_LD_STREAM(out_index + ray_i) : ray_i;
+        if (!CLOSEST) {
+          ((uint8_t *)out)[o] = hit ? 1 : 0;
         } else {
-          rl = load_ray(rays, ray_i);
-        }
-#if SKW_TRAV_RAYSMEM
-        s_ray[0][threadIdx.x] = rl.ox;
-        s_ray[1][threadIdx.x] = rl.oy;
-        s_ray[2][threadIdx.x] = rl.oz;
-        s_ray[3][threadIdx.x] = rl.dx;
-        s_ray[4][threadIdx.x] = rl.dy;
-        s_ray[5][threadIdx.x] = rl.dz;
-        s_ray[6][threadIdx.x] = rl.tmin;
-        s_ray[7][threadIdx.x] = rl.tmax;
-#else
-        r_reg = rl;
-#endif
-        const SlabRay s = make_slab_ray(rl, scene_abs, DRAY ? 9.0f : 6.0f);
-        if (!kSlabRound) s_keep = s;
-        best_slot = -1;
-        lo_t = hi_t = rl.tmax;
-        flags = 8u;
-        st.sp = 0;
-        const float4 na = __ldg(nodes), nb = __ldg(nodes + 1);
-        float lo;
-        cur_a = __float_as_uint(nb.z);
-        cur_b = __float_as_uint(nb.w);
-        if (!node_visit(na, nb, s, rl.tmax, lo)) {  // root culled: a miss
-          if (DRAY && CLOSEST) {
-            ((int4 *)out)[out_index ? out_index[ray_i] : ray_i] = make_int4(0, 0x7ff00000, -1, -1);
-          } else {
-            store_result<CLOSEST>(out, out_index, ray_i, make_int4(0x7f800000, -1, -1, 0), false);
+          int4 h = DRAY ? make_int4(0, 0x7ff00000, -1, -1)  // t = +inf, a miss
+                        : make_int4(0x7f800000, -1, -1, (int)(flags & 7u));
+          if (best_slot >= 0) {
+            const int prim = __float_as_int(__ldg(tris + 3 * best_slot).w),
+                      tri = __float_as_int(__ldg(tris + 3 * best_slot + 1).w);
+            float tout = 0.5f * lo_t + 0.5f * hi_t;
+            if (DRAY) {
+              const long long t64 =
+                  __double_as_longlong(exact_t<DRAY>(tris, rays, ray_i, best_slot, tout));
+              h = make_int4((int)(t64 & 0xffffffffll), (int)(t64 >> 32), prim, tri);
+            } else {
+              // A float-decided hit whose bracket is wider than the 1e-5 reporting
+              // tolerance (grazing incidence) takes t from the exact test.
+              if (!(flags & 8u) && hi_t - lo_t > 1.0e-5f * fabsf(tout)) {
+                tout = (float)exact_t<DRAY>(tris, rays, ray_i, best_slot, tout);
+                flags |= 4u;
+              }
+              h = make_int4(__float_as_int(tout), prim, tri, (int)(flags & 7u));
+            }
           }
-          ray_i = -1;
+          SKW_ST_STREAM((int4 *)out + o, h);
         }
-#if SKW_TRAV_POSTPONE
-        trav = true;
-        has_post = false;
-        cur_lo = lo;
-#endif
+        ray_i = -1;
+      }
+      // new rays
+      if (end >= 0 && next >= end) {
+        if (lane == 0) gbase = atomicAdd(work, (unsigned)group);
+        gbase = __shfl_sync(0xffffffffu, gbase, 0);
+        next = 0;
+        end = gbase < (unsigned)n ? min(group, n - (int)gbase) : -1;
+      }
+      if (next < end) {
+        const int mine = next + __popc(idle & ((1u << lane) - 1u));
+        next += __popc(idle);
+        if (fin && mine < end) {
+          ray_i = (int)gbase + mine;
+          if (DRAY) {
+            const RayD rd = load_ray_d(rays, ray_i);
+            r = RayF{(float)rd.ox, (float)rd.oy, (float)rd.oz, (float)rd.dx, (float)rd.dy, (float)rd.dz,
+                     __double2float_rd(rd.tmin), __double2float_ru(rd.tmax)};
+            lo_t = __double2float_rd(rd.tmax);
+          } else {
+            r = load_ray(rays, ray_i);
+            lo_t = r.tmax;
+          }
+          hi_t = r.tmax;
+          const SlabRay s = make_slab_ray(r, scene_abs, kSlabWiden);
+          best_slot = -1;
+          flags = 8u;
+          hit = false;
+          st.sp = 0;
+          const float4 na = __ldg(nodes), nb = __ldg(nodes + 1);
+          cur_a = __float_as_uint(nb.z);
+          cur_b = __float_as_uint(nb.w);
+          fin = !node_visit(na, nb, s, r.tmax, cur_lo);  // root culled: a miss
+        }
       }
     }
-    const unsigned busy = __ballot_sync(0xffffffffu, ray_i >= 0);
+    const unsigned busy = __ballot_sync(0xffffffffu, !fin);
     if (busy == 0u) {
-      if (next >= end && (!work || end < 0)) break;
+      if (end < 0 && __ballot_sync(0xffffffffu, ray_i >= 0) == 0u) break;
       continue;
     }
-    if (ray_i < 0) continue;
+    if (fin) continue;
     // Independent thread scheduling does not promise that the busy lanes run
     // the rest of the iteration as one group; without an explicit sync they
     // were measured to split into 2-3 groups that each walked on their own.
     __syncwarp(busy);
-    const SlabRay s = kSlabRound ? make_slab_ray(SKW_RAY(), scene_abs, DRAY ? 9.0f : 6.0f) : s_keep;
+    // The slab data (14 words) is made from the ray in every round instead of
+    // being held through the triangle tests (measured at 80 registers, 4M
+    // closest hits: 3.69 -> 3.50 ms).
+    const SlabRay s = make_slab_ray(r, scene_abs, kSlabWiden);
 
-#if SKW_TRAV_POSTPONE
     // Node steps continue past a lane's first leaf (postponed) until all but
     // SKW_TRAV_LAG walking lanes hold one, or the lane reaches a second leaf;
     // the leaves are then tested in the order they were reached, which is
@@ -719,72 +583,42 @@ __global__ void __launch_bounds__(SKW_TRAV_BLOCK, SKW_TRAV_MINB)
     // is tested see a larger tmax than the reference's -- a superset of its
     // visits, whose extra triangles all lie beyond the final tmax.
     //
-    // Every busy lane is walking when the round starts (a busy lane whose
-    // walk had ended would have finished its ray).  All of them stay in the
-    // loop -- a lane that is done idles -- and vote on every step over the
-    // busy mask, so they stay one group (a vote over __activemask() would
+    // Every busy lane is walking when the round starts.  All of them stay in
+    // the loop -- a lane that is done idles -- and vote on every step over
+    // the busy mask, so they stay one group (a vote over __activemask() would
     // only cover whatever fragment happens to be running together) and one
     // vote per step suffices.
     const float tcull = CLOSEST ? hi_t : s.tmax;
-    bool walking = trav;
+    const int lag = min(SKW_TRAV_LAG, __popc(busy) >> 1);
+    bool walking = true, trav = true, has_post = false;
+    uint32_t post_a = 0, post_cnt = 0;
     while (true) {
       if (walking) {
-        bool stop = false;
+        bool pop = true;
         if ((cur_b & 3u) == 0u) {  // a leaf
           if (has_post) {
-            stop = true;  // a second leaf: it waits for the next round
-          } else {
-            if (!(cur_lo > tcull)) {
-              post_a = cur_a;
-              post_cnt = cur_b >> 8;
-              has_post = true;
-            }
-            trav = st.pop(tcull, cur_a, cur_b, cur_lo);
+            walking = pop = false;  // a second leaf: it waits for the next round
+          } else if (!(cur_lo > tcull)) {
+            post_a = cur_a;
+            post_cnt = cur_b >> 8;
+            has_post = true;
           }
-        } else {
-          trav = step_internal(nodes, s, tcull, st, cur_a, cur_b, cur_lo, status);
+        } else if (!(cur_lo > tcull)) {
+          pop = !expand(nodes, s, tcull, st, cur_a, cur_b, cur_lo, status);
         }
-        walking = trav && !stop;
+        if (pop) walking = trav = st.pop(tcull, cur_a, cur_b, cur_lo);
       }
-      if (__popc(__ballot_sync(busy, walking && !has_post)) <= SKW_TRAV_LAG) break;
+      if (__popc(__ballot_sync(busy, walking && !has_post)) <= lag) break;
     }
     __syncwarp(busy);
-    bool hit = false;
-    if (DRAY && has_post) {
-      // every triangle of the leaf in the reference's double arithmetic
-      has_post = false;
-      const RayD rd = load_ray_d(rays, ray_i);
+    if (has_post) {
       for (uint32_t k = 0; k < post_cnt; ++k) {
         const int slot = (int)(post_a + k);
         float3 v0, v1, v2;
         int prim, tri;
         load_tri(tris, (uint32_t)slot, v0, v1, v2, prim, tri);
-        double t64;
-        if (tri_test64v(rd.ox, rd.oy, rd.oz, rd.dx, rd.dy, rd.dz, v0, v1, v2, rd.tmin,
-                        CLOSEST && best_slot >= 0 ? best_t : rd.tmax, t64)) {
-          if (!CLOSEST) {
-            hit = true;
-            break;
-          }
-          if (best_slot >= 0 && fabs(t64 - best_t) <= 1e-12 * fabs(t64)) flags |= 2u;
-          best_slot = slot;
-          best_t = t64;
-          lo_t = __double2float_rd(t64);
-          hi_t = __double2float_ru(t64);
-        }
-      }
-    }
-    if (!DRAY && has_post) {
-      has_post = false;
-      const RayF r = SKW_RAY();
-      const uint32_t a = post_a, cnt = post_cnt;
-      for (uint32_t k = 0; k < cnt; ++k) {
-        const int slot = (int)(a + k);
-        float3 v0, v1, v2;
-        int prim, tri;
-        load_tri(tris, (uint32_t)slot, v0, v1, v2, prim, tri);
         float t, et;
-        int res = tri_test32(r, v0, v1, v2, t, et);
+        const int res = tri_test32<DRAY>(r, v0, v1, v2, t, et);
         if (res == kMiss) continue;
         // A ray leaving a surface (surf) starts at an upper bound of the
         // reference's GetNextMinT: a triangle whose t cannot be told apart
@@ -804,14 +638,12 @@ __global__ void __launch_bounds__(SKW_TRAV_BLOCK, SKW_TRAV_MINB)
             }
           }
           // Exact re-test against the reference's exact current tmax.
-          const double cur_max = best_slot < 0 ? (double)r.tmax : exact_t(tris, r, best_slot, hi_t);
-          double t64;
-          if (tri_test64(r, v0, v1, v2, (double)r.tmin, cur_max, t64)) {
-            if (best_slot >= 0 && fabs(t64 - cur_max) <= 1e-12 * fabs(t64)) flags |= 2u;
+          const ExactHit x = exact_hit<DRAY>(tris, rays, ray_i, slot, best_slot, hi_t);
+          if (x.flags != 0u) {
             best_slot = slot;
-            lo_t = __double2float_rd(t64);
-            hi_t = __double2float_ru(t64);
-            flags |= 1u | 8u;
+            lo_t = x.lo;
+            hi_t = x.hi;
+            flags |= x.flags | 8u;
           }
         } else {
           if (res == kHit) {
@@ -821,105 +653,14 @@ __global__ void __launch_bounds__(SKW_TRAV_BLOCK, SKW_TRAV_MINB)
             }
             if (t - et > r.tmax) continue;
           }
-          double t64;
-          if (tri_test64(r, v0, v1, v2, (double)r.tmin, (double)r.tmax, t64)) {
+          if (exact_hit<DRAY>(tris, rays, ray_i, slot, -1, 0.0f).flags != 0u) {
             hit = true;
             break;
           }
         }
       }
     }
-    bool done = hit || (!trav && !has_post);
-#else
-    const float tcull = CLOSEST ? hi_t : s.tmax;
-    bool done = !descend(nodes, s, tcull, st, cur_a, cur_b, status);
-    bool hit = false;
-    if (!done) {
-      const RayF r = SKW_RAY();
-      // cur is a leaf: test its triangles in order.
-      const uint32_t a = cur_a, cnt = cur_b >> 8;
-      for (uint32_t k = 0; k < cnt; ++k) {
-        const int slot = (int)(a + k);
-        float3 v0, v1, v2;
-        int prim, tri;
-        load_tri(tris, (uint32_t)slot, v0, v1, v2, prim, tri);
-        float t, et;
-        int res = tri_test32(r, v0, v1, v2, t, et);
-        if (res == kMiss) continue;
-        // A ray leaving a surface (surf) starts at an upper bound of the
-        // reference's GetNextMinT: a triangle whose t cannot be told apart
-        // from that tmin in float lies on the ray's own plane crossing --
-        // the triangle it leaves, or geometry touching it there -- and is
-        // skipped, as the reference's tmin skips the triangle it leaves.
-        if (surf && res == kAmbiguous && t - et < r.tmin) continue;
-        if (CLOSEST) {
-          if (res == kHit) {
-            if (__fsub_rd(t, et) > hi_t) continue;  // certainly beyond the current tmax
-            if (__fadd_ru(t, et) < lo_t) {          // certainly nearer: accept in float
-              best_slot = slot;
-              lo_t = __fsub_rd(t, et);
-              hi_t = __fadd_ru(t, et);
-              flags &= ~8u;
-              continue;
-            }
-          }
-          // Exact re-test against the reference's exact current tmax.
-          const double cur_max = best_slot < 0 ? (double)r.tmax : exact_t(tris, r, best_slot, hi_t);
-          double t64;
-          if (tri_test64(r, v0, v1, v2, (double)r.tmin, cur_max, t64)) {
-            if (best_slot >= 0 && fabs(t64 - cur_max) <= 1e-12 * fabs(t64)) flags |= 2u;
-            best_slot = slot;
-            lo_t = __double2float_rd(t64);
-            hi_t = __double2float_ru(t64);
-            flags |= 1u | 8u;
-          }
-        } else {
-          if (res == kHit) {
-            if (t + et < r.tmax) {
-              hit = true;
-              break;
-            }
-            if (t - et > r.tmax) continue;
-          }
-          double t64;
-          if (tri_test64(r, v0, v1, v2, (double)r.tmin, (double)r.tmax, t64)) {
-            hit = true;
-            break;
-          }
-        }
-      }
-      done = hit || !st.pop(CLOSEST ? hi_t : s.tmax, cur_a, cur_b);
-    }
-#endif
-    if (DRAY && done) {
-      if (CLOSEST) {
-        int4 h = make_int4(0, 0x7ff00000, -1, -1);  // t = +inf, a miss
-        if (best_slot >= 0) {
-          const float4 ta = __ldg(tris + 3 * best_slot), tb = __ldg(tris + 3 * best_slot + 1);
-          const long long tb64 = __double_as_longlong(best_t);
-          h = make_int4((int)(tb64 & 0xffffffffll), (int)(tb64 >> 32), __float_as_int(ta.w), __float_as_int(tb.w));
-        }
-        ((int4 *)out)[out_index ? out_index[ray_i] : ray_i] = h;
-      } else {
-        store_result<CLOSEST>(out, out_index, ray_i, int4{}, hit);
-      }
-      ray_i = -1;
-    } else if (done) {
-      int4 h = make_int4(0x7f800000, -1, -1, (int)(flags & 7u));
-      if (CLOSEST && best_slot >= 0) {
-        const float4 ta = __ldg(tris + 3 * best_slot), tb = __ldg(tris + 3 * best_slot + 1);
-        float tout = 0.5f * lo_t + 0.5f * hi_t;
-        // A float-decided hit whose bracket is wider than the 1e-5 reporting
-        // tolerance (grazing incidence) takes t from the exact test.
-        if (!(flags & 8u) && hi_t - lo_t > 1.0e-5f * fabsf(tout)) {
-          tout = (float)exact_t(tris, SKW_RAY(), best_slot, tout);
-          flags |= 4u;
-        }
-        h = make_int4(__float_as_int(tout), __float_as_int(ta.w), __float_as_int(tb.w), (int)(flags & 7u));
-      }
-      store_result<CLOSEST>(out, out_index, ray_i, h, hit);
-      ray_i = -1;
-    }
+    fin = hit || !trav;
   }
 }
 
@@ -1143,14 +884,8 @@ cudaError_t cap_prepare(int dev) {
   for (int v = 0; v < 4; ++v) {
     std::atomic<int> &slot = cap_occupancy<CAP>(dev, v);
     if (slot.load(std::memory_order_relaxed) != 0) continue;
-    cudaError_t e;
-    if (SKW_TRAV_CARVEOUT >= 0) {
-      e = cudaFuncSetAttribute(trace_kernel<CAP>(v), cudaFuncAttributePreferredSharedMemoryCarveout,
-                               SKW_TRAV_CARVEOUT);
-      if (e != cudaSuccess) return e;
-    }
     int occ = 0;
-    e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, trace_kernel<CAP>(v), SKW_TRAV_BLOCK, 0);
+    const cudaError_t e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, trace_kernel<CAP>(v), SKW_TRAV_BLOCK, 0);
     if (e != cudaSuccess) return e;
     slot.store(occ < 1 ? 1 : occ, std::memory_order_release);
   }
@@ -1225,6 +960,7 @@ template <int CAP>
 cudaError_t launch_cap(int variant, const void *nodes, const void *tris, const void *rays, int64_t n,
                        const int *n_dev, float scene_abs, const int32_t *out_index, void *out, unsigned *status,
                        cudaStream_t stream, int ctas_per_sm, int *work, int surf) {
+  if (!work) return cudaErrorInvalidValue;
   int dev = 0, sms = 0;
   cudaError_t e = current_device(dev);
   if (e != cudaSuccess || (e = cap_prepare<CAP>(dev)) != cudaSuccess || (e = device_sms(dev, sms)) != cudaSuccess)
@@ -1236,29 +972,31 @@ cudaError_t launch_cap(int variant, const void *nodes, const void *tris, const v
   if (ctas_per_sm > 0 && ctas_per_sm < per_sm) per_sm = ctas_per_sm;
   const int64_t warps_per_block = SKW_TRAV_BLOCK / 32;
   int64_t blocks = (int64_t)per_sm * sms;
-  const int64_t needed = (n + 32 * warps_per_block - 1) / (32 * warps_per_block);
+  // A launch of fewer rays than the grid has lanes spreads them over all
+  // resident warps, down to one ray per warp: a warp's time is the sum of its
+  // lanes' divergent paths (1,000 rays over 18,000 triangles: 142 us in groups
+  // of 16, 106 us in groups of 1).
+  const int64_t needed = (n + warps_per_block - 1) / warps_per_block;
   if (blocks > needed) blocks = needed;
-  // every warp draws at most one group past the end: keep the counter in int range
-  if (n > (int64_t)INT32_MAX - 32 * warps_per_block * blocks) work = nullptr;
-  if (work && (e = cudaMemsetAsync(work, 0, sizeof(int), stream)) != cudaSuccess) return e;
+  if ((e = cudaMemsetAsync(work, 0, sizeof(int), stream)) != cudaSuccess) return e;
   const float4 *nd = (const float4 *)nodes, *tr = (const float4 *)tris, *ry = (const float4 *)rays;
   const dim3 grid((unsigned)blocks), block(SKW_TRAV_BLOCK);
   switch (variant) {
     case 0:
       k_trace<CAP, false, false><<<grid, block, 0, stream>>>(nd, tr, ry, (int)n, n_dev, scene_abs, out_index, out,
-                                                             status, work, surf, T.traced);
+                                                             status, (unsigned *)work, surf, T.traced);
       break;
     case 1:
       k_trace<CAP, true, false><<<grid, block, 0, stream>>>(nd, tr, ry, (int)n, n_dev, scene_abs, out_index, out,
-                                                            status, work, surf, T.traced);
+                                                            status, (unsigned *)work, surf, T.traced);
       break;
     case 2:
       k_trace<CAP, false, true><<<grid, block, 0, stream>>>(nd, tr, ry, (int)n, n_dev, scene_abs, out_index, out,
-                                                            status, work, surf, T.traced);
+                                                            status, (unsigned *)work, surf, T.traced);
       break;
     default:
       k_trace<CAP, true, true><<<grid, block, 0, stream>>>(nd, tr, ry, (int)n, n_dev, scene_abs, out_index, out,
-                                                           status, work, surf, T.traced);
+                                                           status, (unsigned *)work, surf, T.traced);
   }
   return cudaGetLastError();
 }
