@@ -200,7 +200,7 @@ cudaError_t launch_resolve_media(bool adjoint, int64_t capacity, const uint8_t *
 // dL/d(triangle albedo) (3 floats per global triangle) and dL/d(emission
 // scale) from dfilm = dL/dI (3 floats per global pixel).
 cudaError_t launch_shade_adjoint(const SceneDev &S, const ViewDev *views, int n_views, int n, int64_t px_begin, int spp,
-                                 int n_light_samples, const float *dfilm, float *g_albedo, double *g_emission,
+                                 int n_light_samples, const float *dfilm, double *g_emission,
                                  const void *rays, const void *hits, void *srays, int *stri, float *s_dkd,
                                  float *s_dem, int *scount, void *brays, int *btri, float *b_dkd, float *brgb,
                                  int *bcount, float *bnrm, const float *tcam, cudaStream_t s, int ld = 0,
@@ -208,7 +208,7 @@ cudaError_t launch_shade_adjoint(const SceneDev &S, const ViewDev *views, int n_
 // Adjoint of one specular level (the entries' weights multiply dL/dI).
 cudaError_t launch_shade_specular_adjoint(const SceneDev &S, const ViewDev *views, int n_views, int64_t capacity,
                                           int64_t px_begin, int spp, int n_light_samples, const float *dfilm,
-                                          float *g_albedo, double *g_emission, const SpecQueues &spec, int depth,
+                                          double *g_emission, const SpecQueues &spec, int depth,
                                           const void *hits, void *srays, int *stri, float *s_dkd, float *s_dem,
                                           int *scount, void *brays, int *btri, float *b_dkd, float *brgb,
                                           int *bcount, float *bnrm, cudaStream_t s,
@@ -216,8 +216,11 @@ cudaError_t launch_shade_specular_adjoint(const SceneDev &S, const ViewDev *view
 cudaError_t launch_resolve_adjoint(const SceneDev &S, int capacity, int n_light_samples, const uint8_t *occ,
                                    const int *stri, const float *s_dkd, const float *s_dem, const int *scount,
                                    const void *brays, const void *bhits, const int *btri, const float *b_dkd,
-                                   const float *brgb, const int *bcount, const float *bnrm, float *g_albedo,
-                                   double *g_emission, cudaStream_t s, bool capped = false);
+                                   const float *brgb, const int *bcount, const float *bnrm, void *g_albedo,
+                                   double *g_emission, cudaStream_t s);
+// launch_resolve_adjoint's g_albedo: 4 floats per global triangle, 16-byte
+// aligned; launch_albedo_grad adds the first three of each to g_albedo.
+cudaError_t launch_albedo_grad(const void *sum, int64_t n, float *g_albedo, cudaStream_t s);
 
 // Photon mapping (photon.cu).  trace(rays, n, n_dev, hits, stream) runs the
 // closest-hit traversal of the scene's accelerator.

@@ -1481,16 +1481,19 @@ int skw_render_direct_adjoint(skw_scene *s, const skw_camera *cam, const skw_ren
   if ((e = skw::ctx_pool(ctx, &pool)) != cudaSuccess) return cuda_fail(ctx, e, "workspace pool");
   const int64_t sh = std::max<int64_t>(P.cap_shadow, 1), bs = std::max<int64_t>(P.cap_bsdf, 1);
   const size_t wbytes = workspace_bytes(P), vbytes = al256(sizeof(skw::ViewDev)), xbytes = al256(sh * 4) + al256(bs * 12);
+  const size_t sbytes = (size_t)s->n_triangles * 16;  // the albedo gradient's sums
   char *w = nullptr;
-  if ((e = cudaMallocFromPoolAsync((void **)&w, wbytes + vbytes + xbytes, pool, st)) != cudaSuccess)
+  if ((e = cudaMallocFromPoolAsync((void **)&w, wbytes + vbytes + xbytes + sbytes, pool, st)) != cudaSuccess)
     return cuda_fail(ctx, e, "adjoint workspace");
   Workspace W;
   workspace_carve(P, w, &W);
   skw::ViewDev *d_view = (skw::ViewDev *)(w + wbytes);
   float *s_dem = (float *)(w + wbytes + vbytes), *b_dkd = (float *)(w + wbytes + vbytes + al256(sh * 4));
   float *s_dkd = W.srgb;  // 3 floats per shadow entry, like the forward pass's radiance
+  void *sum = w + wbytes + vbytes + xbytes;
   skw_accel *a = s->accel;
   e = cudaMemcpyAsync(d_view, P.views.data(), sizeof(skw::ViewDev), cudaMemcpyHostToDevice, st);
+  if (e == cudaSuccess) e = cudaMemsetAsync(sum, 0, sbytes, st);
   skw::SpecQueues sq0{};  // the camera level's children go to queue 0
   if (P.spec_levels) {
     sq0.out_rays = W.qrays[0];
@@ -1509,7 +1512,7 @@ int skw_render_direct_adjoint(skw_scene *s, const skw_camera *cam, const skw_ren
                                    W.hits, a->d_status, st, 0, W.counts + 8)) != cudaSuccess)
       break;
     if (P.media && (e = record_media(s, P, W, d_view, px0, n, true, d_film, g_emission, st)) != cudaSuccess) break;
-    if ((e = skw::launch_shade_adjoint(s->dev, d_view, 1, n, px0, P.spp, P.nl, d_film, g_albedo, g_emission, W.rays,
+    if ((e = skw::launch_shade_adjoint(s->dev, d_view, 1, n, px0, P.spp, P.nl, d_film, g_emission, W.rays,
                                        W.hits, W.srays, W.starget, s_dkd, s_dem, W.counts, W.brays, W.btarget, b_dkd,
                                        W.brgb, W.counts + 1, W.bnrm, P.media ? W.tcam : nullptr, st, P.ld,
                                        P.spec_levels ? &sq0 : nullptr)) != cudaSuccess)
@@ -1523,7 +1526,7 @@ int skw_render_direct_adjoint(skw_scene *s, const skw_camera *cam, const skw_ren
       break;
     if ((e = skw::launch_resolve_adjoint(s->dev, (int)std::max(csh, cbs), P.nl, W.occ, W.starget, s_dkd, s_dem,
                                          W.counts, W.brays, W.bhits, W.btarget, b_dkd, W.brgb, W.counts + 1, W.bnrm,
-                                         g_albedo, g_emission, st)) != cudaSuccess)
+                                         sum, g_emission, st)) != cudaSuccess)
       break;
     launches += 7;
     // The specular levels, replayed as in record_specular with the adjoint
@@ -1554,7 +1557,7 @@ int skw_render_direct_adjoint(skw_scene *s, const skw_camera *cam, const skw_ren
       if (P.media &&
           (e = record_media_level(s, P, W, d_view, px0, qi, cl, true, d_film, g_emission, st, nullptr)) != cudaSuccess)
         break;
-      if ((e = skw::launch_shade_specular_adjoint(s->dev, d_view, 1, cl, px0, P.spp, P.nl, d_film, g_albedo,
+      if ((e = skw::launch_shade_specular_adjoint(s->dev, d_view, 1, cl, px0, P.spp, P.nl, d_film,
                                                   g_emission, q, L, W.qhits, W.srays, W.starget, s_dkd, s_dem,
                                                   W.counts, W.brays, W.btarget, b_dkd, W.brgb, W.counts + 1,
                                                   W.bnrm, st, P.media ? W.tcam : nullptr)) != cudaSuccess)
@@ -1568,11 +1571,12 @@ int skw_render_direct_adjoint(skw_scene *s, const skw_camera *cam, const skw_ren
         break;
       if ((e = skw::launch_resolve_adjoint(s->dev, (int)std::max(lsh, lbs), P.nl, W.occ, W.starget, s_dkd, s_dem,
                                            W.counts, W.brays, W.bhits, W.btarget, b_dkd, W.brgb, W.counts + 1,
-                                           W.bnrm, g_albedo, g_emission, st, true)) != cudaSuccess)
+                                           W.bnrm, sum, g_emission, st)) != cudaSuccess)
         break;
       launches += 6;
     }
   }
+  if (e == cudaSuccess) e = skw::launch_albedo_grad(sum, s->n_triangles, g_albedo, st);
   cudaFreeAsync(w, st);
   if (e != cudaSuccess) return cuda_fail(ctx, e, "direct-lighting adjoint");
   ctx->launches.fetch_add(launches);
