@@ -14,11 +14,14 @@
 //     first of equal values (it matters only for the sign of a zero);
 //   * leaf rule (<= 4 triangles, all three axes split through the middle,
 //     depth 200), candidate count tries = min(200, 2n), per-axis scale;
-//   * buckets: per candidate plane the left / middle / right boxes and
-//     counts, filled by atomics on order-preserving float keys (box unions
-//     and counts do not depend on the order they are formed in);
-//   * split search: one thread per (node, axis), suffix unions of the right
-//     boxes, then the costs in the reference's double arithmetic in order;
+//   * split search, by node size: per candidate plane the left / middle /
+//     right boxes and counts (box unions and counts do not depend on the
+//     order they are formed in), then the costs in the reference's double
+//     arithmetic, which only the planes that could be the least by their
+//     float costs need.  Up to 32 triangles one warp holds the node's boxes
+//     and each lane a plane (k_split_small); up to 4,096 a block per axis
+//     fills buckets in shared memory (k_split_mid); above that blocks of 4,096
+//     triangles do and merge them into global ones (k_fill_big, k_score_big);
 //   * partition: the reference's sequential swap loop (left to the front in
 //     order of processing, right to the back, a rotating middle block)
 //     computed in parallel.  Elements are processed from the front, except
@@ -48,6 +51,10 @@ constexpr int kB = 256;
 constexpr int kTries = 200;    // TriangleAccelerator.h:131
 constexpr int kLeafMax = 4;    // TriangleAccelerator.h:128
 constexpr int kDepthMax = 200; // TriangleAccelerator.h:134
+// Split search by node size.  Below 33 triangles a node has at most 64
+// planes, two per lane; a chunk of 4,096 triangles outweighs the 4,200 words
+// of an axis' buckets that its block empties and merges.
+constexpr int kSmall = 32, kMid = 4096;
 
 // Order-preserving key of a float (NaN excluded by the callers).
 __device__ __forceinline__ uint32_t okey(float f) {
@@ -100,13 +107,17 @@ struct Dev {
   float *hbox;                // 6 floats
   double *hcoef;              // 3 per node
   double *hsplit;
-  // (a node's bucket base is cnt2[b] between the bucket scan and the split search)
-  int32_t *hid, *htries, *haxis;
+  int32_t *hid, *htries, *haxis, *hbase;  // hbase: a big node's first bucket
   uint32_t *heads;            // the level's nodes' first slots, by rank
   uint32_t *hnl, *hnr;
   uint8_t *hleaf;
   double *bcost, *bpos;       // 3 per node
-  uint32_t *buckets;          // 7 words per bucket: lo keys, hi keys, count
+  uint32_t *buckets;          // big nodes, 7 words per bucket: lo keys, hi keys, count
+  // The level's nodes to split, by size (their first slots), and the chunks
+  // of the big ones (first slot of the node, chunk); count: their numbers.
+  uint32_t *small, *mid, *big;
+  uint2 *chunks;
+  int *count;                 // small, mid, big, chunks
   // per level
   uint8_t *cls;
   uint64_t *cnt, *cnt2, *cnt3, *sums;  // n + 1 each (sums: block totals)
@@ -196,11 +207,9 @@ __global__ void k_node_box(Dev D) {
 
 // A node's record and leaf decision (Node::Node, TriangleAccelerator.cpp:
 // 621-636); internal nodes get their candidate count and per-axis scale
-// (_DetermineBestSplit, :512-530) and ask for 9 * tries buckets.
+// (_DetermineBestSplit, :512-530) and go to the list of their size.
 __global__ void k_head_setup(Dev D, int64_t level_base, int depth) {
   const int64_t s = (int64_t)blockIdx.x * kB + threadIdx.x;
-  if (s > D.n) return;
-  uint64_t need = 0;
   if (s < D.n && D.seg[s].x == (int)s) {
     const int2 r = D.seg[s];
     const int64_t id = level_base + (int64_t)D.cnt[s];
@@ -235,99 +244,16 @@ __global__ void k_head_setup(Dev D, int64_t level_base, int depth) {
         // size_t / float converts the count to float: a float division
         D.hcoef[s * 3 + a] = (double)__fdiv_rn((float)tries, __fsub_rn(hi[a], lo[a]));
       }
-      need = 9ull * (uint64_t)tries;
-    }
-  }
-  D.cnt2[s] = need;
-}
-
-__global__ void k_bucket_init(Dev D) {
-  const int64_t total = (int64_t)D.cnt2[D.n];
-  for (int64_t i = (int64_t)blockIdx.x * kB + threadIdx.x; i < total; i += (int64_t)gridDim.x * kB) {
-    uint32_t *r = D.buckets + i * 7;
-    r[0] = r[1] = r[2] = 0xFFFFFFFFu;
-    r[3] = r[4] = r[5] = 0u;
-    r[6] = 0u;
-  }
-}
-
-// Adds a box to bucket idx (-1: none) for the lanes that reach this call
-// together: lanes adding to the same bucket are merged first, one atomic
-// per bucket and key (NaN coordinates take no part, as in the reference's
-// min / max).
-__device__ __forceinline__ void bucket_add_grouped(uint32_t *buckets, int64_t idx, const float *lo, const float *hi) {
-  const unsigned grp = __match_any_sync(__activemask(), idx);
-  if (idx < 0) return;
-  uint32_t kl[3], kh[3];
-  for (int c = 0; c < 3; ++c) {
-    kl[c] = __reduce_min_sync(grp, isnan(lo[c]) ? 0xFFFFFFFFu : okey(lo[c]));
-    kh[c] = __reduce_max_sync(grp, isnan(hi[c]) ? 0u : okey(hi[c]));
-  }
-  if ((threadIdx.x & 31) != __ffs(grp) - 1) return;
-  uint32_t *r = buckets + idx * 7;
-  for (int c = 0; c < 3; ++c) {
-    if (kl[c] != 0xFFFFFFFFu) atomicMin(r + c, kl[c]);
-    if (kh[c] != 0u) atomicMax(r + 3 + c, kh[c]);
-  }
-  atomicAdd(r + 6, (uint32_t)__popc(grp));
-}
-
-// The buckets of every internal node (_DetermineBestSplit, :531-565): per
-// axis not split through the middle on the path, a triangle's box goes to
-// the right bucket of its first candidate plane, the left one of its last,
-// and the middle ones of the planes it straddles.
-__global__ void k_bucket_fill(Dev D) {
-  const int64_t s = (int64_t)blockIdx.x * kB + threadIdx.x;
-  if (s >= D.n) return;
-  const int b = D.seg[s].x;
-  if (b < 0 || D.hleaf[b]) return;
-  const unsigned mask = D.smask[s];
-  const uint64_t tries = (uint64_t)D.htries[b];
-  const int64_t base = (int64_t)D.cnt2[b];
-  float lo[3], hi[3];
-  for (int c = 0; c < 3; ++c) {
-    lo[c] = D.box[s * 6 + c];
-    hi[c] = D.box[s * 6 + 3 + c];
-  }
-  for (int a = 0; a < 3; ++a) {
-    if (mask & (1u << a)) continue;
-    const float nlo = D.hbox[(int64_t)b * 6 + a];
-    const double coef = D.hcoef[(int64_t)b * 3 + a];
-    const float dmax = __fsub_rn(hi[a], nlo), dmin = __fsub_rn(lo[a], nlo);
-    const uint64_t lefts_begin = min(tries, cast_size(__dadd_rn(__dmul_rn((double)dmax, coef), 1.0)));
-    const uint64_t rights_end = min(tries, cast_size(__dadd_rn(__dmul_rn((double)dmin, coef), 1.0)));
-    const int64_t lb = base + (int64_t)(a * 3) * (int64_t)tries;  // bucket index of L[0]
-    bucket_add_grouped(D.buckets, rights_end > 0 ? lb + 2 * (int64_t)tries + (int64_t)(rights_end - 1) : -1, lo, hi);
-    bucket_add_grouped(D.buckets, lefts_begin < tries ? lb + (int64_t)lefts_begin : -1, lo, hi);
-    // the middle buckets: the lanes of one node walk the union of their
-    // ranges together, one merged add per bucket
-    uint32_t *M = D.buckets + (lb + (int64_t)tries) * 7;
-    const unsigned grp = __match_any_sync(__activemask(), b);
-    const bool any = rights_end < lefts_begin;
-    const uint32_t jlo = __reduce_min_sync(grp, any ? (uint32_t)rights_end : 0xFFFFFFFFu);
-    const uint32_t jhi = __reduce_max_sync(grp, any ? (uint32_t)lefts_begin : 0u);
-    uint32_t kl[3], kh[3];
-    for (int c = 0; c < 3; ++c) {
-      kl[c] = isnan(lo[c]) ? 0xFFFFFFFFu : okey(lo[c]);
-      kh[c] = isnan(hi[c]) ? 0u : okey(hi[c]);
-    }
-    const bool leader = (threadIdx.x & 31) == __ffs(grp) - 1;
-    for (uint32_t j = jlo; j < jhi; ++j) {
-      const bool in = rights_end <= j && j < lefts_begin;
-      const unsigned who = __ballot_sync(grp, in);
-      if (who == 0u) continue;
-      uint32_t ml[3], mh[3];
-      for (int c = 0; c < 3; ++c) {
-        ml[c] = __reduce_min_sync(grp, in ? kl[c] : 0xFFFFFFFFu);
-        mh[c] = __reduce_max_sync(grp, in ? kh[c] : 0u);
-      }
-      if (leader) {
-        uint32_t *r = M + (int64_t)j * 7;
-        for (int c = 0; c < 3; ++c) {
-          if (ml[c] != 0xFFFFFFFFu) atomicMin(r + c, ml[c]);
-          if (mh[c] != 0u) atomicMax(r + 3 + c, mh[c]);
-        }
-        atomicAdd(r + 6, (uint32_t)__popc(who));
+      if (count <= kSmall) {
+        D.small[atomicAdd(D.count, 1)] = (uint32_t)s;
+      } else if (count <= kMid) {
+        D.mid[atomicAdd(D.count + 1, 1)] = (uint32_t)s;
+      } else {
+        const int k = atomicAdd(D.count + 2, 1), nc = (count + kMid - 1) / kMid;
+        D.big[k] = (uint32_t)s;
+        D.hbase[s] = k * 9 * kTries;
+        const int c0 = atomicAdd(D.count + 3, nc);
+        for (int c = 0; c < nc; ++c) D.chunks[c0 + c] = make_uint2((uint32_t)s, (uint32_t)c);
       }
     }
   }
@@ -383,31 +309,217 @@ __device__ __forceinline__ BoxN box_shfl_down(const BoxN &a, int o) {
   return b;
 }
 
-// One axis of one node's split search (_DetermineBestSplit, :566-608),
-// one warp: lane l takes a contiguous slice of the candidate planes.  The
-// right buckets' suffix unions and the left buckets' prefix unions come
-// from warp scans of the slices' unions; each lane then walks its slice
-// (the right suffixes stored back in place), computing the cost
-// sum(n_child * area_child / area_node) in the reference's double
-// arithmetic with the 0.8 bonus for an empty side; the first strict
-// minimum over all planes is the smallest (cost, plane) pair.
-__global__ void k_score(Dev D, int64_t level_nodes) {
-  const int64_t w = ((int64_t)blockIdx.x * kB + threadIdx.x) >> 5;
-  const int lane = threadIdx.x & 31;
-  if (w >= 3 * level_nodes) return;  // whole warps
-  const int64_t node = w / 3;
-  const int a = (int)(w - 3 * node);
-  const int64_t s = D.heads[node];
-  if (D.hleaf[s]) return;
-  if (D.smask[s] & (1u << a)) {
-    if (lane == 0) {
-      D.bcost[3 * s + a] = INFINITY;
-      D.bpos[3 * s + a] = 0.0;
-    }
-    return;
+// min(tries, (size_t)((double)d * coef + 1.0)) (_DetermineBestSplit, :536-540).
+// coef is a float, so the product is exact in double; in float the fused
+// multiply-add is the correctly rounded sum, and where that is not within its
+// rounding of a whole number both have the same whole part.
+__device__ __forceinline__ int plane_of(float d, double coef, int tries) {
+  const float v = fmaf(d, (float)coef, 1.0f);
+  if (v >= 1.0f && v < 4194304.0f && fabsf(v - rintf(v)) > v * 2.4e-7f) return min(tries, (int)v);
+  return (int)min((uint64_t)tries, cast_size(__dadd_rn(__dmul_rn((double)d, coef), 1.0)));
+}
+
+// The cost of a plane, sum(n_child * area_child / area_node) with the 0.8
+// bonus for an empty side, in the reference's double arithmetic.
+__device__ __forceinline__ double plane_cost(const BoxN &l, const BoxN &m, const BoxN &r, double inv_area) {
+  const double p1 = min1(__dmul_rn(area_d(l.lo, l.hi), inv_area));
+  const double p2 = min1(__dmul_rn(area_d(m.lo, m.hi), inv_area));
+  const double p3 = min1(__dmul_rn(area_d(r.lo, r.hi), inv_area));
+  const double cost =
+      __dadd_rn(__dadd_rn(__dmul_rn((double)l.n, p1), __dmul_rn((double)m.n, p2)), __dmul_rn((double)r.n, p3));
+  return l.n == 0 || r.n == 0 ? __dmul_rn(cost, 0.8) : cost;
+}
+// The same in float: all terms are positive, so it is within 20u of the
+// double cost (u = 2^-24) unless an area underflows or is not finite; lo / hi
+// bound the double cost (-inf / +inf where that is not certain).
+__device__ __forceinline__ void plane_cost_bounds(const BoxN &l, const BoxN &m, const BoxN &r, float inv_area,
+                                                  float &lo, float &hi) {
+  const BoxN *b[3] = {&l, &m, &r};
+  float cost = 0.0f;
+  bool sure = true;
+#pragma unroll
+  for (int k = 0; k < 3; ++k) {
+    if (b[k]->n == 0u) continue;  // an empty box counts 0 * 1
+    const float a = area_f(b[k]->lo, b[k]->hi), v = a * inv_area;
+    sure = sure && a > 1e-30f && a < 1e30f;
+    cost += (float)b[k]->n * (v < 1.0f ? v : 1.0f);
   }
+  if (l.n == 0u || r.n == 0u) cost *= 0.8f;
+  sure = sure && inv_area > 1e-30f && inv_area < 1e30f;
+  lo = sure ? cost * (1.0f - 1.3e-6f) : -INFINITY;
+  hi = sure ? cost * (1.0f + 1.3e-6f) : INFINITY;
+}
+
+// The least (cost, plane) of a warp.
+__device__ __forceinline__ void warp_least(double &cost, int &plane) {
+  for (int o = 16; o > 0; o >>= 1) {
+    const double oc = __shfl_xor_sync(0xffffffffu, cost, o);
+    const int oi = __shfl_xor_sync(0xffffffffu, plane, o);
+    if (oc < cost || (oc == cost && oi < plane)) {
+      cost = oc;
+      plane = oi;
+    }
+  }
+}
+__device__ __forceinline__ float warp_min(float v) {
+  for (int o = 16; o > 0; o >>= 1) v = fminf(v, __shfl_xor_sync(0xffffffffu, v, o));
+  return v;
+}
+
+// min + i * (max - min) / tries, evaluated in float; 0 where no plane has a
+// finite cost.
+__device__ __forceinline__ double plane_position(int i, float nlo, float nhi, int tries) {
+  if (i >= tries) return 0.0;
+  const float ext = __fsub_rn(nhi, nlo);
+  return (double)__fadd_rn(nlo, __fdiv_rn(__fmul_rn((float)i, ext), (float)tries));
+}
+
+// The split search of a node of at most 32 triangles, one warp: the boxes and
+// their first / last planes wait in shared memory, every lane unites the
+// boxes on the two sides of its plane (lane + 32 in a second round) and across
+// it.  Every (node, axis) is bound by these 32 n updates; the double costs are
+// made for a round only if one of its planes could still be the least.
+// (1,098,576 triangles: all split searches of the build: bucket fill, init and scores 18.8 -> 6.3 ms with the other two.)
+constexpr int kSmallWarps = 4;
+__global__ void __launch_bounds__(kSmallWarps * 32) k_split_small(Dev D) {
+  __shared__ float4 s_lo[kSmallWarps][32], s_hi[kSmallWarps][32];
+  const int lane = threadIdx.x & 31, wi = threadIdx.x >> 5;
+  const int64_t w = (int64_t)blockIdx.x * kSmallWarps + wi;
+  if (w >= D.count[0]) return;  // whole warps
+  const int64_t b = D.small[w];
+  const int n = D.seg[b].y - (int)b, tries = D.htries[b];
+  const unsigned mask = D.smask[b];
+  float lo[3] = {0.0f, 0.0f, 0.0f}, hi[3] = {0.0f, 0.0f, 0.0f}, nlo[3], nhi[3];
+  for (int c = 0; c < 3; ++c) {
+    if (lane < n) {
+      lo[c] = D.box[(b + lane) * 6 + c];
+      hi[c] = D.box[(b + lane) * 6 + 3 + c];
+    }
+    nlo[c] = D.hbox[b * 6 + c];
+    nhi[c] = D.hbox[b * 6 + 3 + c];
+  }
+  const float area = area_f(nlo, nhi), inv_f = 1.0f / area;
+  const double inv_area = __ddiv_rn(1.0, (double)area);
+  double best = INFINITY;
+  int bi = 0x7FFFFFFF, ba = 0;
+  for (int a = 0; a < 3; ++a) {
+    if (mask & (1u << a)) continue;
+    const double coef = D.hcoef[b * 3 + a];
+    int first = 0, last = 0;  // planes >= first have the box on their left, planes < last on their right
+    if (lane < n) {
+      first = plane_of(__fsub_rn(hi[a], nlo[a]), coef, tries);
+      last = plane_of(__fsub_rn(lo[a], nlo[a]), coef, tries);
+    }
+    __syncwarp();
+    s_lo[wi][lane] = make_float4(lo[0], lo[1], lo[2], __int_as_float(first));
+    s_hi[wi][lane] = make_float4(hi[0], hi[1], hi[2], __int_as_float(last));
+    __syncwarp();
+    for (int i0 = 0; i0 < tries; i0 += 32) {
+      const int i = i0 + lane;
+      BoxN L = box_empty(), M = box_empty(), R = box_empty();
+      for (int t = 0; t < n; ++t) {
+        const float4 p = s_lo[wi][t], q = s_hi[wi][t];
+        BoxN x;
+        x.lo[0] = p.x, x.lo[1] = p.y, x.lo[2] = p.z;
+        x.hi[0] = q.x, x.hi[1] = q.y, x.hi[2] = q.z;
+        x.n = 1u;
+        if (i >= __float_as_int(p.w)) box_unite(L, x);
+        else if (i < __float_as_int(q.w)) box_unite(R, x);
+        else box_unite(M, x);
+      }
+      float cl = INFINITY, ch = INFINITY;
+      if (i < tries) plane_cost_bounds(L, M, R, inv_f, cl, ch);
+      const float least = fminf(warp_min(ch), __double2float_ru(best));
+      if (__ballot_sync(0xffffffffu, cl <= least) == 0u) continue;
+      double cost = INFINITY;
+      int plane = 0x7FFFFFFF;
+      if (i < tries && cl <= least) {
+        const double c = plane_cost(L, M, R, inv_area);
+        if (c < INFINITY) {
+          cost = c;
+          plane = i;
+        }
+      }
+      warp_least(cost, plane);
+      if (cost < best) {
+        best = cost;
+        bi = plane;
+        ba = a;
+      }
+    }
+  }
+  if (lane == 0) {
+    D.haxis[b] = ba;
+    D.hsplit[b] = plane_position(bi, nlo[ba], nhi[ba], tries);
+    D.rflags[D.hid[b]] = (uint8_t)(ba + 1);
+  }
+}
+
+// Adds triangle boxes to the buckets of one axis in shared memory (L at
+// 0, M at tries, R at 2 tries, 7 words each): a box goes to the right bucket
+// of its first candidate plane, the left one of its last, and the middle ones
+// of the planes it straddles (NaN coordinates take no part, as in the
+// reference's min / max).
+__device__ __forceinline__ void bucket_add(uint32_t *r, const uint32_t *kl, const uint32_t *kh) {
+#pragma unroll
+  for (int c = 0; c < 3; ++c) {
+    if (kl[c] < r[c]) atomicMin(r + c, kl[c]);  // (a stale read only costs the atomic)
+    if (kh[c] > r[3 + c]) atomicMax(r + 3 + c, kh[c]);
+  }
+  atomicAdd(r + 6, 1u);
+}
+__device__ __forceinline__ void fill_buckets(const Dev &D, uint32_t *sb, int64_t b, int64_t s0, int64_t s1, int a,
+                                             int tries) {
+  for (int i = threadIdx.x; i < 21 * tries; i += blockDim.x) {
+    const int k = i % 7;
+    sb[i] = k < 3 ? 0xFFFFFFFFu : 0u;
+  }
+  __syncthreads();
+  const float nlo = D.hbox[b * 6 + a];
+  const double coef = D.hcoef[b * 3 + a];
+  for (int64_t s = s0 + threadIdx.x; s < s1; s += blockDim.x) {
+    float lo[3], hi[3];
+    uint32_t kl[3], kh[3];
+    for (int c = 0; c < 3; ++c) {
+      lo[c] = D.box[s * 6 + c];
+      hi[c] = D.box[s * 6 + 3 + c];
+      kl[c] = isnan(lo[c]) ? 0xFFFFFFFFu : okey(lo[c]);
+      kh[c] = isnan(hi[c]) ? 0u : okey(hi[c]);
+    }
+    const int lefts_begin = plane_of(__fsub_rn(hi[a], nlo), coef, tries);
+    const int rights_end = plane_of(__fsub_rn(lo[a], nlo), coef, tries);
+    if (rights_end > 0) bucket_add(sb + 7 * (2 * tries + rights_end - 1), kl, kh);
+    if (lefts_begin < tries) bucket_add(sb + 7 * lefts_begin, kl, kh);
+    for (int j = rights_end; j < lefts_begin; ++j) bucket_add(sb + 7 * (tries + j), kl, kh);
+  }
+  __syncthreads();
+}
+
+// One axis of one node's split search over its filled buckets
+// (_DetermineBestSplit, :566-608), one warp: lane l takes a contiguous slice
+// of the candidate planes.  The right buckets' suffix unions and the left
+// buckets' prefix unions come from warp scans of the slices' unions and are
+// stored back in place, decoded; then the costs: the float ones first, the
+// double ones of the planes that could be the least.
+__device__ __forceinline__ void store_box(uint32_t *r, const BoxN &b) {
+  for (int c = 0; c < 3; ++c) {
+    r[c] = __float_as_uint(b.lo[c]);
+    r[3 + c] = __float_as_uint(b.hi[c]);
+  }
+  r[6] = b.n;
+}
+__device__ __forceinline__ BoxN load_box(const uint32_t *r) {
+  BoxN b;
+  for (int c = 0; c < 3; ++c) {
+    b.lo[c] = __uint_as_float(r[c]);
+    b.hi[c] = __uint_as_float(r[3 + c]);
+  }
+  b.n = r[6];
+  return b;
+}
+__device__ __forceinline__ void score_axis(const Dev &D, int64_t s, int a, uint32_t *L) {
+  const int lane = threadIdx.x & 31;
   const int tries = D.htries[s];
-  uint32_t *L = D.buckets + ((int64_t)D.cnt2[s] + (int64_t)(a * 3) * tries) * 7;
   uint32_t *M = L + (int64_t)tries * 7, *R = M + (int64_t)tries * 7;
   const int per = (tries + 31) / 32, i0 = min(tries, lane * per), i1 = min(tries, i0 + per);
   BoxN ls = box_empty(), rs = box_empty();
@@ -424,64 +536,111 @@ __global__ void k_score(Dev D, int64_t level_nodes) {
   BoxN lp = box_shfl_up(ls, 1), rp = box_shfl_down(rs, 1);  // exclusive
   if (lane == 0) lp = box_empty();
   if (lane == 31) rp = box_empty();
-  // the right suffixes of the slice, stored back decoded
   for (int i = i1 - 1; i >= i0; --i) {
     uint32_t *r = R + (int64_t)i * 7;
     box_unite(rp, box_keys(r));
-    for (int c = 0; c < 3; ++c) {
-      r[c] = __float_as_uint(rp.lo[c]);
-      r[3 + c] = __float_as_uint(rp.hi[c]);
-    }
-    r[6] = rp.n;
+    store_box(r, rp);
   }
   const float *nlo = D.hbox + s * 6, *nhi = nlo + 3;
-  const double inv_area = __ddiv_rn(1.0, (double)area_f(nlo, nhi));
+  const float area = area_f(nlo, nhi), inv_f = 1.0f / area;
+  const double inv_area = __ddiv_rn(1.0, (double)area);
+  float least = INFINITY;
+  for (int i = i0; i < i1; ++i) {
+    uint32_t *l = L + (int64_t)i * 7;
+    box_unite(lp, box_keys(l));
+    store_box(l, lp);
+    float cl, ch;
+    plane_cost_bounds(lp, box_keys(M + (int64_t)i * 7), load_box(R + (int64_t)i * 7), inv_f, cl, ch);
+    least = fminf(least, ch);
+  }
+  least = warp_min(least);
   double best = INFINITY;
   int bi = 0x7FFFFFFF;
   for (int i = i0; i < i1; ++i) {
-    box_unite(lp, box_keys(L + (int64_t)i * 7));
-    const BoxN m = box_keys(M + (int64_t)i * 7);
-    const uint32_t *r = R + (int64_t)i * 7;
-    float sl[3], sh[3];
-    for (int c = 0; c < 3; ++c) {
-      sl[c] = __uint_as_float(r[c]);
-      sh[c] = __uint_as_float(r[3 + c]);
-    }
-    const uint32_t sn = r[6];
-    const double p1 = min1(__dmul_rn(area_d(lp.lo, lp.hi), inv_area));
-    const double p2 = min1(__dmul_rn(area_d(m.lo, m.hi), inv_area));
-    const double p3 = min1(__dmul_rn(area_d(sl, sh), inv_area));
-    double cost = __dadd_rn(__dadd_rn(__dmul_rn((double)lp.n, p1), __dmul_rn((double)m.n, p2)), __dmul_rn((double)sn, p3));
-    if (lp.n == 0 || sn == 0) cost = __dmul_rn(cost, 0.8);
-    if (cost < best) {
-      best = cost;
-      bi = i;
+    const BoxN l = load_box(L + (int64_t)i * 7), m = box_keys(M + (int64_t)i * 7), r = load_box(R + (int64_t)i * 7);
+    float cl, ch;
+    plane_cost_bounds(l, m, r, inv_f, cl, ch);
+    if (cl <= least) {
+      const double cost = plane_cost(l, m, r, inv_area);
+      if (cost < best) {
+        best = cost;
+        bi = i;
+      }
     }
   }
-  for (int o = 16; o > 0; o >>= 1) {
-    const double oc = __shfl_xor_sync(0xffffffffu, best, o);
-    const int oi = __shfl_xor_sync(0xffffffffu, bi, o);
-    if (oc < best || (oc == best && oi < bi)) {
-      best = oc;
-      bi = oi;
-    }
-  }
+  warp_least(best, bi);
   if (lane == 0) {
     D.bcost[3 * s + a] = best;
-    if (bi < tries) {
-      // min + i * (max - min) / tries, evaluated in float
-      const float ext = __fsub_rn(nhi[a], nlo[a]);
-      D.bpos[3 * s + a] = (double)__fadd_rn(nlo[a], __fdiv_rn(__fmul_rn((float)bi, ext), (float)tries));
-    } else {
-      D.bpos[3 * s + a] = 0.0;
-    }
+    D.bpos[3 * s + a] = plane_position(bi, nlo[a], nhi[a], tries);
   }
 }
 
-// The split axis: the lowest of the axes with the least cost.
+// A node of 33 to 4,096 triangles, one block per axis.
+__global__ void __launch_bounds__(128) k_split_mid(Dev D) {
+  __shared__ uint32_t sb[21 * kTries];
+  const int64_t k = blockIdx.x / 3u;
+  const int a = (int)(blockIdx.x % 3u);
+  if (k >= D.count[1]) return;
+  const int64_t b = D.mid[k];
+  if (D.smask[b] & (1u << a)) {
+    if (threadIdx.x == 0) {
+      D.bcost[3 * b + a] = INFINITY;
+      D.bpos[3 * b + a] = 0.0;
+    }
+    return;
+  }
+  fill_buckets(D, sb, b, b, D.seg[b].y, a, D.htries[b]);
+  if (threadIdx.x < 32) score_axis(D, b, a, sb);
+}
+
+// Larger nodes: their buckets emptied, filled chunk by chunk (the chunk's own
+// buckets merged into them) and searched.
+__global__ void k_big_init(Dev D) {
+  const int64_t total = (int64_t)D.count[2] * 9 * kTries * 7;
+  for (int64_t i = (int64_t)blockIdx.x * kB + threadIdx.x; i < total; i += (int64_t)gridDim.x * kB)
+    D.buckets[i] = i % 7 < 3 ? 0xFFFFFFFFu : 0u;
+}
+__global__ void __launch_bounds__(256) k_fill_big(Dev D) {
+  __shared__ uint32_t sb[21 * kTries];
+  const int64_t k = blockIdx.x / 3u;
+  const int a = (int)(blockIdx.x % 3u);
+  if (k >= D.count[3]) return;
+  const int64_t b = D.chunks[k].x, s0 = b + (int64_t)D.chunks[k].y * kMid;
+  if (D.smask[b] & (1u << a)) return;
+  fill_buckets(D, sb, b, s0, min((int64_t)D.seg[b].y, s0 + kMid), a, kTries);
+  uint32_t *g = D.buckets + ((int64_t)D.hbase[b] + (int64_t)a * 3 * kTries) * 7;
+  for (int i = threadIdx.x; i < 3 * kTries; i += blockDim.x) {
+    const uint32_t *r = sb + 7 * i;
+    if (r[6] == 0u) continue;
+    for (int c = 0; c < 3; ++c) {
+      atomicMin(g + 7 * i + c, r[c]);
+      atomicMax(g + 7 * i + 3 + c, r[3 + c]);
+    }
+    atomicAdd(g + 7 * i + 6, r[6]);
+  }
+}
+__global__ void __launch_bounds__(32) k_score_big(Dev D) {
+  const int64_t k = blockIdx.x / 3u;
+  const int a = (int)(blockIdx.x % 3u);
+  if (k >= D.count[2]) return;
+  const int64_t s = D.big[k];
+  if (D.smask[s] & (1u << a)) {
+    if (threadIdx.x == 0) {
+      D.bcost[3 * s + a] = INFINITY;
+      D.bpos[3 * s + a] = 0.0;
+    }
+    return;
+  }
+  score_axis(D, s, a, D.buckets + ((int64_t)D.hbase[s] + (int64_t)a * 3 * kTries) * 7);
+}
+
+// The split axis of the mid and big nodes: the lowest of the axes with the
+// least cost.
 __global__ void k_choose(Dev D) {
-  const int64_t s = (int64_t)blockIdx.x * kB + threadIdx.x;
-  if (s >= D.n || D.seg[s].x != (int)s || D.hleaf[s]) return;
+  const int64_t k = (int64_t)blockIdx.x * kB + threadIdx.x;
+  const int n_mid = D.count[1];
+  if (k >= (int64_t)n_mid + D.count[2]) return;
+  const int64_t s = k < n_mid ? D.mid[k] : D.big[k - n_mid];
   const double c0 = D.bcost[3 * s], c1 = D.bcost[3 * s + 1], c2 = D.bcost[3 * s + 2];
   int a;
   if (c0 <= c1 && c0 <= c2)
@@ -647,18 +806,26 @@ __global__ void k_jump_init(Dev D) {
   const uint32_t x = (uint32_t)p - (uint32_t)b;
   D.f0[p] = x < D.hnl[b] ? D.iarr[p] : x;
 }
+// Eight applications a round (253 rounds of two over a 1,098,576-triangle
+// build took 2.2 ms).
+constexpr int kJumps = 8;
 __global__ void k_jump(Dev D, const uint32_t *__restrict__ fin, uint32_t *__restrict__ fout) {
   const int64_t p = (int64_t)blockIdx.x * kB + threadIdx.x;
   if (p >= D.n) return;
   const int2 g = D.seg[p];
   if (g.x < 0 || D.hleaf[g.x]) return;
-  const uint32_t v = fin[p];
-  if (v >= (uint32_t)(g.y - g.x)) {  // only after an inconsistent step map
-    atomicOr(D.err, 4);
-    fout[p] = v;
-    return;
+  uint32_t v = fin[p];
+#pragma unroll
+  for (int k = 1; k < kJumps; ++k) {
+    if (v >= (uint32_t)(g.y - g.x)) {  // only after an inconsistent step map
+      atomicOr(D.err, 4);
+      break;
+    }
+    const uint32_t x = fin[(uint32_t)g.x + v];
+    if (x == v) break;
+    v = x;
   }
-  fout[p] = fin[(uint32_t)g.x + v];
+  fout[p] = v;
 }
 __global__ void k_dest_middle(Dev D, const uint32_t *__restrict__ f) {
   const int64_t p = (int64_t)blockIdx.x * kB + threadIdx.x;
@@ -754,8 +921,13 @@ cudaError_t build_accel_tree_gpu(const float *tbox, int64_t n, cudaStream_t st, 
   want(&D.hleaf, nn);
   want(&D.bcost, nn * 24);
   want(&D.bpos, nn * 24);
-  // buckets: sum over internal nodes of 9 min(200, 2 count) <= 18 n
-  want(&D.buckets, nn * 18 * 28);
+  want(&D.hbase, nn * 4);
+  want(&D.small, (nn / (kLeafMax + 1) + 1) * 4);
+  want(&D.mid, (nn / (kSmall + 1) + 1) * 4);
+  want(&D.big, (nn / (kMid + 1) + 1) * 4);
+  want(&D.chunks, (nn / kMid + nn / (kMid + 1) + 2) * 8);
+  want(&D.buckets, (nn / (kMid + 1) + 1) * 9 * kTries * 28);
+  want(&D.count, 256);
   want(&D.cls, nn);
   want(&D.cnt, n1 * 8);
   want(&D.cnt2, n1 * 8);
@@ -858,19 +1030,29 @@ cudaError_t build_accel_tree_gpu(const float *tbox, int64_t n, cudaStream_t st, 
     if ((e = cudaStreamSynchronize(st)) != cudaSuccess) break;
     const int64_t level_nodes = (int64_t)h_count[0];
     if (level_nodes == 0 || (uint32_t)h_count[1] != 0) break;
-    // a middle element's chain stays inside its node: 2^rounds >= its size
+    // a middle element's chain stays inside its node: kJumps^rounds >= its size
     const int64_t maxseg = (int64_t)(h_count[1] >> 32);
     int rounds = 1;
-    while (((int64_t)1 << rounds) < maxseg) ++rounds;
+    for (int64_t reach = kJumps; reach < maxseg; reach *= kJumps) ++rounds;
     if ((e = grow(n_nodes + level_nodes)) != cudaSuccess) break;
     k_node_box<<<gn, kB, 0, st>>>(D);
-    k_head_setup<<<gn1, kB, 0, st>>>(D, n_nodes, depth);
+    if ((e = cudaMemsetAsync(D.count, 0, 16, st)) != cudaSuccess) break;
+    k_head_setup<<<gn, kB, 0, st>>>(D, n_nodes, depth);
     n_nodes += level_nodes;
-    if ((e = scan64(D.cnt2, (int64_t)n1, D.sums, st)) != cudaSuccess) break;
-    k_bucket_init<<<4096, kB, 0, st>>>(D);
-    k_bucket_fill<<<gn, kB, 0, st>>>(D);
-    k_score<<<grid_of(3 * 32 * level_nodes), kB, 0, st>>>(D, level_nodes);
-    k_choose<<<gn, kB, 0, st>>>(D);
+    // at most this many nodes of each size; the kernels' blocks past the
+    // level's own numbers return at once
+    const int64_t most_mid = std::min(level_nodes, n / (kSmall + 1)), most_big = std::min(level_nodes, n / (kMid + 1));
+    const int64_t most_small = maxseg > kLeafMax ? std::min(level_nodes, n / (kLeafMax + 1)) : 0;
+    if (maxseg > kMid) {
+      k_big_init<<<512, kB, 0, st>>>(D);
+      k_fill_big<<<(unsigned)(3 * (n / kMid + most_big + 1)), 256, 0, st>>>(D);
+      k_score_big<<<(unsigned)(3 * most_big), 32, 0, st>>>(D);
+    }
+    if (maxseg > kSmall) {
+      if (most_mid > 0) k_split_mid<<<(unsigned)(3 * most_mid), 128, 0, st>>>(D);
+      if (most_mid + most_big > 0) k_choose<<<grid_of(most_mid + most_big), kB, 0, st>>>(D);
+    }
+    if (most_small > 0) k_split_small<<<(unsigned)((most_small + kSmallWarps - 1) / kSmallWarps), kSmallWarps * 32, 0, st>>>(D);
     k_classify<<<gn1, kB, 0, st>>>(D);
     if ((e = scan64(D.cnt, (int64_t)n1, D.sums, st)) != cudaSuccess) break;
     k_runs<<<gn, kB, 0, st>>>(D);
