@@ -52,6 +52,13 @@ cudaError_t launch_traversal_d(bool closest, int stack_cap, const void *nodes, c
 
 
 
+// A tree's normal ids on the device: uint16 per photon, then at nids_offset
+// the same normals as 4 floats each (launch_normals fills them from the ids;
+// dirs: direction_table_device()).
+__host__ __device__ inline size_t nids_offset(int64_t n) { return ((size_t)n * 2 + 255) & ~(size_t)255; }
+inline size_t nids_bytes(int64_t n) { return nids_offset(n) + (size_t)(n > 0 ? n : 1) * 16; }
+cudaError_t launch_normals(uint16_t *nids, int64_t n, const double *dirs, cudaStream_t st);
+
 // Photon kd-tree lookups (knn.cu).  nodes: KdNode[n]; nids: uint16 normal
 // id per node; dirs: direction_table_device() (3 doubles per 16-bit
 // direction id, then the same as 3 floats per id); q / qn: 3 doubles

@@ -26,7 +26,8 @@
 // multiply-add changes a result.
 //
 // Layout: 16-byte nodes (x, y, z, word) read with one vector load; the
-// photon normal ids (uint16) are read only for points inside the radius.
+// photons' normals (float4, behind their 16-bit ids) are read only for points
+// inside the radius.
 // The walk stack lives in shared memory; for k <= 128 the heap (8-byte
 // entries: float key, tree position) lives in local memory, larger k use a
 // heap in a caller-provided global scratch buffer of k entries per query.
@@ -35,6 +36,7 @@
 
 #include <cstdint>
 #include <mutex>
+#include <type_traits>
 
 #include "kernels.h"
 
@@ -59,17 +61,10 @@ namespace {
 #define SKW_KNN_BLOCK 32
 #endif
 constexpr int kKnnBlock = SKW_KNN_BLOCK;  // threads per block of the lookup kernels
-// Load the near child's node as soon as the node word is read, so that the
-// load overlaps the node's own distance, filter and heap work (off: at one
-// warp per block it measured slower, 42.4 against 32.7 ms, at 128 threads
-// the same).
-#ifndef SKW_KNN_EARLY
-#define SKW_KNN_EARLY 0
-#endif
-constexpr bool kEarlyLoad = SKW_KNN_EARLY != 0;
-// minimum resident blocks per SM of k_knn: 32 one-warp blocks bound its
-// registers at 64 (with 128-thread blocks, measured on the k = 100 photon
-// lookups: 72 registers 57 ms, 64 50.5 ms, 48 58.5 ms)
+// Minimum resident blocks per SM: 32 one-warp blocks bound the registers at
+// 64.  Heaps of more than 32 entries leave room for at most 28 blocks, at
+// k = 100 for 14, so that kernel is bound at 128 (k = 100, 669,824 queries:
+// 7.44 -> 7.29 ms).
 #ifndef SKW_KNN_MINB
 #define SKW_KNN_MINB (1024 / SKW_KNN_BLOCK)
 #endif
@@ -80,9 +75,8 @@ struct Query {
   double n[3];
   double cos_t, sin_t;
   bool filter;
-  float qf[3];  // q rounded to float
+  float qf[3];  // q rounded up to float
   float eq;     // max |q - qf| over the axes
-  bool qle[3];  // q <= qf on the axis (decides q <= split when split == qf)
   float nf[3];  // the normal in float (filter pre-test)
   float cos_f, sin_f;  // cos_t, sin_t in float (filter pre-test)
   float ke0, ke1;      // error bound of a float squared distance k: ke0 + ke1 k (key_err)
@@ -92,8 +86,7 @@ struct Query {
 __device__ __forceinline__ void query_float(Query &Q) {
   float e = 0.0f;
   for (int k = 0; k < 3; ++k) {
-    Q.qf[k] = (float)Q.q[k];
-    Q.qle[k] = Q.q[k] <= (double)Q.qf[k];
+    Q.qf[k] = __double2float_ru(Q.q[k]);
     e = fmaxf(e, (float)fabs(Q.q[k] - (double)Q.qf[k]));
     Q.nf[k] = (float)Q.n[k];
   }
@@ -113,12 +106,10 @@ __device__ __forceinline__ double q_at(const Query &Q, uint32_t a) {
   return a == 0 ? Q.q[0] : (a == 1 ? Q.q[1] : Q.q[2]);
 }
 
-// q[axis] <= split for a float split, exactly, without double arithmetic:
-// qf is the float nearest to q, so qf < split implies q < split and
-// qf > split implies q > split.
-__device__ __forceinline__ bool q_le_split(const Query &Q, uint32_t axis, float split) {
-  const float qf = qf_at(Q, axis);
-  return qf < split || (qf == split && (axis == 0 ? Q.qle[0] : (axis == 1 ? Q.qle[1] : Q.qle[2])));
+// The normals as floats, behind the ids (kernels.h, nids_bytes): one load per
+// accepted point instead of the id and then its entry in the 768 KB table.
+__device__ __forceinline__ const float4 *node_normals(const uint16_t *nids, int n) {
+  return reinterpret_cast<const float4 *>(reinterpret_cast<const char *>(nids) + nids_offset(n));
 }
 
 // PhotonFilter::operator() (PhotonInternalTypes.h:127-133), with float
@@ -127,11 +118,10 @@ __device__ __forceinline__ bool q_le_split(const Query &Q, uint32_t axis, float 
 // vectors: a few 1e-7), else in double as the reference computes them.
 __device__ __forceinline__ bool photon_filter_exact(const Query &Q, const float4 p, uint16_t nid,
                                                     const double *__restrict__ dirs);
-__device__ __forceinline__ bool photon_filter(const Query &Q, const float4 p, uint16_t nid,
-                                              const double *__restrict__ dirs) {
-  const float *dirs_f = reinterpret_cast<const float *>(dirs + (3 << 16));  // the table rounded to float
-  const float nx = __ldg(dirs_f + 3 * nid), ny = __ldg(dirs_f + 3 * nid + 1), nz = __ldg(dirs_f + 3 * nid + 2);
-  const float cf = nx * Q.nf[0] + ny * Q.nf[1] + nz * Q.nf[2];
+__device__ __forceinline__ bool photon_filter(const Query &Q, const float4 p, int i, const uint16_t *__restrict__ nids,
+                                              const float4 *__restrict__ nrm, const double *__restrict__ dirs) {
+  const float4 m = __ldg(nrm + i);
+  const float cf = m.x * Q.nf[0] + m.y * Q.nf[1] + m.z * Q.nf[2];
   const float ct = Q.cos_f;
   if (cf < ct - 2e-6f) return false;
   if (cf > ct + 2e-6f) {
@@ -149,7 +139,7 @@ __device__ __forceinline__ bool photon_filter(const Query &Q, const float4 p, ui
     if (lhs + err < rhs) return true;
     if (lhs - err > rhs) return false;
   }
-  return photon_filter_exact(Q, p, nid, dirs);
+  return photon_filter_exact(Q, p, __ldg(nids + i), dirs);
 }
 
 __device__ __forceinline__ bool photon_filter_exact(const Query &Q, const float4 p, uint16_t nid,
@@ -207,115 +197,77 @@ __device__ __forceinline__ void radius_thresholds(const Query &Q, float rlo, flo
 // A node's children in the reference's visit order: near = the child on the
 // query's side of the split (visited next), far = the other (postponed and
 // visited only if its plane is within the radius when it is popped); -1
-// where a child is absent or the node is a leaf.
+// where a child is absent or the node is a leaf.  q <= split is decided on
+// the float query: it is q rounded up, and split is a float.  s2: the plane's
+// squared distance in float (dist2f's bound holds for it).
 __device__ __forceinline__ void node_children(const float4 p, int cur, int n, const Query &Q, int &near, int &far,
-                                              uint32_t &axis, float &split) {
-  const uint32_t w = __float_as_uint(p.w);
+                                              float &s2) {
+  const uint32_t w = __float_as_uint(p.w), axis = w & 3u;
   near = far = -1;
-  axis = w & 3u;
-  split = 0.0f;
+  s2 = 0.0f;
   if (axis == 3u) return;
-  split = axis == 0 ? p.x : (axis == 1 ? p.y : p.z);
+  const float split = axis == 0 ? p.x : (axis == 1 ? p.y : p.z), q = qf_at(Q, axis), sd = q - split;
+  s2 = sd * sd;
   const uint32_t right = w >> 3;
-  const bool has_left = (w & 4u) != 0u, has_right = right < (uint32_t)n;
-  const bool le = q_le_split(Q, axis, split);
-  const int l = has_left ? cur + 1 : -1, r = has_right ? (int)right : -1;
+  const int l = (w & 4u) != 0u ? cur + 1 : -1, r = right < (uint32_t)n ? (int)right : -1;
+  const bool le = q <= split;
   near = le ? l : r;
   far = le ? r : l;
 }
 
-// Walks the tree in the reference's order, calling visit(ni, p, d2, maxd2)
-// for every point with d2 < maxd2; visit returns true when it changed
-// maxd2.  A point whose float distance is certainly inside the radius is
-// visited with d2 = -1 (not computed): the exact double distance is only
-// needed for the heap order, and the caller computes it later, many at a
-// time (the exact distance is a chain of dependent double operations, slow
-// on this GPU's FP64 pipe when done one point after another).  Returns
-// nodes visited (for statistics) or -1 on stack overflow.
-//
-// The stack lives in shared memory ([entry][thread], so lanes never share a
-// bank) and holds only the parent of each postponed far child: on pop the
-// parent is read again (a recently visited node, usually still in L1) and
+// The plane's test in double, as the reference's: (q - split)^2.
+__device__ __forceinline__ double plane_d2(const float4 p, const Query &Q) {
+  const uint32_t axis = __float_as_uint(p.w) & 3u;
+  const double pd = __dsub_rn(q_at(Q, axis), (double)(axis == 0 ? p.x : (axis == 1 ? p.y : p.z)));
+  return __dmul_rn(pd, pd);
+}
+
+// The search radius of a walk: max_dist^2 (KDTree::Lookup, KDTree.h:475-482)
+// until set() makes it the exact squared distance of a photon, of which only
+// a float bracket is kept; the exact double is computed when a decision needs
+// it.  tin / tout: radius_thresholds of the bracket.
+struct Radius {
+  double exact;
+  int idx;  // the photon (get's `ids`: its place there) at this distance; -1: `exact` holds it
+  float tin, tout;
+
+  __device__ __forceinline__ void start(const Query &Q, double max_dist) {
+    exact = __dmul_rn(max_dist, max_dist);
+    idx = -1;
+    radius_thresholds(Q, __double2float_rd(exact), __double2float_ru(exact), tin, tout);
+  }
+  // cut: how far `key` may be from the photon's, relative to itself
+  __device__ __forceinline__ void set(const Query &Q, int photon, float key, float cut) {
+    const float e = 1.0001f * fmaf(Q.ke1 + cut, key, Q.ke0);
+    idx = photon;
+    radius_thresholds(Q, __fsub_rd(key, e), __fadd_ru(key, e), tin, tout);
+  }
+  __device__ __forceinline__ double get(const float4 *__restrict__ nodes, const Query &Q,
+                                        const int32_t *ids = nullptr) {
+    if (idx >= 0) {
+      exact = point_d2(__ldg(nodes + (ids ? ids[idx] : idx)), Q);
+      idx = -1;
+    }
+    return exact;
+  }
+};
+
+// The walk stack lives in shared memory ([entry][thread], so lanes never
+// share a bank) and holds only the parent of each postponed far child: on pop
+// the parent is read again (a recently visited node, usually still in L1) and
 // its split gives both the far child and the plane distance to re-test.
 // Shared memory and L1 share the SM's storage, and the walk's node and heap
 // reads want the L1, so the stack is sized by the tree's depth: the
 // median-split tree of n points is floor(log2 n) + 1 levels deep and the
 // walk holds at most one entry per level, so S = 20 serves n < 2^20 and
 // S = 32 any n < 2^31.
-template <int S, class Visit>
-__device__ __forceinline__ int walk(const float4 *__restrict__ nodes, int n, const Query &Q, double &maxd2,
-                                    uint32_t (*stk)[kKnnBlock], Visit &&visit) {
-  if (n <= 0) return 0;
-  int sp = 0, visited = 0;
-  int cur = 0;
-  // maxd2 in float, rounded down / up (a float below the lower one is below
-  // maxd2, one at or above the upper one is not)
-  auto lo_f = [](double m) { return __double2float_rd(m); };
-  auto hi_f = [](double m) { return __double2float_ru(m); };
-  float tin, tout;
-  radius_thresholds(Q, lo_f(maxd2), hi_f(maxd2), tin, tout);
-  float4 p = __ldg(nodes);
-  for (;;) {
-    ++visited;
-    int near, far;
-    uint32_t axis;
-    float split;
-    node_children(p, cur, n, Q, near, far, axis, split);
-    float4 pn = p;
-    if (kEarlyLoad && near >= 0) pn = __ldg(nodes + near);  // overlaps this node's work
-    {
-      const float d2f = dist2f(p, Q);
-      if (d2f < tin) {  // certainly inside
-        if (visit(cur, p, -1.0, maxd2)) radius_thresholds(Q, lo_f(maxd2), hi_f(maxd2), tin, tout);
-      } else if (!(d2f >= tout)) {  // not certainly outside: decide exactly
-        const double d2 = point_d2(p, Q);
-        if (d2 < maxd2 && visit(cur, p, d2, maxd2)) radius_thresholds(Q, lo_f(maxd2), hi_f(maxd2), tin, tout);
-      }
-    }
-    if (far >= 0) {  // the far child waits on the stack
-      if (sp >= S) return -1;
-      stk[sp][threadIdx.x] = (uint32_t)cur;
-      ++sp;
-    }
-    if (near >= 0) {
-      cur = near;
-      p = kEarlyLoad ? pn : __ldg(nodes + near);
-      continue;
-    }
-    int next = -1;
-    while (sp > 0) {
-      --sp;
-      // the reference's pop test: (qa - split)^2 < maxd2, in double
-      const uint32_t par = stk[sp][threadIdx.x];
-      int pnear, pfar;
-      uint32_t ax;
-      float ps;
-      const float4 pp = __ldg(nodes + par);
-      node_children(pp, (int)par, n, Q, pnear, pfar, ax, ps);
-      const float sd = qf_at(Q, ax) - ps, s2 = sd * sd;
-      bool take;
-      if (s2 < tin) {
-        take = true;
-      } else if (s2 >= tout) {
-        take = false;
-      } else {
-        const double pd = __dsub_rn(q_at(Q, ax), (double)ps);
-        take = __dmul_rn(pd, pd) < maxd2;
-      }
-      if (take) {
-        next = pfar;
-        break;
-      }
-    }
-    if (next < 0) return visited;
-    cur = next;
-    p = __ldg(nodes + cur);
-  }
-}
 
 // ------------------------------------------------------------ k_knn --
 // The heap holds float squared distances: an entry's key is the float
-// distance of its point, within key_err of the reference's double value.
+// distance of its point (dist2f), within ke0 + ke1 key of the reference's
+// double value (Query::ke0, ke1): that bounds the error derived above,
+// 5u D + 2 sqrt(3) eq sqrt(D) + 3 eq^2, the square-root term by
+// 2 sqrt(3) eq sqrt(key) <= 2 sqrt(1.001 eq * 3.003 eq key) <= 1.001 eq + 3.003 eq key.
 // Heap comparisons are decided on the keys and their bounds, and only when
 // two keys' intervals overlap are the exact doubles of both points computed
 // (GB300 runs a double operation at ~1/64 of the float rate, and divergent
@@ -336,12 +288,6 @@ struct FCand {
 
 // Entries per query of a global heap: k + 1 rounded up to even.
 __host__ __device__ __forceinline__ int64_t knn_heap_stride(int k) { return ((int64_t)k + 2) & ~(int64_t)1; }
-
-// Bound on |key - d2| for a point whose float squared distance is key
-// (dist2f): ke0 + ke1 key (Query::ke0, ke1) bounds the error derived
-// above, 5u D + 2 sqrt(3) eq sqrt(D) + 3 eq^2, the square-root term by
-// 2 sqrt(3) eq sqrt(key) <= 2 sqrt(1.001 eq * 3.003 eq key) <= 1.001 eq + 3.003 eq key.
-__device__ __forceinline__ float key_err(const Query &Q, float key) { return fmaf(Q.ke1, key, Q.ke0); }
 
 // (d2, idx) lexicographic on the exact distances, decided on the keys when
 // their bounds do not overlap.
@@ -401,25 +347,8 @@ __device__ __forceinline__ void fheap_make(const float4 *__restrict__ nodes, con
   }
 }
 
-// KMAX > 0: heap of KMAX entries in local memory.  KMAX == 0: the heap of
-// query i is scratch[i * k ...].  Until the heap is full its entries are
-// the accepted points in visit order (the reference's array holds them
-// unordered); at k entries it becomes a heap.
-template <int KMAX, int S>
-__global__ void __launch_bounds__(kKnnBlock, SKW_KNN_MINB) k_knn(const float4 *__restrict__ nodes, const uint16_t *__restrict__ nids,
-                                             const double *__restrict__ dirs, int n, const double *__restrict__ q,
-                                             const double *__restrict__ qn, int64_t nq, int k, double max_dist,
-                                             double cos_t, int32_t *__restrict__ out_idx,
-                                             double *__restrict__ out_d2, int32_t *__restrict__ out_count,
-                                             int32_t *__restrict__ out_visited, FCand *__restrict__ scratch,
-                                             unsigned *__restrict__ status, const int *__restrict__ nq_dev,
-                                             const int32_t *__restrict__ order) {
-  __shared__ uint32_t stk[S][kKnnBlock];
-  int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (nq_dev && *nq_dev < nq) nq = *nq_dev;
-  if (i >= nq) return;
-  if (order) i = order[i];
-  Query Q;
+__device__ __forceinline__ void load_query(Query &Q, const double *__restrict__ q, const double *__restrict__ qn,
+                                           int64_t i, double cos_t) {
   Q.q[0] = q[3 * i];
   Q.q[1] = q[3 * i + 1];
   Q.q[2] = q[3 * i + 2];
@@ -435,75 +364,178 @@ __global__ void __launch_bounds__(kKnnBlock, SKW_KNN_MINB) k_knn(const float4 *_
     Q.cos_t = Q.sin_t = 0.0;
   }
   query_float(Q);
-  FCand local_heap[KMAX > 0 ? KMAX : 1];
-  // global heaps: query i's entries from scratch[i * stride + 1], stride even
-  // (16-byte aligned sibling pairs, fheap_adjust<true>)
-  FCand *heap = KMAX > 0 ? local_heap : scratch + i * (int64_t)knn_heap_stride(k) + 1;
+}
+
+// The two heaps of k_knn.  Until a heap is full its entries are the accepted
+// points in visit order (the reference's array holds them unordered); at k
+// entries it becomes a heap.  add(): the i-th point of those; make(): the heap
+// of the first k; replace(): pop_heap (the top goes to the back, the back's
+// old value is re-placed), then the point pushed up from the back; top(): the
+// top as the search radius.
+
+// Heaps in a global scratch buffer (k > 128, and skw_knn_noalloc): query i's
+// entries from scratch[i * stride + 1], stride even (16-byte aligned sibling
+// pairs, fheap_adjust<true>).
+struct GlobalHeap {
+  FCand *h;
+  __device__ __forceinline__ void add(int i, float key, int32_t photon) { h[i] = FCand{key, photon}; }
+  __device__ __forceinline__ void make(const float4 *__restrict__ nodes, const Query &Q, int k) {
+    fheap_make(nodes, Q, h, k);
+  }
+  __device__ __forceinline__ void replace(const float4 *__restrict__ nodes, const Query &Q, int k, float key,
+                                          int32_t photon) {
+    const FCand back = h[k - 1];
+    h[k - 1] = h[0];
+    fheap_adjust<true>(nodes, Q, h, 0, k - 1, back);
+    fheap_push_up(nodes, Q, h, k - 1, 0, FCand{key, photon});
+  }
+  __device__ __forceinline__ int32_t photon(int i) const { return h[i].idx; }
+  __device__ __forceinline__ void top(const Query &Q, Radius &r) const { r.set(Q, h[0].idx, h[0].key, 0.0f); }
+};
+
+// Heaps in shared memory (k <= 128), one word per entry: the key with its low
+// 7 bits replaced by the entry's slot, the place in `ids` that holds its tree
+// position.  A heap operation moves words only -- two loads and a store per
+// level, [entry][thread] so that lanes never share a bank -- and a photon's
+// position is written once, into local memory.  The word is compared as the
+// float it is, within 2^-16 of the photon's key, which joins the error bounds:
+// two keys that close are compared in double.  What bounds the lookup is the
+// latency of its chains of moves and node reads at 14 warps per SM (ncu: issue
+// 34 %): the k = 100 lookups of 669,824 queries took 9.91 ms with 8-byte
+// entries in local memory (1 KB per query, which L1 cannot hold) and took 9.17
+// ms here; 7.64 ms with far children dropped at the push when their plane is
+// outside by then, 7.29 ms with the normals read in one load.
+struct SharedHeap {
+  static constexpr uint32_t kSlot = 127u;
+  static constexpr float kCut = 1.5262e-5f;  // 128 units in the last place: 2^-16, rounded up
+  uint32_t *h;                               // entry i of this thread: h[i * kKnnBlock]
+  int32_t *ids;
+  __device__ __forceinline__ uint32_t at(int i) const { return h[i * kKnnBlock]; }
+  __device__ __forceinline__ void put(int i, uint32_t v) { h[i * kKnnBlock] = v; }
+  static __device__ __forceinline__ uint32_t entry(float key, uint32_t slot) {
+    return (__float_as_uint(key) & ~kSlot) | slot;
+  }
+  // as fcand_less
+  __device__ __forceinline__ bool less(const float4 *__restrict__ nodes, const Query &Q, uint32_t a, uint32_t b) const {
+    const float ka = __uint_as_float(a), kb = __uint_as_float(b), d = ka - kb;
+    const float tol = 1.0001f * fmaf(Q.ke1 + kCut, ka + kb, 2.0f * Q.ke0);
+    if (d < -tol) return true;
+    if (d > tol) return false;
+    const int32_t ia = ids[a & kSlot], ib = ids[b & kSlot];
+    const double da = point_d2(__ldg(nodes + ia), Q), db = point_d2(__ldg(nodes + ib), Q);
+    return da == db ? ia < ib : da < db;
+  }
+  __device__ __forceinline__ void push_up(const float4 *__restrict__ nodes, const Query &Q, int hole, int top,
+                                          uint32_t value) {
+    int parent = (hole - 1) / 2;
+    while (hole > top) {
+      const uint32_t p = at(parent);
+      if (!less(nodes, Q, p, value)) break;
+      put(hole, p);
+      hole = parent;
+      parent = (hole - 1) / 2;
+    }
+    put(hole, value);
+  }
+  __device__ __forceinline__ void adjust(const float4 *__restrict__ nodes, const Query &Q, int hole, int len,
+                                         uint32_t value) {
+    const int top = hole;
+    int second = hole;
+    while (second < (len - 1) / 2) {
+      second = 2 * (second + 1);
+      const uint32_t a = at(second - 1), b = at(second);
+      const bool left = less(nodes, Q, b, a);
+      second -= left ? 1 : 0;
+      put(hole, left ? a : b);
+      hole = second;
+    }
+    if ((len & 1) == 0 && second == (len - 2) / 2) {
+      second = 2 * (second + 1);
+      put(hole, at(second - 1));
+      hole = second - 1;
+    }
+    push_up(nodes, Q, hole, top, value);
+  }
+  __device__ __forceinline__ void add(int i, float key, int32_t photon) {
+    ids[i] = photon;
+    put(i, entry(key, (uint32_t)i));
+  }
+  __device__ __forceinline__ void make(const float4 *__restrict__ nodes, const Query &Q, int k) {
+    for (int parent = (k - 2) / 2; parent >= 0 && k >= 2; --parent) adjust(nodes, Q, parent, k, at(parent));
+  }
+  __device__ __forceinline__ void replace(const float4 *__restrict__ nodes, const Query &Q, int k, float key,
+                                          int32_t photon) {
+    const uint32_t back = at(k - 1), top = at(0);
+    put(k - 1, top);
+    adjust(nodes, Q, 0, k - 1, back);
+    ids[top & kSlot] = photon;
+    push_up(nodes, Q, k - 1, 0, entry(key, top & kSlot));
+  }
+  __device__ __forceinline__ int32_t photon(int i) const { return ids[at(i) & kSlot]; }
+  __device__ __forceinline__ void top(const Query &Q, Radius &r) const {
+    const uint32_t t = at(0);
+    r.set(Q, (int)(t & kSlot), __uint_as_float(t), kCut);
+  }
+};
+
+// KMAX > 0: heaps of k <= KMAX entries in shared memory; KMAX == 0: global
+// heaps.
+template <int KMAX, int S>
+__global__ void __launch_bounds__(kKnnBlock, KMAX == 128 ? SKW_KNN_MINB / 2 : SKW_KNN_MINB) k_knn(const float4 *__restrict__ nodes, const uint16_t *__restrict__ nids,
+                                             const double *__restrict__ dirs, int n, const double *__restrict__ q,
+                                             const double *__restrict__ qn, int64_t nq, int k, double max_dist,
+                                             double cos_t, int32_t *__restrict__ out_idx,
+                                             double *__restrict__ out_d2, int32_t *__restrict__ out_count,
+                                             int32_t *__restrict__ out_visited, FCand *__restrict__ scratch,
+                                             unsigned *__restrict__ status, const int *__restrict__ nq_dev,
+                                             const int32_t *__restrict__ order, int per_warp) {
+  __shared__ uint32_t stk[S][kKnnBlock];
+  const int lane = threadIdx.x & 31;
+  if (lane >= per_warp) return;
+  int64_t i = ((int64_t)blockIdx.x * (kKnnBlock / 32) + (threadIdx.x >> 5)) * per_warp + lane;
+  if (nq_dev && *nq_dev < nq) nq = *nq_dev;
+  if (i >= nq) return;
+  if (order) i = order[i];
+  const float4 *nrm = node_normals(nids, n);
+  Query Q;
+  load_query(Q, q, qn, i, cos_t);
+  int32_t ids[KMAX > 0 ? KMAX : 1];
+  extern __shared__ uint32_t s_heap[];
+  typename std::conditional<(KMAX > 0), SharedHeap, GlobalHeap>::type heap = [&]() {
+    if constexpr (KMAX > 0) return SharedHeap{s_heap + threadIdx.x, ids};
+    else return GlobalHeap{scratch + i * (int64_t)knn_heap_stride(k) + 1};
+  }();
   int size = 0, visited = 0;
   if (k > 0 && n > 0) {
-    // the search radius: max_dist^2 (KDTree::Lookup, KDTree.h:475-482)
-    // until the heap is full, then the top's exact squared distance
-    double rex = __dmul_rn(max_dist, max_dist);
-    bool rex_ok = true;
-    float rlo = __double2float_rd(rex), rhi = __double2float_ru(rex), tin, tout;
-    radius_thresholds(Q, rlo, rhi, tin, tout);
-    auto radius = [&]() -> double {
-      if (!rex_ok) {
-        rex = point_d2(__ldg(nodes + heap[0].idx), Q);
-        rex_ok = true;
-      }
-      return rex;
-    };
-    auto new_top = [&]() {
-      const float t = heap[0].key, e = key_err(Q, t);
-      rlo = __fsub_rd(t, e);
-      rhi = __fadd_ru(t, e);
-      rex_ok = false;
-      radius_thresholds(Q, rlo, rhi, tin, tout);
-    };
+    Radius rad;  // max_dist until the heap is full, then its top
+    rad.start(Q, max_dist);
     int sp = 0, cur = 0;
     bool overflow = false;
     float4 p = __ldg(nodes);
     for (;;) {
       ++visited;
       int near, far;
-      uint32_t axis;
-      float split;
-      node_children(p, cur, n, Q, near, far, axis, split);
-      // the near child is visited next: its node is loaded now, so that the
-      // load overlaps this node's work
-      float4 pn = p;
-      if (kEarlyLoad && near >= 0) pn = __ldg(nodes + near);
+      float s2;
+      node_children(p, cur, n, Q, near, far, s2);
       {
         const float d2f = dist2f(p, Q);
-        bool inside;
-        if (d2f < tin) {
-          inside = true;
-        } else if (d2f >= tout) {
-          inside = false;
-        } else {
-          inside = point_d2(p, Q) < radius();
-        }
-        if (inside && (!Q.filter || photon_filter(Q, p, __ldg(nids + cur), dirs))) {
-          const FCand c{d2f, cur};
+        if ((d2f < rad.tin || (!(d2f >= rad.tout) && point_d2(p, Q) < rad.get(nodes, Q, KMAX > 0 ? ids : nullptr))) &&
+            (!Q.filter || photon_filter(Q, p, cur, nids, nrm, dirs))) {
           if (size < k) {
-            heap[size++] = c;
+            heap.add(size++, d2f, cur);
             if (size == k) {
-              fheap_make(nodes, Q, heap, k);
-              new_top();
+              heap.make(nodes, Q, k);
+              heap.top(Q, rad);
             }
           } else {
-            // pop_heap: the top goes to the back; the back's old value is re-placed
-            const FCand back = heap[k - 1];
-            heap[k - 1] = heap[0];
-            fheap_adjust<KMAX == 0>(nodes, Q, heap, 0, k - 1, back);
-            // the popped back slot takes the new point, pushed up
-            fheap_push_up(nodes, Q, heap, k - 1, 0, c);
-            new_top();
+            heap.replace(nodes, Q, k, d2f, cur);
+            heap.top(Q, rad);
           }
         }
       }
-      if (far >= 0) {  // the far child waits on the stack
+      // The far child waits on the stack, unless its plane is certainly outside
+      // already (the radius only shrinks, so it would be when popped).
+      if (far >= 0 && !(s2 >= rad.tout)) {
         if (sp >= S) {
           overflow = true;
           break;
@@ -513,7 +545,7 @@ __global__ void __launch_bounds__(kKnnBlock, SKW_KNN_MINB) k_knn(const float4 *_
       }
       if (near >= 0) {
         cur = near;
-        p = kEarlyLoad ? pn : __ldg(nodes + near);
+        p = __ldg(nodes + near);
         continue;
       }
       int next = -1;
@@ -522,21 +554,10 @@ __global__ void __launch_bounds__(kKnnBlock, SKW_KNN_MINB) k_knn(const float4 *_
         // the reference's pop test: (qa - split)^2 < radius, in double
         const uint32_t par = stk[sp][threadIdx.x];
         int pnear, pfar;
-        uint32_t ax;
-        float ps;
+        float ps2;
         const float4 pp = __ldg(nodes + par);
-        node_children(pp, (int)par, n, Q, pnear, pfar, ax, ps);
-        const float sd = qf_at(Q, ax) - ps, s2 = sd * sd;
-        bool take;
-        if (s2 < tin) {
-          take = true;
-        } else if (s2 >= tout) {
-          take = false;
-        } else {
-          const double pd = __dsub_rn(q_at(Q, ax), (double)ps);
-          take = __dmul_rn(pd, pd) < radius();
-        }
-        if (take) {
+        node_children(pp, (int)par, n, Q, pnear, pfar, ps2);
+        if (ps2 < rad.tin || (!(ps2 >= rad.tout) && plane_d2(pp, Q) < rad.get(nodes, Q, KMAX > 0 ? ids : nullptr))) {
           next = pfar;
           break;
         }
@@ -551,7 +572,7 @@ __global__ void __launch_bounds__(kKnnBlock, SKW_KNN_MINB) k_knn(const float4 *_
   // the exact squared distances of the output, four chains at a time
   int j = 0;
   for (; j + 4 <= size; j += 4) {
-    const int32_t a0 = heap[j].idx, a1 = heap[j + 1].idx, a2 = heap[j + 2].idx, a3 = heap[j + 3].idx;
+    const int32_t a0 = heap.photon(j), a1 = heap.photon(j + 1), a2 = heap.photon(j + 2), a3 = heap.photon(j + 3);
     const double d0 = point_d2(__ldg(nodes + a0), Q), d1 = point_d2(__ldg(nodes + a1), Q),
                  d2 = point_d2(__ldg(nodes + a2), Q), d3 = point_d2(__ldg(nodes + a3), Q);
     out_idx[i * k + j] = a0;
@@ -564,8 +585,9 @@ __global__ void __launch_bounds__(kKnnBlock, SKW_KNN_MINB) k_knn(const float4 *_
     out_d2[i * k + j + 3] = d3;
   }
   for (; j < size; ++j) {
-    out_idx[i * k + j] = heap[j].idx;
-    out_d2[i * k + j] = point_d2(__ldg(nodes + heap[j].idx), Q);
+    const int32_t a = heap.photon(j);
+    out_idx[i * k + j] = a;
+    out_d2[i * k + j] = point_d2(__ldg(nodes + a), Q);
   }
   for (; j < k; ++j) {
     out_idx[i * k + j] = -1;
@@ -577,62 +599,192 @@ __global__ void __launch_bounds__(kKnnBlock, SKW_KNN_MINB) k_knn(const float4 *_
 // GetNearestPoint (KDTree.h:495-503) with NearestPointProc (:293-323):
 // every accepted point becomes the nearest and shrinks the radius.
 template <int S>
+__device__ __forceinline__ int nearest_walk(const float4 *__restrict__ nodes, const uint16_t *__restrict__ nids,
+                                            const float4 *__restrict__ nrm, const double *__restrict__ dirs, int n,
+                                            const Query &Q, double max_dist, uint32_t (*stk)[kKnnBlock],
+                                            unsigned *__restrict__ status) {
+  int best = -1;
+  if (n <= 0) return best;
+  Radius rad;
+  rad.start(Q, max_dist);
+  int sp = 0, cur = 0;
+  float4 p = __ldg(nodes);
+  for (;;) {
+    int near, far;
+    float s2;
+    node_children(p, cur, n, Q, near, far, s2);
+    const float d2f = dist2f(p, Q);
+    if ((d2f < rad.tin || (!(d2f >= rad.tout) && point_d2(p, Q) < rad.get(nodes, Q))) &&
+        (!Q.filter || photon_filter(Q, p, cur, nids, nrm, dirs))) {
+      best = cur;
+      rad.set(Q, cur, d2f, 0.0f);
+    }
+    // The far child waits on the stack, unless its plane is certainly outside
+    // already (the radius only shrinks, so it would be when popped).
+    if (far >= 0 && !(s2 >= rad.tout)) {
+      if (sp >= S) {
+        atomicOr(status, 2u);
+        return best;
+      }
+      stk[sp][threadIdx.x] = (uint32_t)cur;
+      ++sp;
+    }
+    if (near >= 0) {
+      cur = near;
+      p = __ldg(nodes + near);
+      continue;
+    }
+    int next = -1;
+    while (sp > 0) {
+      --sp;
+      // the reference's pop test: (qa - split)^2 < radius, in double
+      const uint32_t par = stk[sp][threadIdx.x];
+      int pnear, pfar;
+      float ps2;
+      const float4 pp = __ldg(nodes + par);
+      node_children(pp, (int)par, n, Q, pnear, pfar, ps2);
+      if (ps2 < rad.tin || (!(ps2 >= rad.tout) && plane_d2(pp, Q) < rad.get(nodes, Q))) {
+        next = pfar;
+        break;
+      }
+    }
+    if (next < 0) break;
+    cur = next;
+    p = __ldg(nodes + cur);
+  }
+  return best;
+}
+
+template <int S>
 __global__ void __launch_bounds__(kKnnBlock, SKW_KNN_MINB) k_nearest(const float4 *__restrict__ nodes, const uint16_t *__restrict__ nids,
                                                  const double *__restrict__ dirs, int n,
                                                  const double *__restrict__ q, const double *__restrict__ qn,
                                                  int64_t nq, double max_dist, double cos_t,
                                                  int32_t *__restrict__ out_idx, unsigned *__restrict__ status,
-                                                 const int *__restrict__ nq_dev, const int32_t *__restrict__ order) {
+                                                 const int *__restrict__ nq_dev, const int32_t *__restrict__ order,
+                                                 int per_warp) {
   __shared__ uint32_t stk[S][kKnnBlock];
-  int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+  const int lane = threadIdx.x & 31;
+  if (lane >= per_warp) return;
+  int64_t i = ((int64_t)blockIdx.x * (kKnnBlock / 32) + (threadIdx.x >> 5)) * per_warp + lane;
   if (nq_dev && *nq_dev < nq) nq = *nq_dev;
   if (i >= nq) return;
   if (order) i = order[i];
   Query Q;
-  Q.q[0] = q[3 * i];
-  Q.q[1] = q[3 * i + 1];
-  Q.q[2] = q[3 * i + 2];
-  Q.filter = cos_t >= 0.0;
-  if (Q.filter) {
-    Q.n[0] = qn[3 * i];
-    Q.n[1] = qn[3 * i + 1];
-    Q.n[2] = qn[3 * i + 2];
-    Q.cos_t = cos_t;
-    Q.sin_t = __dsqrt_rn(__dsub_rn(1.0, __dmul_rn(cos_t, cos_t)));
-  } else {
-    Q.n[0] = Q.n[1] = Q.n[2] = 0.0;
-    Q.cos_t = Q.sin_t = 0.0;
-  }
-  query_float(Q);
-  double maxd2 = __dmul_rn(max_dist, max_dist);
+  load_query(Q, q, qn, i, cos_t);
+  out_idx[i] = nearest_walk<S>(nodes, nids, node_normals(nids, n), dirs, n, Q, max_dist, stk, status);
+}
+
+// The same by looking at every point, one warp per query: for launches of few
+// queries over few points, whose time is their longest walk -- a query whose
+// filter takes no point near it walks the whole tree, one node after the
+// other.  Equal exact distances are settled by the walk (the first visited
+// stays), and so is the answer wherever one is met.
+template <int S>
+__global__ void __launch_bounds__(kKnnBlock, SKW_KNN_MINB) k_nearest_scan(
+    const float4 *__restrict__ nodes, const uint16_t *__restrict__ nids, const double *__restrict__ dirs, int n,
+    const double *__restrict__ q, const double *__restrict__ qn, int64_t nq, double max_dist, double cos_t,
+    int32_t *__restrict__ out_idx, unsigned *__restrict__ status) {
+  static_assert(kKnnBlock == 32, "one query per block");
+  __shared__ uint32_t stk[S][kKnnBlock];
+  const int64_t i = blockIdx.x;
+  const int lane = threadIdx.x;
+  const float4 *nrm = node_normals(nids, n);
+  Query Q;
+  load_query(Q, q, qn, i, cos_t);
+  Radius rad;
+  rad.start(Q, max_dist);
   int best = -1;
-  const int v = walk<S>(nodes, n, Q, maxd2, stk, [&](int ni, const float4 p, double d2, double &md2) -> bool {
-    if (Q.filter && !photon_filter(Q, p, __ldg(nids + ni), dirs)) return false;
-    best = ni;
-    md2 = d2 < 0.0 ? point_d2(p, Q) : d2;
-    return true;
-  });
-  if (v < 0) atomicOr(status, 2u);
-  out_idx[i] = best;
+  bool tie = false;
+  for (int t0 = lane; t0 < n; t0 += 128) {
+    float4 ps[4];
+#pragma unroll
+    for (int u = 0; u < 4; ++u) ps[u] = __ldg(nodes + min(t0 + 32 * u, n - 1));
+#pragma unroll
+    for (int u = 0; u < 4; ++u) {
+      const int t = t0 + 32 * u;
+      const float4 p = ps[u];
+      const float d2f = dist2f(p, Q);
+      if (t >= n || d2f >= rad.tout) continue;
+      bool equal = false;
+      if (!(d2f < rad.tin)) {
+        const double d = point_d2(p, Q), r = rad.get(nodes, Q);
+        if (!(d <= r)) continue;
+        equal = d == r;
+      }
+      if (Q.filter && !photon_filter(Q, p, t, nids, nrm, dirs)) continue;
+      if (equal) {
+        tie = true;
+      } else {
+        best = t;
+        tie = false;
+        rad.set(Q, t, d2f, 0.0f);
+      }
+    }
+  }
+  const double mine = best >= 0 ? point_d2(__ldg(nodes + best), Q) : INFINITY;
+  double least = mine;
+  for (int o = 16; o > 0; o >>= 1) least = fmin(least, __shfl_xor_sync(0xffffffffu, least, o));
+  const unsigned who = __ballot_sync(0xffffffffu, best >= 0 && mine == least);
+  const bool ties = __ballot_sync(0xffffffffu, tie) != 0u || __popc(who) > 1;
+  if (ties) {
+    if (lane == 0) out_idx[i] = nearest_walk<S>(nodes, nids, nrm, dirs, n, Q, max_dist, stk, status);
+  } else if (who == 0u) {
+    if (lane == 0) out_idx[i] = -1;
+  } else if (lane == __ffs(who) - 1) {
+    out_idx[i] = best;
+  }
 }
 
 // Walk stack entries for a tree of n points (see walk).
 constexpr int kShallowStack = 20;
 inline bool shallow_tree(int n) { return n < (1 << kShallowStack); }
 
+// Queries per warp.  A warp's time is the sum of its lanes' divergent walks,
+// so a launch with fewer queries than kSpreadWarps full warps -- about what is
+// resident at k = 100 -- spreads them (the photon maps' 6,427 irradiance
+// estimates: 3.90 -> 1.94 ms in 4s; 2s and 1s measure the same).
+constexpr int64_t kSpreadWarps = 2048;
+inline int queries_per_warp(int64_t nq) {
+  const int64_t per = (nq + kSpreadWarps - 1) / kSpreadWarps;
+  return (int)(per < 32 ? per : 32);
+}
+inline unsigned knn_grid(int64_t nq, int per_warp) {
+  const int64_t per_block = (int64_t)per_warp * (kKnnBlock / 32);
+  return (unsigned)((nq + per_block - 1) / per_block);
+}
+
+// Nearest points by scan: the query's n / 128 rounds take what they take
+// whatever the filter does, about a usual walk's time at kScanPoints points,
+// but a few queries alone walk a tree of thousands faster than one warp scans
+// it, and unfiltered walks are short (scan against walk: 8,000 points, 100
+// filtered queries 115 / 646 us, 8,000 unfiltered 90 / 129 us, one unfiltered
+// 32 / 19 us; 1,000 points, one query 11 / 15 us; the photon maps' 5,848
+// filtered queries over 6,427 points 0.14 / 2.52 ms).
+constexpr int64_t kScanPoints = 8192, kScanFewPoints = 2048, kScanFewQueries = 64, kScanQueries = 16384,
+                  kScanPairs = (int64_t)1 << 26;
+inline bool nearest_by_scan(int64_t nq, int64_t n, bool filter) {
+  return n <= kScanPoints && nq <= kScanQueries && (n <= kScanFewPoints || nq >= kScanFewQueries) &&
+         (filter || nq * n <= kScanPairs);
+}
+
 // k_knn<KMAX, S> with S chosen by the tree's depth.
 template <int KMAX>
-void knn_kernel(unsigned grid, cudaStream_t stream, const float4 *nodes, const uint16_t *nids, const double *dirs,
+void knn_kernel(cudaStream_t stream, const float4 *nodes, const uint16_t *nids, const double *dirs,
                 int n, const double *q, const double *qn, int64_t nq, int k, double max_dist, double cos_t,
                 int32_t *out_idx, double *out_d2, int32_t *out_count, int32_t *out_visited, FCand *scratch,
                 unsigned *status, const int *nq_dev, const int32_t *order) {
+  const int per_warp = queries_per_warp(nq);
+  const unsigned grid = knn_grid(nq, per_warp);
+  const size_t smem = KMAX > 0 ? (size_t)k * kKnnBlock * sizeof(uint32_t) : 0;
   if (shallow_tree(n))
-    k_knn<KMAX, kShallowStack><<<grid, kKnnBlock, 0, stream>>>(nodes, nids, dirs, n, q, qn, nq, k, max_dist, cos_t,
+    k_knn<KMAX, kShallowStack><<<grid, kKnnBlock, smem, stream>>>(nodes, nids, dirs, n, q, qn, nq, k, max_dist, cos_t,
                                                                out_idx, out_d2, out_count, out_visited, scratch,
-                                                               status, nq_dev, order);
+                                                               status, nq_dev, order, per_warp);
   else
-    k_knn<KMAX, 32><<<grid, kKnnBlock, 0, stream>>>(nodes, nids, dirs, n, q, qn, nq, k, max_dist, cos_t, out_idx,
-                                                    out_d2, out_count, out_visited, scratch, status, nq_dev, order);
+    k_knn<KMAX, 32><<<grid, kKnnBlock, smem, stream>>>(nodes, nids, dirs, n, q, qn, nq, k, max_dist, cos_t, out_idx,
+                                                    out_d2, out_count, out_visited, scratch, status, nq_dev, order,
+                                                    per_warp);
 }
 
 // Spatial bins of queries: a box cut into 64^3 cells, each query's cell as
@@ -764,7 +916,23 @@ __global__ void __launch_bounds__(kSortBlock) k_sort_scatter(const uint32_t *__r
   val2[dst] = val ? val[i] : (int32_t)i;
 }
 
+__global__ void k_normals(const uint16_t *__restrict__ nids, int64_t n, const float *__restrict__ dirs_f,
+                          float4 *__restrict__ out) {
+  const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+  if (i >= n) return;
+  const float *d = dirs_f + 3 * (int)nids[i];
+  out[i] = make_float4(d[0], d[1], d[2], 0.0f);
+}
+
 }  // namespace
+
+cudaError_t launch_normals(uint16_t *nids, int64_t n, const double *dirs, cudaStream_t st) {
+  if (n <= 0) return cudaSuccess;
+  k_normals<<<(unsigned)((n + 255) / 256), 256, 0, st>>>(
+      nids, n, reinterpret_cast<const float *>(dirs + (3 << 16)),
+      reinterpret_cast<float4 *>(reinterpret_cast<char *>(nids) + nids_offset(n)));
+  return cudaGetLastError();
+}
 
 int64_t bin_order_bins() { return kBins; }
 
@@ -838,21 +1006,19 @@ cudaError_t launch_knn(const void *nodes, const uint16_t *nids, const double *di
                        double *out_d2, int32_t *out_count, int32_t *out_visited, void *scratch, unsigned *status,
                        cudaStream_t stream, const int *nq_dev, const int32_t *order) {
   if (nq <= 0) return cudaSuccess;
-  const int block = kKnnBlock;
-  const unsigned grid = (unsigned)((nq + block - 1) / block);
   const float4 *nd = (const float4 *)nodes;
   if (scratch && k >= SKW_KNN_GHEAP) {
-    knn_kernel<0>(grid, stream, nd, nids, dirs, n, q, qn, nq, k, max_dist, cos_t, out_idx, out_d2, out_count,
+    knn_kernel<0>(stream, nd, nids, dirs, n, q, qn, nq, k, max_dist, cos_t, out_idx, out_d2, out_count,
                   out_visited, (FCand *)scratch, status, nq_dev, order);
   } else if (k <= 32) {
-    knn_kernel<32>(grid, stream, nd, nids, dirs, n, q, qn, nq, k, max_dist, cos_t, out_idx, out_d2, out_count,
+    knn_kernel<32>(stream, nd, nids, dirs, n, q, qn, nq, k, max_dist, cos_t, out_idx, out_d2, out_count,
                    out_visited, nullptr, status, nq_dev, order);
   } else if (k <= 128) {
-    knn_kernel<128>(grid, stream, nd, nids, dirs, n, q, qn, nq, k, max_dist, cos_t, out_idx, out_d2, out_count,
+    knn_kernel<128>(stream, nd, nids, dirs, n, q, qn, nq, k, max_dist, cos_t, out_idx, out_d2, out_count,
                     out_visited, nullptr, status, nq_dev, order);
   } else {
     if (!scratch) return cudaErrorInvalidValue;
-    knn_kernel<0>(grid, stream, nd, nids, dirs, n, q, qn, nq, k, max_dist, cos_t, out_idx, out_d2, out_count,
+    knn_kernel<0>(stream, nd, nids, dirs, n, q, qn, nq, k, max_dist, cos_t, out_idx, out_d2, out_count,
                   out_visited, (FCand *)scratch, status, nq_dev, order);
   }
   return cudaGetLastError();
@@ -917,9 +1083,7 @@ cudaError_t launch_knn_noalloc(const void *nodes, const uint16_t *nids, const do
   if (e != cudaSuccess) return e;
   // Every heap slot is written before it is read, so the array needs no
   // clearing between calls.
-  const int block = kKnnBlock;
-  const unsigned grid = (unsigned)((nq + block - 1) / block);
-  knn_kernel<0>(grid, stream, (const float4 *)nodes, nids, dirs, n, q, qn, nq, k, max_dist, cos_t, out_idx, out_d2,
+  knn_kernel<0>(stream, (const float4 *)nodes, nids, dirs, n, q, qn, nq, k, max_dist, cos_t, out_idx, out_d2,
                 out_count, nullptr, (FCand *)scratch, status, nullptr, nullptr);
   return cudaGetLastError();
 }
@@ -928,14 +1092,19 @@ cudaError_t launch_nearest(const void *nodes, const uint16_t *nids, const double
                            const double *qn, int64_t nq, double max_dist, double cos_t, int32_t *out_idx,
                            unsigned *status, cudaStream_t stream, const int *nq_dev, const int32_t *order) {
   if (nq <= 0) return cudaSuccess;
-  const int block = kKnnBlock;
-  const unsigned grid = (unsigned)((nq + block - 1) / block);
+  if (!nq_dev && !order && nearest_by_scan(nq, n, cos_t >= 0.0)) {
+    k_nearest_scan<kShallowStack><<<(unsigned)nq, kKnnBlock, 0, stream>>>(
+        (const float4 *)nodes, nids, dirs, n, q, qn, nq, max_dist, cos_t, out_idx, status);
+    return cudaGetLastError();
+  }
+  const int per_warp = queries_per_warp(nq);
+  const unsigned grid = knn_grid(nq, per_warp);
   if (shallow_tree(n))
-    k_nearest<kShallowStack><<<grid, block, 0, stream>>>((const float4 *)nodes, nids, dirs, n, q, qn, nq, max_dist,
-                                                         cos_t, out_idx, status, nq_dev, order);
+    k_nearest<kShallowStack><<<grid, kKnnBlock, 0, stream>>>((const float4 *)nodes, nids, dirs, n, q, qn, nq, max_dist,
+                                                         cos_t, out_idx, status, nq_dev, order, per_warp);
   else
-    k_nearest<32><<<grid, block, 0, stream>>>((const float4 *)nodes, nids, dirs, n, q, qn, nq, max_dist, cos_t,
-                                              out_idx, status, nq_dev, order);
+    k_nearest<32><<<grid, kKnnBlock, 0, stream>>>((const float4 *)nodes, nids, dirs, n, q, qn, nq, max_dist, cos_t,
+                                              out_idx, status, nq_dev, order, per_warp);
   return cudaGetLastError();
 }
 

@@ -170,12 +170,14 @@ int skw_kdtree_create(skw_ctx *ctx, const float *positions, const uint16_t *norm
   if (normal_ids && e == cudaSuccess)
     for (int64_t i = 0; i < n; ++i) nids[(size_t)i] = normal_ids[t->perm[(size_t)i]];
   const std::vector<double> &dirs = skw::direction_table_device();
-  if (e == cudaSuccess) e = cudaMalloc(&t->d_nids, nids.size() * sizeof(uint16_t));
+  if (e == cudaSuccess) e = cudaMalloc(&t->d_nids, skw::nids_bytes(n));
   if (e == cudaSuccess) e = cudaMalloc(&t->d_dirs, dirs.size() * sizeof(double));
   if (e == cudaSuccess) e = cudaMalloc(&t->d_status, sizeof(unsigned));
   if (e == cudaSuccess) e = cudaMemcpy(t->d_nids, nids.data(), nids.size() * sizeof(uint16_t), cudaMemcpyHostToDevice);
   if (e == cudaSuccess) e = cudaMemcpy(t->d_dirs, dirs.data(), dirs.size() * sizeof(double), cudaMemcpyHostToDevice);
   if (e == cudaSuccess) e = cudaMemset(t->d_status, 0, sizeof(unsigned));
+  if (e == cudaSuccess) e = skw::launch_normals(t->d_nids, n, t->d_dirs, nullptr);
+  if (e == cudaSuccess) e = cudaStreamSynchronize(nullptr);  // lookups may come on any stream
   if (e != cudaSuccess) {
     skw_kdtree_destroy(t);
     return cuda_fail(ctx, e, "photon tree upload");

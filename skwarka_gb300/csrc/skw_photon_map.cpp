@@ -43,6 +43,15 @@ cudaError_t upload(const std::vector<T> &v, T **out) {
   return e;
 }
 
+// Normal ids with their normals behind them (nids_bytes).
+cudaError_t upload_nids(const std::vector<uint16_t> &v, const double *dirs, cudaStream_t st, uint16_t **out) {
+  const int64_t n = (int64_t)v.size();
+  cudaError_t e = cudaMalloc((void **)out, skw::nids_bytes(n));
+  if (e == cudaSuccess && n > 0) e = cudaMemcpy(*out, v.data(), (size_t)n * 2, cudaMemcpyHostToDevice);
+  if (e == cudaSuccess) e = skw::launch_normals(*out, n, dirs, st);
+  return e == cudaSuccess ? cudaStreamSynchronize(st) : e;  // lookups on other streams follow
+}
+
 void free_map(Map &m) {
   cudaFree(m.d_nodes);
   cudaFree(m.d_nids);
@@ -55,8 +64,9 @@ void free_map(Map &m) {
 
 // KDTree<Photon>(photons) (Core/KDTree.h:428-473): on the GPU where that
 // gives the reference's tree (no median ties; build_photon_tree_device),
-// else on the host; the photons' attributes in tree order.
-cudaError_t build_map(Map &m, cudaStream_t st) {
+// else on the host; the photons' attributes in tree order.  dirs: the
+// direction table on the device.
+cudaError_t build_map(Map &m, const double *dirs, cudaStream_t st) {
   m.n = (int64_t)m.input.size();
   const size_t n = (size_t)m.n;
   std::vector<float> pos(n * 3), w(n * 3);
@@ -81,10 +91,11 @@ cudaError_t build_map(Map &m, cudaStream_t st) {
     uint16_t *nin = nullptr, *din = nullptr;
     float *win = nullptr;
     if ((e = upload(nids, &nin)) == cudaSuccess && (e = upload(dirid, &din)) == cudaSuccess &&
-        (e = upload(w, &win)) == cudaSuccess && (e = cudaMalloc(&m.d_nids, n * 2)) == cudaSuccess &&
+        (e = upload(w, &win)) == cudaSuccess && (e = cudaMalloc(&m.d_nids, skw::nids_bytes(m.n))) == cudaSuccess &&
         (e = cudaMalloc(&m.d_dirid, n * 2)) == cudaSuccess && (e = cudaMalloc(&m.d_weight, n * 12)) == cudaSuccess &&
         (e = skw::gather_tree_order(d_perm, m.n, nin, din, win, m.d_nids, m.d_dirid, m.d_weight, st)) ==
-            cudaSuccess)
+            cudaSuccess &&
+        (e = skw::launch_normals(m.d_nids, m.n, dirs, st)) == cudaSuccess)
       e = cudaStreamSynchronize(st);
     cudaFree(nin);
     cudaFree(din);
@@ -102,7 +113,7 @@ cudaError_t build_map(Map &m, cudaStream_t st) {
     dt[t] = dirid[i];
     for (int k = 0; k < 3; ++k) wt[3 * t + k] = w[3 * i + k];
   }
-  if (e == cudaSuccess) e = upload(nt, &m.d_nids);
+  if (e == cudaSuccess) e = upload_nids(nt, dirs, st, &m.d_nids);
   if (e == cudaSuccess) e = upload(dt, &m.d_dirid);
   if (e == cudaSuccess) e = upload(wt, &m.d_weight);
   return e;
@@ -117,15 +128,15 @@ struct SideBuild {
   cudaStream_t s = nullptr;
   cudaError_t e = cudaSuccess;
   bool started = false;
-  void start(Map &m, int device) {
+  void start(Map &m, const double *dirs, int device) {
     if (cudaStreamCreateWithFlags(&s, cudaStreamNonBlocking) != cudaSuccess) {
       s = nullptr;  // the caller builds the map in line
       return;
     }
     started = true;
-    worker = std::thread([this, &m, device]() {
+    worker = std::thread([this, &m, dirs, device]() {
       e = cudaSetDevice(device);
-      if (e == cudaSuccess) e = build_map(m, s);
+      if (e == cudaSuccess) e = build_map(m, dirs, s);
     });
   }
   cudaError_t finish() {
@@ -183,11 +194,11 @@ int build_maps(skw_photon_map *pm, cudaStream_t st) {
   // tie) on a thread of its own while the indirect map's is built and its
   // irradiance photons set up
   SideBuild direct;
-  if (!im.input.empty() && !pm->maps[1].input.empty()) direct.start(pm->maps[1], ctx->device);
-  cudaError_t e = build_map(im, st);
+  if (!im.input.empty() && !pm->maps[1].input.empty()) direct.start(pm->maps[1], pm->d_dirs, ctx->device);
+  cudaError_t e = build_map(im, pm->d_dirs, st);
   if (e != cudaSuccess) return cuda_fail(ctx, e, "photon map upload");
   if (im.n == 0) {  // no indirect map: no irradiance photons
-    for (int i = 0; i < 2 && e == cudaSuccess; ++i) e = build_map(pm->maps[i], st);
+    for (int i = 0; i < 2 && e == cudaSuccess; ++i) e = build_map(pm->maps[i], pm->d_dirs, st);
     return e == cudaSuccess ? SKW_OK : cuda_fail(ctx, e, "photon map upload");
   }
   const std::vector<double> &dirs = skw::direction_table();
@@ -259,7 +270,7 @@ int build_maps(skw_photon_map *pm, cudaStream_t st) {
     for (int mi : {2, 1, 0}) {  // the indirect map's tree exists; the others are built as they are needed
       if (e != cudaSuccess) break;
       Map &m = pm->maps[mi];
-      if (q0 == 0 && mi != 2 && (e = mi == 1 && direct.started ? direct.finish() : build_map(m, st)) != cudaSuccess)
+      if (q0 == 0 && mi != 2 && (e = mi == 1 && direct.started ? direct.finish() : build_map(m, pm->d_dirs, st)) != cudaSuccess)
         break;
       if (!has[mi]) continue;
       e = skw::launch_knn(m.d_nodes, m.d_nids, pm->d_dirs, (int)m.n, B.q + 3 * q0, B.qn + 3 * q0, c,
@@ -276,7 +287,7 @@ int build_maps(skw_photon_map *pm, cudaStream_t st) {
       skw::KdNode *dn = nullptr;
       e = upload(nodes, &dn);
       pm->d_irr_nodes = dn;
-      if (e == cudaSuccess) e = upload(nrm_t, &pm->d_irr_nids);
+      if (e == cudaSuccess) e = upload_nids(nrm_t, pm->d_dirs, st, &pm->d_irr_nids);
       if (e == cudaSuccess)
         e = skw::launch_nearest(pm->d_irr_nodes, pm->d_irr_nids, pm->d_dirs, (int)nq, B.sq, B.sqn, ns,
                                 std::numeric_limits<double>::infinity(), kMaxNormalDeviationCos, B.near,
