@@ -88,30 +88,50 @@ struct FlatTree {
 // elimination with full pivoting, row-major 4x4; false if singular.
 bool invert4(const double *m, double *out);
 
-// The tree built on the GPU over triangle boxes (build_accel_tree_gpu):
-// node records by node id (level by level from the root), and the final
-// slot order.
-struct AccelTreeGpu {
-  std::vector<float> box;       // 6 floats per node: lo xyz, hi xyz
-  std::vector<uint32_t> tb, te; // triangle-slot range per node
-  std::vector<uint8_t> flags;   // 0 leaf, 1..3 split axis + 1
-  std::vector<int32_t> child;   // 3 per node (left, middle, right), -1 if absent
-  std::vector<uint32_t> perm;   // triangle (input order) of each final slot
-  int64_t n_nodes = 0, n_leaves = 0;
-  int32_t max_depth = 0;
-  bool inconsistent = false;    // the partition's step map was not a permutation
+// A primitive's mesh, its matrix (row-major 4x4 or null) and index.
+struct MeshJob {
+  const MeshIn *m;
+  const double *xf;
+  int32_t prim;
 };
 
-// Builds the tree of the host build over n triangle boxes (6 floats each:
-// lo xyz, hi xyz, host memory, in the order the host build starts from) on
-// the current device, on stream st (waits for it).
-cudaError_t build_accel_tree_gpu(const float *tbox, int64_t n, cudaStream_t st, AccelTreeGpu &out);
+// A tree built on the GPU, in device memory: as FlatTree's nodes and tris.
+struct DeviceTree {
+  DevNode *nodes = nullptr;
+  DevTri *tris = nullptr;
+  int64_t n_nodes = 0, n_tris = 0, n_leaves = 0;
+  int32_t max_depth = 0;
+  float bounds[6] = {0, 0, 0, 0, 0, 0};
+  bool few = false;           // fewer triangles kept than asked for: no tree
+  bool inconsistent = false;  // the partition's step map was not a permutation: no tree
+  void release();
+};
+
+// The host build's tree over the jobs' triangles (those TriangleMesh keeps),
+// built on the current device, on stream st (waits for it).
+cudaError_t build_accel_tree_gpu(const std::vector<MeshJob> &jobs, int64_t min_n, cudaStream_t st, DeviceTree &out);
 
 // build_accel for accelerators without instancing, the tree built on the
 // GPU (the same tree; meshes shared by several primitives, or fewer than
-// min_gpu triangles, build on the host).  *on_gpu tells which.
+// min_gpu triangles, build on the host).  *on_gpu tells which: then the tree
+// is in `dev`, which the caller owns, else in `out`.
 std::string build_accel_device(const MeshIn *meshes, int32_t n_meshes, const PrimIn *prims, int32_t n_prims,
-                               int threads, cudaStream_t st, int64_t min_gpu, FlatTree &out, bool *on_gpu);
+                               int threads, cudaStream_t st, int64_t min_gpu, FlatTree &out, DeviceTree &dev,
+                               bool *on_gpu);
+
+// The primitive and mesh triangle of every slot.
+cudaError_t launch_slot_ids(const DevTri *tris, int64_t n, int32_t *prim, int32_t *tri, cudaStream_t st);
+
+// A light's triangle (its primitive's first plus its index in the mesh).
+struct LightKey {
+  int32_t tri, light;
+};
+
+// The leaf records (8 words: box, first slot, slots) of the light triangles
+// in `keys` (ascending by tri); those in no leaf keep what `leaf` holds.
+cudaError_t launch_light_leaves(const DevNode *nodes, int64_t n_nodes, const LeafExt *ext, const DevTri *tris,
+                                const int32_t *prim_first, const LightKey *keys, int64_t n_keys, float *leaf,
+                                cudaStream_t st);
 
 // Builds the tree (same split search, partition order and leaf rule as the
 // reference TriangleAccelerator, instancing included: a mesh used by several

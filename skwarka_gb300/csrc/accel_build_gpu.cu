@@ -134,15 +134,102 @@ struct Dev {
 
 inline unsigned grid_of(int64_t m) { return (unsigned)((m + kB - 1) / kB); }
 
-__global__ void k_init(Dev D, const float *__restrict__ tbox) {
-  const int64_t s = (int64_t)blockIdx.x * kB + threadIdx.x;
-  if (s >= D.n) return;
-  for (int c = 0; c < 6; ++c) D.box[s * 6 + c] = tbox[s * 6 + c];
-  D.perm[s] = (uint32_t)s;
-  D.seg[s] = make_int2(0, (int)D.n);
-  D.smask[s] = 0;
-  D.sord[s] = 0;
-  D.spar[s] = -1;
+// The primitives' meshes: their arrays, where their triangles lie among all,
+// their primitive and matrix.
+struct DevMesh {
+  const float *v;
+  const int32_t *ix;
+  int64_t n_vertices, t0;
+  double m[16];
+  int32_t prim, has_m;
+};
+
+__device__ __forceinline__ const DevMesh &mesh_of(const DevMesh *__restrict__ ms, int n_meshes, int64_t t) {
+  int lo = 0, hi = n_meshes;  // the last mesh whose first triangle is not past t
+  while (hi - lo > 1) {
+    const int mid = (lo + hi) >> 1;
+    if (ms[mid].t0 <= t) lo = mid;
+    else hi = mid;
+  }
+  return ms[lo];
+}
+
+// Whether TriangleMesh keeps a triangle: indices in range and not repeated
+// (TriangleMesh.cpp:176-182).
+__global__ void k_keep(const DevMesh *__restrict__ ms, int n_meshes, int64_t total, uint64_t *cnt) {
+  const int64_t t = (int64_t)blockIdx.x * kB + threadIdx.x;
+  if (t > total) return;
+  uint64_t keep = 0;
+  if (t < total) {
+    const DevMesh &m = mesh_of(ms, n_meshes, t);
+    const int32_t *ix = m.ix + 3 * (t - m.t0);
+    const int32_t i = ix[0], j = ix[1], k = ix[2];
+    keep = i >= 0 && j >= 0 && k >= 0 && i < m.n_vertices && j < m.n_vertices && k < m.n_vertices && i != j &&
+           i != k && j != k;
+  }
+  cnt[t] = keep;
+}
+
+// One row of Matrix4x4 * Point3D<float> in the host build's order.
+__device__ __forceinline__ float row_d(const double *m, float x, float y, float z) {
+  return (float)__dadd_rn(
+      __dadd_rn(__dadd_rn(__dmul_rn(m[0], x), __dmul_rn(m[1], y)), __dmul_rn(m[2], z)), m[3]);
+}
+
+// The kept triangles in world space (cnt: how many are kept before each) as
+// slot records in input order, their boxes and the root's state.  Bound by
+// its scattered vertex reads and 101 bytes of writes a triangle: 0.04 ms with
+// k_keep for 1,098,576 triangles; the same loop on the host's threads and the
+// copy of its boxes took 6.2.
+__global__ void k_collect(Dev D, const DevMesh *__restrict__ ms, int n_meshes, int64_t total, DevTri *__restrict__ src) {
+  const int64_t t = (int64_t)blockIdx.x * kB + threadIdx.x;
+  if (t >= total) return;
+  const uint64_t o = D.cnt[t];
+  if (D.cnt[t + 1] == o) return;
+  const DevMesh &m = mesh_of(ms, n_meshes, t);
+  const int32_t *ix = m.ix + 3 * (t - m.t0);
+  float v[9], lo[3], hi[3];
+  for (int a = 0; a < 3; ++a) {
+    lo[a] = INFINITY;
+    hi[a] = -INFINITY;
+  }
+  for (int q = 0; q < 3; ++q) {
+    const float *p = m.v + 3 * (int64_t)ix[q];
+    float x = p[0], y = p[1], z = p[2];
+    if (m.has_m) {  // Transform on Point3D<float>: a divide by w is a product with its double reciprocal
+      const float xp = row_d(m.m, x, y, z), yp = row_d(m.m + 4, x, y, z), zp = row_d(m.m + 8, x, y, z);
+      const float wp = row_d(m.m + 12, x, y, z);
+      x = xp;
+      y = yp;
+      z = zp;
+      if (!(wp == 1.0f)) {
+        const double inv = __ddiv_rn(1.0, (double)wp);
+        x = (float)__dmul_rn((double)xp, inv);
+        y = (float)__dmul_rn((double)yp, inv);
+        z = (float)__dmul_rn((double)zp, inv);
+      }
+    }
+    v[3 * q] = x;
+    v[3 * q + 1] = y;
+    v[3 * q + 2] = z;
+    for (int a = 0; a < 3; ++a) {  // std::min / std::max: the first of equal values, NaN skipped
+      lo[a] = v[3 * q + a] < lo[a] ? v[3 * q + a] : lo[a];
+      hi[a] = hi[a] < v[3 * q + a] ? v[3 * q + a] : hi[a];
+    }
+  }
+  float4 *r = (float4 *)(src + o);
+  r[0] = make_float4(v[0], v[1], v[2], __int_as_float(m.prim));
+  r[1] = make_float4(v[3], v[4], v[5], __int_as_float((int32_t)(o - D.cnt[m.t0])));
+  r[2] = make_float4(v[6], v[7], v[8], 0.0f);
+  for (int a = 0; a < 3; ++a) {
+    D.box[o * 6 + a] = lo[a];
+    D.box[o * 6 + 3 + a] = hi[a];
+  }
+  D.perm[o] = (uint32_t)o;
+  D.seg[o] = make_int2(0, (int)D.n);
+  D.smask[o] = 0;
+  D.sord[o] = 0;
+  D.spar[o] = -1;
 }
 
 // Heads of the level's nodes: their rank (a scan) gives the node id.
@@ -379,7 +466,8 @@ __device__ __forceinline__ double plane_position(int i, float nlo, float nhi, in
 // boxes on the two sides of its plane (lane + 32 in a second round) and across
 // it.  Every (node, axis) is bound by these 32 n updates; the double costs are
 // made for a round only if one of its planes could still be the least.
-// (1,098,576 triangles: all split searches of the build: bucket fill, init and scores 18.8 -> 6.3 ms with the other two.)
+// All three sizes together, bucket fill and scores before: 18.8 -> 6.3 ms for
+// 1,098,576 triangles.
 constexpr int kSmallWarps = 4;
 __global__ void __launch_bounds__(kSmallWarps * 32) k_split_small(Dev D) {
   __shared__ float4 s_lo[kSmallWarps][32], s_hi[kSmallWarps][32];
@@ -883,23 +971,178 @@ __global__ void k_children(Dev D) {
   }
 }
 
+// Flattening: the tree in pre-order, a node's present children in
+// consecutive places, so that a child's subtree starts where those of its
+// left siblings end.  Levels bottom up give every subtree's size (the root
+// left out), levels top down the places.  Bound by its launches (28 for 21
+// levels): 0.15 ms for 1,098,576 triangles, and 0.02 for the slots, all of it
+// in device memory.  On the host one walk over the records took 5.4 ms, the
+// slots 4.2, their copies to the host and back 2.5.  A launch takes one level, or several of at most kNarrow nodes
+// in one block (the first and last levels are narrow: a launch each costs
+// more than their work).
+constexpr int kNarrow = 1024;
+
+__global__ void k_subtree(Dev D, const int64_t *__restrict__ level, int l0, int l1, uint32_t *sub) {
+  for (int l = l1 - 1; l >= l0; --l) {
+    for (int64_t id = level[l] + (int64_t)blockIdx.x * blockDim.x + threadIdx.x; id < level[l + 1];
+         id += (int64_t)gridDim.x * blockDim.x) {
+      uint32_t n = 0;
+      for (int c = 0; c < 3; ++c) {
+        const int32_t ch = D.rchild[id * 3 + c];
+        if (ch >= 0) n += 1 + sub[ch];
+      }
+      sub[id] = n;
+    }
+    __syncthreads();
+  }
+}
+
+// place: a node's own place and its first child's.
+__global__ void k_flatten(Dev D, const int64_t *__restrict__ level, int l0, int l1, const uint32_t *__restrict__ sub,
+                          uint2 *place, int64_t n_nodes, DevNode *__restrict__ nodes) {
+  for (int l = l0; l < l1; ++l) {
+    for (int64_t id = level[l] + (int64_t)blockIdx.x * blockDim.x + threadIdx.x; id < level[l + 1];
+         id += (int64_t)gridDim.x * blockDim.x) {
+      const uint2 at = id == 0 ? make_uint2(0, 1) : place[id];
+      if (at.x >= n_nodes) {  // no parent: only after an inconsistent step map
+        atomicOr(D.err, 16);
+        continue;
+      }
+      DevNode dn;
+      for (int k = 0; k < 3; ++k) {
+        dn.lo[k] = D.rbox[id * 6 + k];
+        dn.hi[k] = D.rbox[id * 6 + 3 + k];
+      }
+      const uint32_t flags = D.rflags[id];
+      if (flags == 0) {
+        dn.a = D.rtb[id];
+        dn.b = (D.rte[id] - D.rtb[id]) << 8;
+      } else {
+        int32_t ch[3];
+        uint32_t mask = 0;
+        for (int c = 0; c < 3; ++c) {
+          ch[c] = D.rchild[id * 3 + c];
+          if (ch[c] >= 0) mask |= 1u << c;
+        }
+        uint32_t slot = at.y, first = at.y + __popc(mask);
+        for (int c = 0; c < 3; ++c)
+          if (ch[c] >= 0) {
+            place[ch[c]] = make_uint2(slot++, first);
+            first += sub[ch[c]];
+          }
+        dn.a = at.y;
+        dn.b = flags | (mask << 2);
+      }
+      nodes[at.x] = dn;
+    }
+    __syncthreads();
+  }
+}
+
+__global__ void k_tris(Dev D, const DevTri *__restrict__ src, DevTri *__restrict__ tris) {
+  const int64_t i = (int64_t)blockIdx.x * kB + threadIdx.x;
+  if (i >= D.n) return;
+  const float4 *r = (const float4 *)(src + D.perm[i]);
+  float4 *w = (float4 *)(tris + i);
+  const float4 c = r[2];
+  w[0] = r[0];
+  w[1] = r[1];
+  w[2] = make_float4(c.x, c.y, c.z, __int_as_float((int32_t)i));
+}
+
+// A slot's primitive and mesh triangle.
+__global__ void k_slot_ids(const DevTri *__restrict__ tris, int64_t n, int32_t *prim, int32_t *tri) {
+  const int64_t i = (int64_t)blockIdx.x * kB + threadIdx.x;
+  if (i >= n) return;
+  prim[i] = tris[i].prim;
+  tri[i] = tris[i].tri;
+}
+
+// The leaf of every light triangle: each leaf looks its triangles up in the
+// sorted keys.  A light triangle's record stays as it is if no leaf holds it.
+__global__ void k_light_leaves(const DevNode *__restrict__ nodes, int64_t n_nodes, const LeafExt *__restrict__ ext,
+                               const DevTri *__restrict__ tris, const int32_t *__restrict__ prim_first,
+                               const LightKey *__restrict__ keys, int64_t n_keys, float *__restrict__ leaf) {
+  const int64_t id = (int64_t)blockIdx.x * kB + threadIdx.x;
+  if (id >= n_nodes) return;
+  const DevNode nd = nodes[id];
+  if ((nd.b & 3u) != 0u) return;
+  const bool x = (nd.b & kLeafExt) != 0;
+  const uint32_t first = x ? ext[nd.a].tri_first : nd.a, count = x ? ext[nd.a].tri_count : nd.b >> 8;
+  for (uint32_t k = 0; k < count; ++k) {
+    const DevTri &t = tris[first + k];
+    if (t.prim < 0) continue;  // a shared mesh's slot belongs to no one primitive
+    const int32_t key = prim_first[t.prim] + t.tri;
+    int64_t lo = 0, hi = n_keys;
+    while (lo < hi) {
+      const int64_t mid = (lo + hi) >> 1;
+      if (keys[mid].tri < key) lo = mid + 1;
+      else hi = mid;
+    }
+    for (; lo < n_keys && keys[lo].tri == key; ++lo) {
+      float *o = leaf + 8 * (int64_t)keys[lo].light;
+      for (int c = 0; c < 3; ++c) {
+        o[c] = nd.lo[c];
+        o[3 + c] = nd.hi[c];
+      }
+      o[6] = __uint_as_float(first);
+      o[7] = __uint_as_float(count);
+    }
+  }
+}
+
 inline size_t al256(size_t x) { return (x + 255) & ~(size_t)255; }
 
 }  // namespace
 
-cudaError_t build_accel_tree_gpu(const float *tbox, int64_t n, cudaStream_t st, AccelTreeGpu &out) {
-  out = AccelTreeGpu();
+cudaError_t build_accel_tree_gpu(const std::vector<MeshJob> &jobs, int64_t min_n, cudaStream_t st, DeviceTree &out) {
+  out = DeviceTree();
+  // The meshes' arrays: one copy for all the small ones, one each for the
+  // others (a copy costs some microseconds, whatever it moves).
+  constexpr size_t kOwnCopy = 1 << 16;
+  struct Part {
+    const void *src;
+    size_t bytes, at;
+  };
+  std::vector<Part> parts;
+  std::vector<DevMesh> meshes;
+  int64_t n = 0;
+  for (const MeshJob &j : jobs) {
+    if (j.m->n_triangles <= 0) continue;
+    DevMesh d{};
+    d.n_vertices = std::max<int64_t>(j.m->n_vertices, 0);
+    d.t0 = n;
+    d.prim = j.prim;
+    d.has_m = j.xf ? 1 : 0;
+    if (j.xf) std::memcpy(d.m, j.xf, sizeof(d.m));
+    meshes.push_back(d);
+    parts.push_back(Part{j.m->vertices, (size_t)d.n_vertices * 12, 0});
+    parts.push_back(Part{j.m->triangles, (size_t)j.m->n_triangles * 12, 0});
+    n += j.m->n_triangles;
+  }
   if (n <= 0 || n > (int64_t)INT32_MAX / 2) return cudaErrorInvalidValue;
+  size_t staged = al256(meshes.size() * sizeof(DevMesh)), mesh_bytes = 0;
+  for (Part &p : parts)
+    if (p.bytes < kOwnCopy) {
+      p.at = staged;
+      staged += (p.bytes + 15) & ~(size_t)15;
+    }
+  mesh_bytes = al256(staged);
+  for (Part &p : parts)
+    if (p.bytes >= kOwnCopy) {
+      p.at = mesh_bytes;
+      mesh_bytes += al256(p.bytes);
+    }
   Dev D{};
-  D.n = n;
-  const size_t n1 = (size_t)n + 1, nb = (n1 + kB - 1) / kB;
+  size_t n1 = (size_t)n + 1;
+  const size_t nb = (n1 + kB - 1) / kB;
   size_t total = 0;
   std::vector<std::pair<void **, size_t>> plan;
   auto want = [&](void *pp, size_t bytes) {
     plan.push_back({(void **)pp, bytes});
     total += al256(bytes);
   };
-  const size_t nn = (size_t)n;
+  size_t nn = (size_t)n;
   want(&D.box, nn * 24);
   want(&D.box2, nn * 24);
   want(&D.perm, nn * 4);
@@ -944,6 +1187,10 @@ cudaError_t build_accel_tree_gpu(const float *tbox, int64_t n, cudaStream_t st, 
   want(&D.err, 256);
   want(&D.maxseg, 256);
   want(&D.n_leaves, 256);
+  char *mesh_mem = nullptr;
+  DevTri *src = nullptr;
+  want(&mesh_mem, mesh_bytes);
+  want(&src, nn * sizeof(DevTri));
   char *arena = nullptr;
   cudaError_t e = cudaMalloc(&arena, total);
   if (e != cudaSuccess) return e;
@@ -1003,24 +1250,57 @@ cudaError_t build_accel_tree_gpu(const float *tbox, int64_t n, cudaStream_t st, 
     cudaFree(D.rchild);
     cudaFree(arena);
   };
-  float *d_tbox = nullptr;
   uint64_t *h_count = nullptr;
-  if ((e = cudaMalloc(&d_tbox, nn * 24)) != cudaSuccess || (e = cudaMallocHost(&h_count, 16)) != cudaSuccess) {
-    cudaFree(d_tbox);
+  if ((e = cudaMallocHost(&h_count, 16)) != cudaSuccess) {
     release();
     return e;
   }
-  const unsigned gn = grid_of(n), gn1 = grid_of((int64_t)n1);
-  e = cudaMemcpyAsync(d_tbox, tbox, nn * 24, cudaMemcpyHostToDevice, st);
+  const int n_meshes = (int)meshes.size();
+  for (size_t k = 0; k < parts.size(); ++k) {
+    const void *at = mesh_mem + parts[k].at;
+    if (k & 1) meshes[k / 2].ix = (const int32_t *)at;
+    else meshes[k / 2].v = (const float *)at;
+  }
+  std::vector<char> stage(staged);
+  std::memcpy(stage.data(), meshes.data(), meshes.size() * sizeof(DevMesh));
+  for (const Part &p : parts)
+    if (p.bytes > 0 && p.bytes < kOwnCopy) std::memcpy(stage.data() + p.at, p.src, p.bytes);
+  e = cudaMemcpyAsync(mesh_mem, stage.data(), staged, cudaMemcpyHostToDevice, st);
+  for (const Part &p : parts)
+    if (e == cudaSuccess && p.bytes >= kOwnCopy)
+      e = cudaMemcpyAsync(mesh_mem + p.at, p.src, p.bytes, cudaMemcpyHostToDevice, st);
   if (e == cudaSuccess) e = cudaMemsetAsync(D.err, 0, 4, st);
   if (e == cudaSuccess) e = cudaMemsetAsync(D.n_leaves, 0, 8, st);
+  const DevMesh *d_meshes = (const DevMesh *)mesh_mem;
+  const int64_t total_tris = n;
+  if (e == cudaSuccess) {
+    k_keep<<<grid_of(total_tris + 1), kB, 0, st>>>(d_meshes, n_meshes, total_tris, D.cnt);
+    e = scan64(D.cnt, total_tris + 1, D.sums, st);
+  }
+  if (e == cudaSuccess) e = cudaMemcpyAsync(h_count, D.cnt + total_tris, 8, cudaMemcpyDeviceToHost, st);
+  if (e == cudaSuccess) e = cudaStreamSynchronize(st);
+  if (e == cudaSuccess) {
+    n = (int64_t)h_count[0];
+    if (n < std::max<int64_t>(min_n, 1)) {
+      out.few = true;
+      cudaFreeHost(h_count);
+      release();
+      return cudaSuccess;
+    }
+  }
+  D.n = n;
+  nn = (size_t)n;
+  n1 = nn + 1;
+  const unsigned gn = grid_of(n), gn1 = grid_of((int64_t)n1);
   if (e == cudaSuccess) e = grow(std::max<int64_t>(2 * n, 1024));
   if (e == cudaSuccess) {
-    k_init<<<gn, kB, 0, st>>>(D, d_tbox);
+    k_collect<<<grid_of(total_tris), kB, 0, st>>>(D, d_meshes, n_meshes, total_tris, src);
     e = cudaGetLastError();
   }
+  std::vector<int64_t> level_base;  // first node of every level, and the end
   int depth = 0;
   for (; e == cudaSuccess; ++depth) {
+    level_base.push_back(n_nodes);
     if ((e = cudaMemsetAsync(D.maxseg, 0, 4, st)) != cudaSuccess) break;
     k_heads<<<gn1, kB, 0, st>>>(D);
     if ((e = scan64(D.cnt, (int64_t)n1, D.sums, st)) != cudaSuccess) break;
@@ -1079,32 +1359,80 @@ cudaError_t build_accel_tree_gpu(const float *tbox, int64_t n, cudaStream_t st, 
   }
   int err_flag = 0;
   unsigned long long leaves = 0;
-  if (e == cudaSuccess) {
-    out.box.resize((size_t)n_nodes * 6);
-    out.tb.resize((size_t)n_nodes);
-    out.te.resize((size_t)n_nodes);
-    out.flags.resize((size_t)n_nodes);
-    out.child.resize((size_t)n_nodes * 3);
-    out.perm.resize(nn);
-    if ((e = cudaMemcpyAsync(out.box.data(), D.rbox, (size_t)n_nodes * 24, cudaMemcpyDeviceToHost, st)) == cudaSuccess &&
-        (e = cudaMemcpyAsync(out.tb.data(), D.rtb, (size_t)n_nodes * 4, cudaMemcpyDeviceToHost, st)) == cudaSuccess &&
-        (e = cudaMemcpyAsync(out.te.data(), D.rte, (size_t)n_nodes * 4, cudaMemcpyDeviceToHost, st)) == cudaSuccess &&
-        (e = cudaMemcpyAsync(out.flags.data(), D.rflags, (size_t)n_nodes, cudaMemcpyDeviceToHost, st)) == cudaSuccess &&
-        (e = cudaMemcpyAsync(out.child.data(), D.rchild, (size_t)n_nodes * 12, cudaMemcpyDeviceToHost, st)) ==
+  char *flat_mem = nullptr;
+  if (e == cudaSuccess && (uint32_t)h_count[1] != 0) {
+    out.inconsistent = true;
+  } else if (e == cudaSuccess) {
+    // Level k is [level_base[k], level_base[k + 1]): the last one is empty.
+    const int n_levels = (int)level_base.size() - 1;
+    const size_t sub_at = al256(level_base.size() * 8), place_at = sub_at + al256((size_t)n_nodes * 4);
+    std::vector<std::pair<int, int>> runs;
+    for (int l = 0; l < n_levels; ++l) {
+      const bool narrow = level_base[(size_t)l + 1] - level_base[(size_t)l] <= kNarrow;
+      const bool joins = !runs.empty() && narrow &&
+                         level_base[(size_t)l] - level_base[(size_t)l - 1] <= kNarrow;
+      if (joins) runs.back().second = l + 1;
+      else runs.push_back({l, l + 1});
+    }
+    auto grid = [&](const std::pair<int, int> &r) {
+      const int64_t m = level_base[(size_t)r.first + 1] - level_base[(size_t)r.first];
+      return m <= kNarrow ? 1u : grid_of(m);
+    };
+    auto block = [&](const std::pair<int, int> &r) { return grid(r) == 1u ? (unsigned)kNarrow : (unsigned)kB; };
+    if ((e = cudaMalloc(&flat_mem, place_at + (size_t)n_nodes * 8)) == cudaSuccess &&
+        (e = cudaMalloc(&out.nodes, (size_t)n_nodes * sizeof(DevNode))) == cudaSuccess &&
+        (e = cudaMalloc(&out.tris, nn * sizeof(DevTri))) == cudaSuccess &&
+        (e = cudaMemcpyAsync(flat_mem, level_base.data(), level_base.size() * 8, cudaMemcpyHostToDevice, st)) ==
             cudaSuccess &&
-        (e = cudaMemcpyAsync(out.perm.data(), D.perm, nn * 4, cudaMemcpyDeviceToHost, st)) == cudaSuccess &&
+        (e = cudaMemsetAsync(flat_mem + place_at, 0xFF, (size_t)n_nodes * 8, st)) == cudaSuccess) {
+      const int64_t *level = (const int64_t *)flat_mem;
+      uint32_t *sub = (uint32_t *)(flat_mem + sub_at);
+      uint2 *place = (uint2 *)(flat_mem + place_at);
+      for (size_t r = runs.size(); r-- > 0;)
+        k_subtree<<<grid(runs[r]), block(runs[r]), 0, st>>>(D, level, runs[r].first, runs[r].second, sub);
+      for (const auto &r : runs)
+        k_flatten<<<grid(r), block(r), 0, st>>>(D, level, r.first, r.second, sub, place, n_nodes,
+                                                 out.nodes);
+      k_tris<<<gn, kB, 0, st>>>(D, src, out.tris);
+      e = cudaGetLastError();
+    }
+    if (e == cudaSuccess &&
+        (e = cudaMemcpyAsync(out.bounds, D.rbox, 24, cudaMemcpyDeviceToHost, st)) == cudaSuccess &&
         (e = cudaMemcpyAsync(&err_flag, D.err, 4, cudaMemcpyDeviceToHost, st)) == cudaSuccess &&
         (e = cudaMemcpyAsync(&leaves, D.n_leaves, 8, cudaMemcpyDeviceToHost, st)) == cudaSuccess)
       e = cudaStreamSynchronize(st);
   }
   out.n_nodes = n_nodes;
+  out.n_tris = n;
   out.max_depth = depth - 1;
   out.n_leaves = (int64_t)leaves;
-  out.inconsistent = err_flag != 0;
-  cudaFree(d_tbox);
+  out.inconsistent = out.inconsistent || err_flag != 0;
+  if (e != cudaSuccess || out.inconsistent) out.release();
+  cudaFree(flat_mem);
   cudaFreeHost(h_count);
   release();
   return e;
+}
+
+void DeviceTree::release() {
+  cudaFree(nodes);
+  cudaFree(tris);
+  nodes = nullptr;
+  tris = nullptr;
+}
+
+cudaError_t launch_slot_ids(const DevTri *tris, int64_t n, int32_t *prim, int32_t *tri, cudaStream_t st) {
+  if (n <= 0) return cudaSuccess;
+  k_slot_ids<<<grid_of(n), kB, 0, st>>>(tris, n, prim, tri);
+  return cudaGetLastError();
+}
+
+cudaError_t launch_light_leaves(const DevNode *nodes, int64_t n_nodes, const LeafExt *ext, const DevTri *tris,
+                                const int32_t *prim_first, const LightKey *keys, int64_t n_keys, float *leaf,
+                                cudaStream_t st) {
+  if (n_nodes <= 0 || n_keys <= 0) return cudaSuccess;
+  k_light_leaves<<<grid_of(n_nodes), kB, 0, st>>>(nodes, n_nodes, ext, tris, prim_first, keys, n_keys, leaf);
+  return cudaGetLastError();
 }
 
 }  // namespace skw

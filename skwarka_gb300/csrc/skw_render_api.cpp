@@ -11,6 +11,7 @@
 #include <string>
 #include <vector>
 
+#include "accel_build.h"
 #include "kernels.h"
 #include "photon_map_internal.h"
 #include "photon_types.h"
@@ -422,52 +423,19 @@ int skw_scene_create(skw_ctx *ctx, const skw_mesh *meshes, int32_t n_meshes, con
       pls[(size_t)i].position[k] = point_lights[i].position[k];
       pls[(size_t)i].intensity[k] = point_lights[i].intensity[k];
     }
-  // The accelerator leaf of every light triangle (its box and slot range).
+  // The accelerator leaf of every light triangle (its box and slot range),
+  // found on the device.  Those in no leaf (an instanced light mesh) keep an
+  // empty box and range, which test nothing.
   std::vector<float> light_leaf(8 * std::max<size_t>(light_tri.size(), 1), 0.0f);
-  {
-    const std::vector<skw::DevNode> &nodes = s->accel->h_nodes;
-    const std::vector<skw::DevTri> &slots = s->accel->h_tris;
-    std::vector<int32_t> leaf_of_slot(slots.size(), -1), slot_of_tri((size_t)std::max(tri_count, 1), -1);
-    // a leaf's triangle-slot range (leaves holding instances keep it in the ext table)
-    auto leaf_range = [&](const skw::DevNode &nd, uint32_t &first, uint32_t &count) {
-      if (nd.b & skw::kLeafExt) {
-        first = s->accel->h_leaf_ext[nd.a].tri_first;
-        count = s->accel->h_leaf_ext[nd.a].tri_count;
-      } else {
-        first = nd.a;
-        count = nd.b >> 8;
-      }
-    };
-    for (size_t n = 0; n < nodes.size(); ++n)
-      if ((nodes[n].b & 3u) == 0u) {
-        uint32_t first, count;
-        leaf_range(nodes[n], first, count);
-        for (uint32_t k = 0; k < count; ++k) leaf_of_slot[first + k] = (int32_t)n;
-      }
-    for (size_t k = 0; k < slots.size(); ++k)  // (a shared mesh's slots, prim -1, belong to no one primitive)
-      if (slots[k].prim >= 0)
-        slot_of_tri[(size_t)(prim_tri_offset[(size_t)slots[k].prim] + slots[k].tri)] = (int32_t)k;
-    for (size_t j = 0; j < light_tri.size(); ++j) {
-      const int32_t slot = slot_of_tri[(size_t)light_tri[j]];
-      const int32_t leaf = slot >= 0 ? leaf_of_slot[(size_t)slot] : -1;
-      float *o = light_leaf.data() + 8 * j;
-      if (leaf < 0) {  // an instanced light mesh: an empty range tests nothing
-        o[0] = o[1] = o[2] = INFINITY;
-        o[3] = o[4] = o[5] = -INFINITY;
-        continue;
-      }
-      const skw::DevNode &L = nodes[(size_t)leaf];
-      for (int c = 0; c < 3; ++c) {
-        o[c] = L.lo[c];
-        o[3 + c] = L.hi[c];
-      }
-      uint32_t ufirst, ucount;
-      leaf_range(L, ufirst, ucount);
-      const int32_t first = (int32_t)ufirst, count = (int32_t)ucount;
-      std::memcpy(o + 6, &first, 4);
-      std::memcpy(o + 7, &count, 4);
-    }
+  std::vector<skw::LightKey> light_key;
+  for (size_t j = 0; j < light_tri.size(); ++j) {
+    float *o = light_leaf.data() + 8 * j;
+    o[0] = o[1] = o[2] = INFINITY;
+    o[3] = o[4] = o[5] = -INFINITY;
+    light_key.push_back(skw::LightKey{light_tri[j], (int32_t)j});
   }
+  std::sort(light_key.begin(), light_key.end(),
+            [](const skw::LightKey &x, const skw::LightKey &y) { return x.tri < y.tri; });
   cudaError_t e = cudaSetDevice(ctx->device);
   skw::SceneDev &D = s->dev;
   D.accel_tris = (const float4 *)s->accel->d_tris;
@@ -494,6 +462,14 @@ int skw_scene_create(skw_ctx *ctx, const skw_mesh *meshes, int32_t n_meshes, con
   if (e == cudaSuccess) e = upload(s, light_tri, &D.light_tri);
   if (e == cudaSuccess) e = upload(s, light_cdf, &D.light_cdf);
   if (e == cudaSuccess) e = upload(s, pls, &D.point_lights);
+  if (e == cudaSuccess && !light_key.empty()) {
+    const skw::LightKey *keys = nullptr;
+    e = upload(s, light_key, &keys);
+    if (e == cudaSuccess)
+      e = skw::launch_light_leaves(s->accel->d_nodes, s->accel->info.n_nodes, s->accel->d_leaf_ext, s->accel->d_tris,
+                                   D.prim_tri_offset, keys, (int64_t)light_key.size(), (float *)D.light_leaf, nullptr);
+    if (e == cudaSuccess) e = cudaStreamSynchronize(nullptr);
+  }
   if (e != cudaSuccess) {
     skw_scene_destroy(s);
     return cuda_fail(ctx, e, "render scene upload");
