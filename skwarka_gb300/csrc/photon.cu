@@ -103,8 +103,8 @@ __device__ __forceinline__ float bounce_rnd(uint64_t seed, uint64_t path, int bo
 // (black on total internal reflection, with the mirror direction).  The
 // host admits at most one layer with specular components.
 __device__ bool specular_parts(const Bsdf &b, V3 inc_w, V3 &dr, V3 &fr, V3 &dt, V3 &ft) {
-  for (int i = 0; i < b.nl; ++i) {
-    const Layer l = i == 0 ? b.L0 : layer1(b);
+  for (int i = 0; i < b.L.nl; ++i) {
+    const Layer l = layer_at(b.L, i);
     const V3 r = layer_spec_r(l), t = layer_spec_t(l);
     if (black(r) && black(t)) continue;
     const V3 wi = b.local(inc_w);
@@ -141,8 +141,8 @@ __device__ V3 specular_sample_photon(const Bsdf &b, V3 inc_w, float uc, V3 &dir,
   pdf = 0.0f;
   dir = inc_w;
   if (!specular_parts(b, inc_w, dr, fr, dt, ft)) return v3(0, 0, 0);
-  const bool has_r = !black(layer_spec_r(b.L0)) || (b.nl == 2 && !black(layer_spec_r(layer1(b))));
-  const bool has_t = !black(layer_spec_t(b.L0)) || (b.nl == 2 && !black(layer_spec_t(layer1(b))));
+  const bool has_r = !black(layer_spec_r(layer0(b.L))) || (b.L.nl == 2 && !black(layer_spec_r(layer1(b.L))));
+  const bool has_t = !black(layer_spec_t(layer0(b.L))) || (b.L.nl == 2 && !black(layer_spec_t(layer1(b.L))));
   pdf = 1.0f;
   if (has_r && has_t) {
     const float lr = 0.05316285f * fr.x + 0.58515348f * fr.y + 0.36168367f * fr.z;
@@ -196,7 +196,7 @@ __device__ V3 bsdf_sample_all(const Bsdf &b, V3 inc_w, float uc, float u0, float
   specular = true;
   V3 dr, fr, dt, ft;
   specular_parts(b, inc_w, dr, fr, dt, ft);
-  const bool has_r = !black(layer_spec_r(b.L0)) || (b.nl == 2 && !black(layer_spec_r(layer1(b))));
+  const bool has_r = !black(layer_spec_r(layer0(b.L))) || (b.L.nl == 2 && !black(layer_spec_r(layer1(b.L))));
   const bool refl = has_r && c == nn;  // the reflection comes first when both are present
   dir = refl ? dr : dt;
   pdf = 1.0f / n;
@@ -884,8 +884,8 @@ __device__ __forceinline__ V3 clamp01(V3 r) {
 // the Fresnel term and the total-internal-reflection test read its world z.
 __device__ void total_scattering(const Bsdf &bs, V3 wi, V3 &refl, V3 &trans) {
   refl = trans = v3(0, 0, 0);
-  for (int i = 0; i < bs.nl; ++i) {
-    const Layer b = i == 0 ? bs.L0 : layer1(bs);
+  for (int i = 0; i < bs.L.nl; ++i) {
+    const Layer b = layer_at(bs.L, i);
     V3 r = v3(0, 0, 0), t = v3(0, 0, 0);
     switch (b.kind) {
       case kMeasured: r = total_scattering_measured(b, wi); break;

@@ -168,15 +168,26 @@ struct Layer {
   MerlDev merl;
   V3 scale;
 };
-// The second layer of a mix is kept as its material (read again where it
-// is needed, an L1-resident line) so that the common one-layer BSDF stays
-// in registers.
-struct Bsdf {
-  V3 n, e1, e2, ng;  // shading frame and geometric normal
-  int nl;            // layers (1, or 2 for a mix)
-  Layer L0;
+// The layers as the kernels hold them: what a diffuse one-layer surface
+// needs, and the materials (L1-resident lines) that the other kinds read
+// again where they are evaluated.  Nearly every hit is diffuse, so its few
+// operations are inlined at each use and the rest is called: inlined at all
+// of them, it was most of the kernels' code and registers (k_shade: 168 of
+// them, 12 warps per SM, and 4 in 10 of its stalls waits for instructions).
+struct Layers {
+  int nl;                 // layers (1, or 2 for a mix)
+  int kind;               // the first layer's kind, diffuse reflectance, Oren-Nayar terms and scale
+  V3 kd;
+  float on_a, on_b;
+  V3 scale;
+  const DevMaterial *m0;  // the first layer's material (null: it scatters nothing)
   const DevMaterial *m1;  // nl == 2: the second layer's material
   V3 s1;                  // nl == 2: its scale
+  __device__ __forceinline__ bool diffuse() const { return nl == 1 && (kind == kLambert || kind == kOrenNayar); }
+};
+struct Bsdf {
+  V3 n, e1, e2, ng;  // shading frame and geometric normal
+  Layers L;
   __device__ __forceinline__ V3 local(V3 w) const { return v3(dot(w, e1), dot(w, e2), dot(w, n)); }
   __device__ __forceinline__ V3 world(V3 l) const { return e1 * l.x + e2 * l.y + n * l.z; }
 };
@@ -254,14 +265,24 @@ __device__ __forceinline__ bool blinn_sample(float exponent, V3 wi, float u0, fl
 
 // Diffuse component: Lambertian (BxDFs/Lambertian.cpp:18-30) or the
 // reference's Oren-Nayar (BxDFs/OrenNayar.cpp:19-42).
-__device__ __forceinline__ V3 diffuse_eval(const Layer &b, V3 wi, V3 wo) {
-  if (b.kind != kOrenNayar) return b.kd * kInvPi;
+__device__ __forceinline__ V3 diffuse_eval(int kind, V3 kd, float on_a, float on_b, V3 wi, V3 wo) {
+  if (kind != kOrenNayar) return kd * kInvPi;
   const float dcos = fmaxf(0.0f, wi.x * wo.x + wi.y * wo.y);
   const float denom = fmaxf(fabsf(wi.z), fabsf(wo.z));
-  return b.kd * (kInvPi * (b.on_a + b.on_b * dcos / denom));
+  return kd * (kInvPi * (on_a + on_b * dcos / denom));
+}
+__device__ __forceinline__ V3 diffuse_eval(const Layer &b, V3 wi, V3 wo) {
+  return diffuse_eval(b.kind, b.kd, b.on_a, b.on_b, wi, wo);
 }
 __device__ __forceinline__ float diffuse_pdf(V3 wi, V3 wo) {  // BxDF::PDF (Core/BxDF.cpp:33-37)
   return wi.z * wo.z > 0.0f ? fabsf(wo.z) * kInvPi : 0.0f;
+}
+
+// BxDF::Sample (Core/BxDF.cpp:20-31): cosine hemisphere on the incident side.
+__device__ __forceinline__ V3 diffuse_sample(V3 wi, float u0, float u1) {
+  V3 wo = cosine_hemisphere(u0, u1);
+  if (wi.z < 0.0f) wo.z = -wo.z;
+  return wo;
 }
 
 // FresnelBlend<BlinnDistribution> (BxDFs/FresnelBlend.h): Ashikhmin and
@@ -508,18 +529,29 @@ __device__ Layer make_layer(const DevMaterial &m) {
   l.scale = v3(1.0f, 1.0f, 1.0f);
   return l;
 }
-// The second layer of a mix (nl == 2).
-__device__ __forceinline__ Layer layer1(const Bsdf &b) {
-  Layer l = make_layer(*b.m1);
-  l.scale = b.s1;
+__device__ __forceinline__ Layer layer0(const Layers &L) {
+  Layer l{};
+  if (L.m0) l = make_layer(*L.m0);
+  l.kind = L.kind;
+  l.kd = L.kd;
+  l.scale = L.scale;
   return l;
 }
-__device__ __forceinline__ int bsdf_ncomp(const Bsdf &b) {
-  return layer_ncomp(b.L0) + (b.nl == 2 ? layer_ncomp(layer1(b)) : 0);
+// The second layer of a mix (nl == 2).
+__device__ __forceinline__ Layer layer1(const Layers &L) {
+  Layer l = make_layer(*L.m1);
+  l.scale = L.s1;
+  return l;
 }
-__device__ __forceinline__ int bsdf_nspec(const Bsdf &b) {
-  return layer_nspec(b.L0) + (b.nl == 2 ? layer_nspec(layer1(b)) : 0);
+__device__ __forceinline__ Layer layer_at(const Layers &L, int i) { return i == 0 ? layer0(L) : layer1(L); }
+__device__ __noinline__ int layers_ncomp(Layers L) {
+  return layer_ncomp(layer0(L)) + (L.nl == 2 ? layer_ncomp(layer1(L)) : 0);
 }
+__device__ __noinline__ int layers_nspec(Layers L) {
+  return layer_nspec(layer0(L)) + (L.nl == 2 ? layer_nspec(layer1(L)) : 0);
+}
+__device__ __forceinline__ int bsdf_ncomp(const Bsdf &b) { return b.L.diffuse() ? 1 : layers_ncomp(b.L); }
+__device__ __forceinline__ int bsdf_nspec(const Bsdf &b) { return b.L.diffuse() ? 0 : layers_nspec(b.L); }
 
 // A layer's non-specular components summed (local frame, unscaled).
 __device__ V3 layer_eval(const Layer &b, V3 wi, V3 wo) {
@@ -577,52 +609,88 @@ __device__ float layer_sample(const Layer &b, int c, V3 wi, float u0, float u1, 
     if (!blinn_sample(b.exponent, wi, u0, u1, wo)) return 0.0f;
     return microfacet_pdf(b, wi, wo);
   }
-  // BxDF::Sample (Core/BxDF.cpp:20-31): cosine hemisphere on the incident side
-  wo = cosine_hemisphere(u0, u1);
-  if (wi.z < 0.0f) wo.z = -wo.z;
+  wo = diffuse_sample(wi, u0, u1);
   return diffuse_pdf(wi, wo);
 }
 
+// The layers' components summed, each layer scaled (local frame).
+__device__ __noinline__ V3 layers_eval(Layers L, V3 wi, V3 wo) {
+  const Layer l0 = layer0(L);
+  const V3 f = mul(l0.scale, layer_eval(l0, wi, wo));
+  if (L.nl == 1) return f;
+  const Layer l = layer1(L);
+  return f + mul(l.scale, layer_eval(l, wi, wo));
+}
 // BSDF::Evaluate (Core/BSDF.cpp:22-40): every non-specular component is a
 // reflection, so directions on opposite sides of the geometric normal give
-// zero; the layers' components are summed, each layer scaled.
-__device__ V3 bsdf_eval(const Bsdf &b, V3 wi_w, V3 wo_w) {
+// zero.
+__device__ __forceinline__ V3 bsdf_eval(const Bsdf &b, V3 wi_w, V3 wo_w) {
   if (!(dot(wi_w, b.ng) * dot(wo_w, b.ng) > 0.0f)) return v3(0, 0, 0);
   const V3 wi = b.local(wi_w), wo = b.local(wo_w);
-  const V3 f = mul(b.L0.scale, layer_eval(b.L0, wi, wo));
-  if (b.nl == 1) return f;
-  const Layer l = layer1(b);
-  return f + mul(l.scale, layer_eval(l, wi, wo));
+  if (b.L.diffuse()) return mul(b.L.scale, diffuse_eval(b.L.kind, b.L.kd, b.L.on_a, b.L.on_b, wi, wo));
+  return layers_eval(b.L, wi, wo);
 }
 
 // The derivative of bsdf_eval with respect to the per-triangle albedo kd of
 // a single-layer matte, plastic or substrate surface (the diffuse term with
 // kd = 1); zero for the others, whose reflectance the albedo does not set.
-__device__ V3 bsdf_eval_dkd(const Bsdf &b, V3 wi_w, V3 wo_w) {
-  const Layer &l = b.L0;
-  const bool albedo = b.nl == 1 && (l.kind == kLambert || l.kind == kOrenNayar || l.kind == kPlastic ||
+__device__ __forceinline__ V3 bsdf_eval_dkd(const Bsdf &b, V3 wi_w, V3 wo_w) {
+  const Layers &l = b.L;
+  const bool albedo = l.nl == 1 && (l.kind == kLambert || l.kind == kOrenNayar || l.kind == kPlastic ||
                                     l.kind == kSubstrate);
   if (!albedo || !(dot(wi_w, b.ng) * dot(wo_w, b.ng) > 0.0f)) return v3(0, 0, 0);
   const V3 wi = b.local(wi_w), wo = b.local(wo_w);
   if (l.kind == kSubstrate) {
     const float t1 = 1.0f - 0.5f * fabsf(wo.z), t2 = 1.0f - 0.5f * fabsf(wi.z);
     const float p1 = t1 * t1 * t1 * t1 * t1, p2 = t2 * t2 * t2 * t2 * t2;
-    return (v3(1.0f, 1.0f, 1.0f) - l.ks) * ((28.0f / (23.0f * kPi)) * (1.0f - p1) * (1.0f - p2));
+    return (v3(1.0f, 1.0f, 1.0f) - load3(l.m0->ks)) * ((28.0f / (23.0f * kPi)) * (1.0f - p1) * (1.0f - p2));
   }
-  Layer u = l;
-  u.kd = v3(1.0f, 1.0f, 1.0f);
-  return diffuse_eval(u, wi, wo);
+  return diffuse_eval(l.kind, v3(1.0f, 1.0f, 1.0f), l.on_a, l.on_b, wi, wo);
 }
 
 // BSDF::PDF (Core/BSDF.cpp:42-58): the average of the non-specular
 // component densities.
-__device__ float bsdf_pdf(const Bsdf &b, V3 wi_w, V3 wo_w) {
-  const int n = bsdf_ncomp(b);
+__device__ __noinline__ float layers_pdf(Layers L, V3 wi, V3 wo) {
+  const Layer l0 = layer0(L);
+  int n = layer_ncomp(l0);
+  if (L.nl == 2) n += layer_ncomp(layer1(L));
   if (n == 0) return 0.0f;
-  const V3 wi = b.local(wi_w), wo = b.local(wo_w);
-  float p = layer_pdf_sum(b.L0, wi, wo);
-  if (b.nl == 2) p += layer_pdf_sum(layer1(b), wi, wo);
+  float p = layer_pdf_sum(l0, wi, wo);
+  if (L.nl == 2) p += layer_pdf_sum(layer1(L), wi, wo);
   return n == 1 ? p : p / n;
+}
+__device__ __forceinline__ float bsdf_pdf(const Bsdf &b, V3 wi_w, V3 wo_w) {
+  const V3 wi = b.local(wi_w), wo = b.local(wo_w);
+  return b.L.diffuse() ? diffuse_pdf(wi, wo) : layers_pdf(b.L, wi, wo);
+}
+
+// Component comp of the layers, sampled: wo and the density averaged over
+// n_all (0: the sample is rejected).
+__device__ __noinline__ float layers_sample(Layers L, int comp, V3 wi, float u0, float u1, int n_all, V3 &wo_out) {
+  const Layer l0 = layer0(L);
+  const int n0 = layer_ncomp(l0);
+  const int n = n0 + (L.nl == 2 ? layer_ncomp(layer1(L)) : 0);
+  V3 wo = v3(0, 0, 0);
+  float pc;
+  int kind;
+  MerlDev merl;
+  if (comp < n0 || L.nl == 1) {
+    pc = layer_sample(l0, comp, wi, u0, u1, wo);
+    kind = l0.kind;
+    merl = l0.merl;
+  } else {
+    const Layer l = layer1(L);
+    pc = layer_sample(l, comp - n0, wi, u0, u1, wo);
+    kind = l.kind;
+    merl = l.merl;
+  }
+  wo_out = wo;
+  if (!(pc > 0.0f)) return 0.0f;
+  if (n == 1 && n_all == 1) return pc;
+  // the sampled component's own density, plus the others' at wo
+  float p = layer_pdf_sum(l0, wi, wo) + (L.nl == 2 ? layer_pdf_sum(layer1(L), wi, wo) : 0.0f);
+  if (kind == kMeasured) p += pc - merl_pdf(merl, wi, wo);  // MERL's sample density as it returned it
+  return p / n_all;
 }
 
 // BSDF::Sample (Core/BSDF.cpp:110-168) over the non-specular components:
@@ -631,37 +699,24 @@ __device__ float bsdf_pdf(const Bsdf &b, V3 wi_w, V3 wo_w) {
 // and average over n_all (the non-specular count for direct lighting;
 // every component, specular ones included, when the caller samples
 // BSDF_ALL), evaluate the whole BSDF.
-__device__ V3 bsdf_sample_c(const Bsdf &b, int comp, V3 wi_w, float u0, float u1, V3 &wo_w, float &pdf, int n_all) {
-  const int n = bsdf_ncomp(b);
+__device__ __forceinline__ V3 bsdf_sample_c(const Bsdf &b, int comp, V3 wi_w, float u0, float u1, V3 &wo_w, float &pdf,
+                                            int n_all) {
   pdf = 0.0f;
   wo_w = wi_w;
-  if (n == 0) return v3(0, 0, 0);
+  if (bsdf_ncomp(b) == 0) return v3(0, 0, 0);
   const V3 wi = b.local(wi_w);
   V3 wo;
-  float pc;
-  int kind;
-  MerlDev merl;
-  const int n0 = layer_ncomp(b.L0);
-  if (comp < n0 || b.nl == 1) {
-    pc = layer_sample(b.L0, comp, wi, u0, u1, wo);
-    kind = b.L0.kind;
-    merl = b.L0.merl;
+  float p;
+  if (b.L.diffuse()) {
+    wo = diffuse_sample(wi, u0, u1);
+    p = diffuse_pdf(wi, wo);
+    if (n_all != 1) p /= n_all;
   } else {
-    const Layer l = layer1(b);
-    pc = layer_sample(l, comp - n0, wi, u0, u1, wo);
-    kind = l.kind;
-    merl = l.merl;
+    p = layers_sample(b.L, comp, wi, u0, u1, n_all, wo);
   }
   wo_w = b.world(wo);
-  if (!(pc > 0.0f)) return v3(0, 0, 0);
-  if (n == 1 && n_all == 1) {
-    pdf = pc;
-  } else {
-    // the sampled component's own density, plus the others' at wo
-    float p = layer_pdf_sum(b.L0, wi, wo) + (b.nl == 2 ? layer_pdf_sum(layer1(b), wi, wo) : 0.0f);
-    if (kind == kMeasured) p += pc - merl_pdf(merl, wi, wo);  // MERL's sample density as it returned it
-    pdf = p / n_all;
-  }
+  if (!(p > 0.0f)) return v3(0, 0, 0);
+  pdf = p;
   return bsdf_eval(b, wi_w, wo_w);
 }
 // The direct-lighting form: a non-specular component picked uniformly with uc.
@@ -756,25 +811,40 @@ __device__ __noinline__ float next_min_t_instance(const SceneDev &S, const Hit &
   return __double2float_ru(fmax(0.0, __dadd_rn(__dmul_rn(mdot, __ddiv_rn(1.0, div)), 1e-14)));
 }
 
-__device__ __forceinline__ float next_min_t(const SceneDev &S, const Hit &h, V3 w) {
-  if (S.prim_inst && S.prim_inst[h.prim]) return next_min_t_instance(S, h, w);
+// What next_min_t needs of the hit triangle, made once per hit.
+struct ExitPlane {
+  V3 n, A;        // normal (e1 x e2) and the componentwise magnitude of its terms
+  float num, en;  // (v0 - p) . n and the bound on its error
+};
+__device__ __forceinline__ ExitPlane exit_plane(const SceneDev &S, const Hit &h) {
   const int i0 = S.tri_vidx[3 * h.g], i1 = S.tri_vidx[3 * h.g + 1], i2 = S.tri_vidx[3 * h.g + 2];
   const V3 p0 = load3(S.vpos + 3 * i0), p1 = load3(S.vpos + 3 * i1), p2 = load3(S.vpos + 3 * i2);
-  const V3 e1 = p1 - p0, e2 = p2 - p0, n = cross(e1, e2), q = p0 - h.p;
+  const V3 e1 = p1 - p0, e2 = p2 - p0, q = p0 - h.p;
+  ExitPlane P;
+  P.n = cross(e1, e2);
   // componentwise magnitude of the cross product, bounding its terms
   const V3 a1 = v3(fabsf(e1.x), fabsf(e1.y), fabsf(e1.z)), a2 = v3(fabsf(e2.x), fabsf(e2.y), fabsf(e2.z));
-  const V3 A = v3(a1.y * a2.z + a1.z * a2.y, a1.z * a2.x + a1.x * a2.z, a1.x * a2.y + a1.y * a2.x);
-  const float num = dot(q, n), den = dot(w, n);
+  P.A = v3(a1.y * a2.z + a1.z * a2.y, a1.z * a2.x + a1.x * a2.z, a1.x * a2.y + a1.y * a2.x);
+  P.num = dot(q, P.n);
   // u = 2^-24: the edges carry <= u relative error, the cross product
   // <= 4u A, q <= u |q|; the dot products add 3u of their magnitude sums
   const float u = 5.9604645e-8f;
-  const float en = 9.0f * u * (fabsf(q.x) * A.x + fabsf(q.y) * A.y + fabsf(q.z) * A.z) + 1e-35f;
-  const float ed = 8.0f * u * (fabsf(w.x) * A.x + fabsf(w.y) * A.y + fabsf(w.z) * A.z) + 1e-35f;
+  P.en = 9.0f * u * (fabsf(q.x) * P.A.x + fabsf(q.y) * P.A.y + fabsf(q.z) * P.A.z) + 1e-35f;
+  return P;
+}
+__device__ __forceinline__ float next_min_t(const SceneDev &S, const Hit &h, const ExitPlane &P, V3 w) {
+  if (S.prim_inst && S.prim_inst[h.prim]) return next_min_t_instance(S, h, w);
+  const float den = dot(w, P.n);
+  const float u = 5.9604645e-8f;
+  const float ed = 8.0f * u * (fabsf(w.x) * P.A.x + fabsf(w.y) * P.A.y + fabsf(w.z) * P.A.z) + 1e-35f;
   const float ad = fabsf(den);
   if (!(ad > 4.0f * ed)) return next_min_t_exact(S, h, w);
-  const float t = num / den;
-  const float et = 1.01f * (en + fabsf(t) * ed) / (ad - ed) + 4.0f * u * fabsf(t);
+  const float t = P.num / den;
+  const float et = 1.01f * (P.en + fabsf(t) * ed) / (ad - ed) + 4.0f * u * fabsf(t);
   return fmaxf(0.0f, __fadd_ru(__fadd_ru(t, et), 1e-14f));
+}
+__device__ __forceinline__ float next_min_t(const SceneDev &S, const Hit &h, V3 w) {
+  return next_min_t(S, h, exit_plane(S, h), w);
 }
 
 // MathRoutines::CoordinateSystem (Math/MathRoutines.h:298-313): the first
@@ -832,35 +902,44 @@ __device__ Bsdf make_bsdf(const SceneDev &S, const Hit &h, int prim) {
   b.n = h.ns;
   b.e1 = shading_tangent(S, h);
   b.e2 = cross(b.n, b.e1);  // BSDF::BSDF (Core/BSDF.h:182-192): e2 = n x tangent
-  b.m1 = nullptr;
-  b.s1 = v3(0, 0, 0);
+  Layers &L = b.L;
+  L.nl = 1;
+  L.m0 = &m;
+  L.m1 = nullptr;
+  L.s1 = v3(0, 0, 0);
+  L.scale = v3(1.0f, 1.0f, 1.0f);
   if (m.kind == kMix) {
     const V3 s0 = load3(m.mix_scale), s1 = v3(1.0f - s0.x, 1.0f - s0.y, 1.0f - s0.z);
     const bool has0 = !black(s0), has1 = !black(s1) && m.mix[1] >= 0;
-    b.nl = has0 && has1 ? 2 : 1;
     if (has0) {
-      b.L0 = make_layer(S.materials[m.mix[0]]);
-      b.L0.scale = s0;
+      L.m0 = S.materials + m.mix[0];
+      L.scale = s0;
       if (has1) {
-        b.m1 = S.materials + m.mix[1];
-        b.s1 = s1;
+        L.nl = 2;
+        L.m1 = S.materials + m.mix[1];
+        L.s1 = s1;
       }
     } else if (has1) {
-      b.L0 = make_layer(S.materials[m.mix[1]]);
-      b.L0.scale = s1;
-    } else {  // nothing scatters
-      b.L0 = make_layer(m);
-      b.L0.kind = kTransparent;
-      b.L0.kd = b.L0.ks = v3(0, 0, 0);
+      L.m0 = S.materials + m.mix[1];
+      L.scale = s1;
+    } else {
+      L.m0 = nullptr;
     }
+  }
+  if (!L.m0) {  // nothing scatters
+    L.kind = kTransparent;
+    L.kd = v3(0, 0, 0);
+    L.on_a = L.on_b = 0.0f;
     return b;
   }
-  b.nl = 1;
-  b.L0 = make_layer(m);
-  if (S.tri_albedo && m.kind != kTransparent && m.kind != kUber) {
+  L.kind = L.m0->kind;
+  L.kd = load3(L.m0->kd);
+  L.on_a = L.m0->on_a;
+  L.on_b = L.m0->on_b;
+  if (m.kind != kMix && S.tri_albedo && m.kind != kTransparent && m.kind != kUber) {
     const float *ta = S.tri_albedo + 3 * (int64_t)h.g;
-    if (ta[0] == ta[0]) b.L0.kd = v3(fminf(1.0f, fmaxf(0.0f, ta[0])), fminf(1.0f, fmaxf(0.0f, ta[1])),
-                                     fminf(1.0f, fmaxf(0.0f, ta[2])));
+    if (ta[0] == ta[0]) L.kd = v3(fminf(1.0f, fmaxf(0.0f, ta[0])), fminf(1.0f, fmaxf(0.0f, ta[1])),
+                                  fminf(1.0f, fmaxf(0.0f, ta[2])));
   }
   return b;
 }
@@ -883,8 +962,8 @@ __device__ __forceinline__ V3 layer_spec_t(const Layer &l) {
 // weight is black or the direction grazes the shading plane.  (A BSDF has
 // at most one specular reflection: the host refuses mixes of two.)
 __device__ __forceinline__ bool specular_reflect(const Bsdf &b, V3 wo_w, V3 &dir, V3 &val) {
-  for (int i = 0; i < b.nl; ++i) {
-    const Layer l = i == 0 ? b.L0 : layer1(b);
+  for (int i = 0; i < b.L.nl; ++i) {
+    const Layer l = layer_at(b.L, i);
     const V3 r = layer_spec_r(l);
     if (black(r)) continue;
     const V3 wi = b.local(wo_w);
@@ -902,8 +981,8 @@ __device__ __forceinline__ bool specular_reflect(const Bsdf &b, V3 wo_w, V3 &dir
 // leaving); false on total internal reflection (black weight), at
 // normal-grazing incidence, or when the BSDF has no transmission component.
 __device__ __forceinline__ bool specular_transmit(const Bsdf &b, V3 wo_w, V3 &dir, V3 &val) {
-  for (int i = 0; i < b.nl; ++i) {
-    const Layer l = i == 0 ? b.L0 : layer1(b);
+  for (int i = 0; i < b.L.nl; ++i) {
+    const Layer l = layer_at(b.L, i);
     const V3 t = layer_spec_t(l);
     if (black(t)) continue;
     const float cn = dot(wo_w, b.n);
@@ -1030,7 +1109,7 @@ __device__ float box_solid_angle(V3 p, const float lo[3], const float hi[3]) {
 // weight of area light `li`: solid angle of its bounds times its intensity
 // times the average (clamped) cosine of the bounds' corners, pi * intensity
 // inside the bounds.
-__device__ float light_weight(const AreaLight &L, V3 p, V3 n) {
+__device__ __noinline__ float light_weight(const AreaLight &L, V3 p, V3 n) {
   if (p.x >= L.lo[0] && p.y >= L.lo[1] && p.z >= L.lo[2] && p.x <= L.hi[0] && p.y <= L.hi[1] && p.z <= L.hi[2])
     return kPi * L.intensity;
   float avg = 0.0f;
@@ -1046,9 +1125,8 @@ __device__ float light_weight(const AreaLight &L, V3 p, V3 n) {
 
 // Probability of choosing light `li` at (p, n) among all area lights
 // (_Weights_To_CDF: equal probabilities when every weight is 0).
-__device__ float light_choice_pdf(const SceneDev &S, int li, V3 p, V3 n) {
+__device__ __noinline__ float light_choice_pdf_many(const SceneDev &S, int li, V3 p, V3 n) {
   const int nl = S.n_area_lights;
-  if (nl <= 1) return 1.0f;
   float tot = 0.0f, mine = 0.0f;
   for (int i = 0; i < nl; ++i) {
     const float w = light_weight(S.area_lights[i], p, n);
@@ -1057,17 +1135,15 @@ __device__ float light_choice_pdf(const SceneDev &S, int li, V3 p, V3 n) {
   }
   return tot > 0.0f ? mine / tot : 1.0f / nl;
 }
+__device__ __forceinline__ float light_choice_pdf(const SceneDev &S, int li, V3 p, V3 n) {
+  return S.n_area_lights <= 1 ? 1.0f : light_choice_pdf_many(S, li, p, n);
+}
 
 // Chooses a light with u (BinarySearchCDF over the normalised cumulative
 // weights); returns its index, its probability and the remainder of u
 // rescaled to [0, 1) for the triangle choice.
-__device__ int choose_light(const SceneDev &S, float u, V3 p, V3 n, float &pdf, float &u_rest) {
+__device__ __noinline__ int choose_light_many(const SceneDev &S, float u, V3 p, V3 n, float &pdf, float &u_rest) {
   const int nl = S.n_area_lights;
-  if (nl <= 1) {
-    pdf = 1.0f;
-    u_rest = u;
-    return 0;
-  }
   float tot = 0.0f;
   for (int i = 0; i < nl; ++i) tot += light_weight(S.area_lights[i], p, n);
   const bool uniform = !(tot > 0.0f);
@@ -1098,6 +1174,12 @@ __device__ int choose_light(const SceneDev &S, float u, V3 p, V3 n, float &pdf, 
   }
   u_rest = pdf > 0.0f ? fminf(fmaxf((u - prev) / pdf, 0.0f), 0.99999994f) : 0.0f;
   return li;
+}
+__device__ __forceinline__ int choose_light(const SceneDev &S, float u, V3 p, V3 n, float &pdf, float &u_rest) {
+  if (S.n_area_lights > 1) return choose_light_many(S, u, p, n, pdf, u_rest);
+  pdf = 1.0f;
+  u_rest = u;
+  return 0;
 }
 
 // BBox3D::Intersect (Math/BBox3D.h:150-171) of the ray segment [t0, t1] with
