@@ -189,7 +189,13 @@ struct Bsdf {
   V3 n, e1, e2, ng;  // shading frame and geometric normal
   Layers L;
   __device__ __forceinline__ V3 local(V3 w) const { return v3(dot(w, e1), dot(w, e2), dot(w, n)); }
-  __device__ __forceinline__ V3 world(V3 l) const { return e1 * l.x + e2 * l.y + n * l.z; }
+  // Fused as written in every kernel: a direction that differs by a rounding
+  // sends a photon elsewhere, and left to the compiler the sums are fused one
+  // way or another with what surrounds them.
+  __device__ __forceinline__ V3 world(V3 l) const {
+    return v3(fmaf(n.x, l.z, fmaf(e2.x, l.y, e1.x * l.x)), fmaf(n.y, l.z, fmaf(e2.y, l.y, e1.y * l.x)),
+              fmaf(n.z, l.z, fmaf(e2.z, l.y, e1.z * l.x)));
+  }
 };
 
 // FresnelDielectric(inner, 1)::operator() (Core/Fresnel.h:96-124).
