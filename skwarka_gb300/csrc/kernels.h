@@ -53,14 +53,14 @@ cudaError_t launch_traversal_d(bool closest, int stack_cap, const void *nodes, c
 
 
 // A tree's normal ids on the device: uint16 per photon, then at nids_offset
-// the same normals as 4 floats each (launch_normals fills them from the ids;
-// dirs: direction_table_device()).
+// its node records, each node with its photon's normal as 4 floats (filled
+// by launch_node_records; dirs: direction_table_device()).
 __host__ __device__ inline size_t nids_offset(int64_t n) { return ((size_t)n * 2 + 255) & ~(size_t)255; }
-inline size_t nids_bytes(int64_t n) { return nids_offset(n) + (size_t)(n > 0 ? n : 1) * 16; }
-cudaError_t launch_normals(uint16_t *nids, int64_t n, const double *dirs, cudaStream_t st);
+inline size_t nids_bytes(int64_t n) { return nids_offset(n) + (size_t)(n > 0 ? n : 1) * 32; }
+cudaError_t launch_node_records(const void *nodes, uint16_t *nids, int64_t n, const double *dirs, cudaStream_t st);
 
-// Photon kd-tree lookups (knn.cu).  nodes: KdNode[n]; nids: uint16 normal
-// id per node; dirs: direction_table_device() (3 doubles per 16-bit
+// Photon kd-tree lookups (knn.cu).  nodes: KdNode[n]; nids: normal ids and
+// node records (above); dirs: direction_table_device() (3 doubles per 16-bit
 // direction id, then the same as 3 floats per id); q / qn: 3 doubles
 // per query (qn may be null when cos_t < 0, which disables the filter).
 // Outputs per query: k slots of tree positions and squared distances in the

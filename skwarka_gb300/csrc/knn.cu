@@ -25,12 +25,11 @@
 // Double products and sums use round-to-nearest intrinsics so that no fused
 // multiply-add changes a result.
 //
-// Layout: 16-byte nodes (x, y, z, word) read with one vector load; the
-// photons' normals (float4, behind their 16-bit ids) are read only for points
-// inside the radius.
-// The walk stack lives in shared memory; for k <= 128 the heap (8-byte
-// entries: float key, tree position) lives in local memory, larger k use a
-// heap in a caller-provided global scratch buffer of k entries per query.
+// Layout: 16-byte nodes (x, y, z, word) read with one vector load, or 32-byte
+// records of a node and its photon's normal (struct Tree).  The walk stack
+// lives in shared memory, and so does the heap for k <= 128 (one word per
+// entry); larger k use a heap in a caller-provided global scratch buffer of k
+// entries per query.
 #include <cuda.h>
 #include <cuda_runtime.h>
 
@@ -61,40 +60,49 @@ namespace {
 #define SKW_KNN_BLOCK 32
 #endif
 constexpr int kKnnBlock = SKW_KNN_BLOCK;  // threads per block of the lookup kernels
-// Minimum resident blocks per SM: 32 one-warp blocks bound the registers at
-// 64.  Heaps of more than 32 entries leave room for at most 28 blocks, at
-// k = 100 for 14, so that kernel is bound at 128 (k = 100, 669,824 queries:
-// 7.44 -> 7.29 ms).
+// Minimum resident blocks per SM of k_knn and k_nearest: 32 one-warp blocks
+// bound the registers at 64, too few for heaps of up to 32 entries (28 blocks,
+// 72 registers: 669,824 filtered queries of k = 32 2.04 -> 1.97 ms; 24 blocks
+// are slower for k = 1); larger ones leave room for 16 or fewer.
 #ifndef SKW_KNN_MINB
 #define SKW_KNN_MINB (1024 / SKW_KNN_BLOCK)
 #endif
+constexpr int knn_min_blocks(int kmax) { return kmax == 128 ? 16 : kmax == 32 ? 28 : SKW_KNN_MINB; }
 
+constexpr float kKe1 = 6.2e-7f;
 
+// The doubles stay where the caller put them: only what float cannot decide
+// reads them (16 registers less, which the walks need).
 struct Query {
-  double q[3];
-  double n[3];
-  double cos_t, sin_t;
+  const double *q, *n;  // n: where the filter is on
+  double cos_t;
   bool filter;
   float qf[3];  // q rounded up to float
-  float eq;     // max |q - qf| over the axes
+  float dq[3];  // q - qf in float
+  float e0;     // max |q - qf| over the axes
+  float eq;     // what a float difference may be off besides its relative roundings (dist2f)
   float nf[3];  // the normal in float (filter pre-test)
   float cos_f, sin_f;  // cos_t, sin_t in float (filter pre-test)
-  float ke0, ke1;      // error bound of a float squared distance k: ke0 + ke1 k (key_err)
+  float ke0;           // a float squared distance k is within ke0 + kKe1 k of the exact one
 };
+
+__device__ __forceinline__ double sin_of(double cos_t) { return __dsqrt_rn(__dsub_rn(1.0, __dmul_rn(cos_t, cos_t))); }
 
 // Fills the float copy of the query point used by the pre-tests.
 __device__ __forceinline__ void query_float(Query &Q) {
   float e = 0.0f;
   for (int k = 0; k < 3; ++k) {
-    Q.qf[k] = __double2float_ru(Q.q[k]);
-    e = fmaxf(e, (float)fabs(Q.q[k] - (double)Q.qf[k]));
-    Q.nf[k] = (float)Q.n[k];
+    const double qk = __ldg(Q.q + k);
+    Q.qf[k] = __double2float_ru(qk);
+    Q.dq[k] = (float)(qk - (double)Q.qf[k]);
+    e = fmaxf(e, fabsf(Q.dq[k]));
+    Q.nf[k] = Q.filter ? (float)__ldg(Q.n + k) : 0.0f;
   }
-  Q.eq = e * 1.0001f;
-  Q.ke0 = 1.001f * (Q.eq + 9.0f * Q.eq * Q.eq) + 1e-37f;
-  Q.ke1 = 3.003f * Q.eq + 6.0e-7f;
+  Q.e0 = e * 1.0001f;
+  Q.eq = e * 1.2e-7f;  // 2u e, rounded up
+  Q.ke0 = 1.76e7f * Q.eq * Q.eq + 1e-37f;
   Q.cos_f = (float)Q.cos_t;
-  Q.sin_f = (float)Q.sin_t;
+  Q.sin_f = (float)sin_of(Q.cos_t);
 }
 
 // Coordinates of the query by a run-time axis, selected without indexing so
@@ -102,15 +110,39 @@ __device__ __forceinline__ void query_float(Query &Q) {
 __device__ __forceinline__ float qf_at(const Query &Q, uint32_t a) {
   return a == 0 ? Q.qf[0] : (a == 1 ? Q.qf[1] : Q.qf[2]);
 }
+__device__ __forceinline__ float dq_at(const Query &Q, uint32_t a) {
+  return a == 0 ? Q.dq[0] : (a == 1 ? Q.dq[1] : Q.dq[2]);
+}
 __device__ __forceinline__ double q_at(const Query &Q, uint32_t a) {
-  return a == 0 ? Q.q[0] : (a == 1 ? Q.q[1] : Q.q[2]);
+  return __ldg(Q.q + a);
 }
 
-// The normals as floats, behind the ids (kernels.h, nids_bytes): one load per
-// accepted point instead of the id and then its entry in the 768 KB table.
-__device__ __forceinline__ const float4 *node_normals(const uint16_t *nids, int n) {
-  return reinterpret_cast<const float4 *>(reinterpret_cast<const char *>(nids) + nids_offset(n));
-}
+// A tree as the lookups read it: its 16-byte nodes, and its records of a node
+// and its photon's normal (4 floats; kernels.h, nids_bytes).  A record is one
+// load, of the sector that the node alone would take, so walks with the filter
+// and registers to spare read those; the others read the nodes, of which twice
+// as many fit into L1, and a normal once the distance is known.
+struct NodeN {
+  float4 p, m;
+};
+struct Tree {
+  const float4 *nodes, *records;
+  int n;
+  __device__ __forceinline__ float4 at(int i) const { return __ldg(nodes + i); }
+  __device__ __forceinline__ float4 normal(int i) const { return __ldg(records + 2 * (int64_t)i + 1); }
+  __device__ __forceinline__ NodeN load(int i, bool with_normal) const {
+    NodeN r;
+    if (with_normal) {
+      asm("ld.global.nc.v8.f32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
+          : "=f"(r.p.x), "=f"(r.p.y), "=f"(r.p.z), "=f"(r.p.w), "=f"(r.m.x), "=f"(r.m.y), "=f"(r.m.z), "=f"(r.m.w)
+          : "l"(records + 2 * (int64_t)i));
+    } else {
+      r.p = __ldg(nodes + i);
+      r.m = make_float4(0, 0, 0, 0);
+    }
+    return r;
+  }
+};
 
 // PhotonFilter::operator() (PhotonInternalTypes.h:127-133), with float
 // pre-tests: the normal's cosine and the in-plane test are decided in float
@@ -118,9 +150,9 @@ __device__ __forceinline__ const float4 *node_normals(const uint16_t *nids, int 
 // vectors: a few 1e-7), else in double as the reference computes them.
 __device__ __forceinline__ bool photon_filter_exact(const Query &Q, const float4 p, uint16_t nid,
                                                     const double *__restrict__ dirs);
-__device__ __forceinline__ bool photon_filter(const Query &Q, const float4 p, int i, const uint16_t *__restrict__ nids,
-                                              const float4 *__restrict__ nrm, const double *__restrict__ dirs) {
-  const float4 m = __ldg(nrm + i);
+__device__ __forceinline__ bool photon_filter(const Query &Q, const NodeN &node, int i,
+                                              const uint16_t *__restrict__ nids, const double *__restrict__ dirs) {
+  const float4 p = node.p, m = node.m;
   const float cf = m.x * Q.nf[0] + m.y * Q.nf[1] + m.z * Q.nf[2];
   const float ct = Q.cos_f;
   if (cf < ct - 2e-6f) return false;
@@ -131,11 +163,11 @@ __device__ __forceinline__ bool photon_filter(const Query &Q, const float4 p, in
     const float l2 = tx * tx + ty * ty + tz * tz;
     const float st = Q.sin_f;
     const float lhs = dn * dn, rhs = st * st * l2;
-    // error: the float query rounding eq on each component plus relative rounding
+    // error: the float query's rounding e0 on each component plus relative rounding
     const float a = fabsf(tx) + fabsf(ty) + fabsf(tz);
-    // |d(dn)| <= 3 eq + 5e-7 a and |d(l2)| <= 2 a (eq + 6e-8 a) (a = |tx| + |ty| + |tz|), so
+    // |d(dn)| <= 3 e0 + 5e-7 a and |d(l2)| <= 2 a (e0 + 6e-8 a) (a = |tx| + |ty| + |tz|), so
     // the squares move by at most 2 a |d(dn)| + |d(dn)|^2 and st^2 |d(l2)|
-    const float err = 12.0f * Q.eq * (a + Q.eq) + 4e-6f * a * a + 2e-6f * (lhs + rhs) + 1e-37f;
+    const float err = 12.0f * Q.e0 * (a + Q.e0) + 4e-6f * a * a + 2e-6f * (lhs + rhs) + 1e-37f;
     if (lhs + err < rhs) return true;
     if (lhs - err > rhs) return false;
   }
@@ -145,42 +177,48 @@ __device__ __forceinline__ bool photon_filter(const Query &Q, const float4 p, in
 __device__ __forceinline__ bool photon_filter_exact(const Query &Q, const float4 p, uint16_t nid,
                                                     const double *__restrict__ dirs) {
   const double nx = __ldg(dirs + 3 * nid), ny = __ldg(dirs + 3 * nid + 1), nz = __ldg(dirs + 3 * nid + 2);
-  const double cosn = __dadd_rn(__dadd_rn(__dmul_rn(nx, Q.n[0]), __dmul_rn(ny, Q.n[1])), __dmul_rn(nz, Q.n[2]));
+  const double qx = __ldg(Q.q), qy = __ldg(Q.q + 1), qz = __ldg(Q.q + 2);
+  const double mx = __ldg(Q.n), my = __ldg(Q.n + 1), mz = __ldg(Q.n + 2);
+  const double cosn = __dadd_rn(__dadd_rn(__dmul_rn(nx, mx), __dmul_rn(ny, my)), __dmul_rn(nz, mz));
   if (!(cosn > Q.cos_t)) return false;
-  const double tx = __dsub_rn((double)p.x, Q.q[0]), ty = __dsub_rn((double)p.y, Q.q[1]),
-               tz = __dsub_rn((double)p.z, Q.q[2]);
-  const double dotn = __dadd_rn(__dadd_rn(__dmul_rn(tx, Q.n[0]), __dmul_rn(ty, Q.n[1])), __dmul_rn(tz, Q.n[2]));
+  const double tx = __dsub_rn((double)p.x, qx), ty = __dsub_rn((double)p.y, qy), tz = __dsub_rn((double)p.z, qz);
+  const double dotn = __dadd_rn(__dadd_rn(__dmul_rn(tx, mx), __dmul_rn(ty, my)), __dmul_rn(tz, mz));
   const double len = __dsqrt_rn(__dadd_rn(__dadd_rn(__dmul_rn(tx, tx), __dmul_rn(ty, ty)), __dmul_rn(tz, tz)));
-  return fabs(dotn) < __dmul_rn(Q.sin_t, len);
+  return fabs(dotn) < __dmul_rn(sin_of(Q.cos_t), len);
 }
 
-__device__ __forceinline__ double point_d2(const float4 p, const Query &Q) {
-  const double dx = __dsub_rn((double)p.x, Q.q[0]), dy = __dsub_rn((double)p.y, Q.q[1]),
-               dz = __dsub_rn((double)p.z, Q.q[2]);
+__device__ __forceinline__ double point_d2(const float4 p, const double *__restrict__ q) {
+  const double dx = __dsub_rn((double)p.x, __ldg(q)), dy = __dsub_rn((double)p.y, __ldg(q + 1)),
+               dz = __dsub_rn((double)p.z, __ldg(q + 2));
   return __dadd_rn(__dadd_rn(__dmul_rn(dx, dx), __dmul_rn(dy, dy)), __dmul_rn(dz, dz));
 }
+
+__device__ __forceinline__ double point_d2(const float4 p, const Query &Q) { return point_d2(p, Q.q); }
 
 // Float pre-tests.  A point's squared distance and a splitting plane's
 // squared distance are first computed in float and compared with two
 // thresholds derived from the current radius and a bound on the float
 // value's distance from the reference's double value; only a value between
 // the thresholds is decided in double.
-// The float squared distance of a point from the float query, and a bound
-// E(F) on its distance from the reference's double value, as a function of
-// the float value F: with u = 2^-24, each float difference d within u|d| +
-// eq of the exact one, its square, the fused sum's three roundings and the
-// double result's own rounding give
-//   |F - d2| <= 5u D + 2 eq sum|d| + 3 eq^2 (+ 2^-52 D),  D = sum d^2 <= F (1 + 3u),
-// and sum|d| <= sqrt(3 D):  E(F) = 3.0e-7 F + 3.47 eq sqrt(F) + 3.01 eq^2,
+// A difference from the query is (p - qf) - dq: with u = 2^-24 and e the
+// largest |dq|, the two subtractions and dq's own rounding put it within
+// 2u|d| + 2u e =: 2u|d| + eq of the exact difference d.  (Without dq the
+// difference is off by e itself: near keys of a heap, a millionth of the
+// coordinates apart, could then not be told apart in float, and the double
+// comparisons of some lane held up nearly every heap operation of a warp.)
+// The squared distance F from those differences, its fused sum's three
+// roundings and the double result's own rounding give
+//   |F - d2| <= 7u D + 2 eq sum|d| + 3 eq^2 (+ 2^-52 D),  D = sum d^2 <= F (1 + 5u),
+// and sum|d| <= sqrt(3 D):  E(F) = 4.3e-7 F + 3.47 eq sqrt(F) + 3.01 eq^2,
 // plus 1e-37 for roundings in the subnormal range.  A plane's squared
-// distance (one axis, one rounding fewer) is within the same bound.
+// distance (one axis, two roundings fewer) is within the same bound.
 __device__ __forceinline__ float dist2f(const float4 p, const Query &Q) {
-  const float dx = p.x - Q.qf[0], dy = p.y - Q.qf[1], dz = p.z - Q.qf[2];
+  const float dx = (p.x - Q.qf[0]) - Q.dq[0], dy = (p.y - Q.qf[1]) - Q.dq[1], dz = (p.z - Q.qf[2]) - Q.dq[2];
   return fmaf(dz, dz, fmaf(dy, dy, dx * dx));
 }
 __device__ __forceinline__ float d2_err(const Query &Q, float x) {
   // 1.0001: the roundings of this float evaluation (about 6u)
-  return (3.0e-7f * x + 3.47f * Q.eq * __fsqrt_ru(x) + 3.01f * Q.eq * Q.eq + 1e-37f) * 1.0001f;
+  return (4.3e-7f * x + 3.47f * Q.eq * __fsqrt_ru(x) + 3.01f * Q.eq * Q.eq + 1e-37f) * 1.0001f;
 }
 // Thresholds on a float squared distance F against a radius known to lie
 // in [rlo, rhi]: F < tin => inside, F >= tout => outside (else decide in
@@ -206,7 +244,7 @@ __device__ __forceinline__ void node_children(const float4 p, int cur, int n, co
   near = far = -1;
   s2 = 0.0f;
   if (axis == 3u) return;
-  const float split = axis == 0 ? p.x : (axis == 1 ? p.y : p.z), q = qf_at(Q, axis), sd = q - split;
+  const float split = axis == 0 ? p.x : (axis == 1 ? p.y : p.z), q = qf_at(Q, axis), sd = (q - split) + dq_at(Q, axis);
   s2 = sd * sd;
   const uint32_t right = w >> 3;
   const int l = (w & 4u) != 0u ? cur + 1 : -1, r = right < (uint32_t)n ? (int)right : -1;
@@ -220,6 +258,18 @@ __device__ __forceinline__ double plane_d2(const float4 p, const Query &Q) {
   const uint32_t axis = __float_as_uint(p.w) & 3u;
   const double pd = __dsub_rn(q_at(Q, axis), (double)(axis == 0 ? p.x : (axis == 1 ? p.y : p.z)));
   return __dmul_rn(pd, pd);
+}
+
+// The node whose child `child` is: the tree lies in pre-order, so the descent
+// from the root goes right where `child` is not before the right child.
+__device__ __noinline__ int node_parent(Tree T, int child) {
+  int cur = 0;
+  for (int next = 0; cur < child; cur = next) {
+    const uint32_t right = __float_as_uint(T.at(cur).w) >> 3;
+    next = right < (uint32_t)T.n && child >= (int)right ? (int)right : cur + 1;
+    if (next == child) break;
+  }
+  return cur;
 }
 
 // The search radius of a walk: max_dist^2 (KDTree::Lookup, KDTree.h:475-482)
@@ -238,14 +288,13 @@ struct Radius {
   }
   // cut: how far `key` may be from the photon's, relative to itself
   __device__ __forceinline__ void set(const Query &Q, int photon, float key, float cut) {
-    const float e = 1.0001f * fmaf(Q.ke1 + cut, key, Q.ke0);
+    const float e = 1.0001f * fmaf(kKe1 + cut, key, Q.ke0);
     idx = photon;
     radius_thresholds(Q, __fsub_rd(key, e), __fadd_ru(key, e), tin, tout);
   }
-  __device__ __forceinline__ double get(const float4 *__restrict__ nodes, const Query &Q,
-                                        const int32_t *ids = nullptr) {
+  __device__ __forceinline__ double get(const Tree &T, const Query &Q, const int32_t *ids = nullptr) {
     if (idx >= 0) {
-      exact = point_d2(__ldg(nodes + (ids ? ids[idx] : idx)), Q);
+      exact = point_d2(T.at(ids ? ids[idx] : idx), Q);
       idx = -1;
     }
     return exact;
@@ -253,21 +302,23 @@ struct Radius {
 };
 
 // The walk stack lives in shared memory ([entry][thread], so lanes never
-// share a bank) and holds only the parent of each postponed far child: on pop
+// share a bank).  k_knn's entry is the parent of a postponed far child: on pop
 // the parent is read again (a recently visited node, usually still in L1) and
-// its split gives both the far child and the plane distance to re-test.
-// Shared memory and L1 share the SM's storage, and the walk's node and heap
-// reads want the L1, so the stack is sized by the tree's depth: the
-// median-split tree of n points is floor(log2 n) + 1 levels deep and the
-// walk holds at most one entry per level, so S = 20 serves n < 2^20 and
-// S = 32 any n < 2^31.
+// its split gives both the far child and the plane distance to re-test.  Shared
+// memory and L1 share the SM's storage, and the walk's reads want the L1, so
+// the stack is sized by the tree's depth: the median-split tree of n points is
+// floor(log2 n) + 1 levels deep and the walk holds at most one entry per level,
+// so S = 20 serves n < 2^20 and S = 32 any n < 2^31.  k_knn_gang and the nearest
+// points' walks, whose L1 holds little or whose pops are most of the work, keep
+// the far child and its plane's float distance instead, and look the parent up
+// (node_parent) when that does not decide.
 
 // ------------------------------------------------------------ k_knn --
 // The heap holds float squared distances: an entry's key is the float
-// distance of its point (dist2f), within ke0 + ke1 key of the reference's
-// double value (Query::ke0, ke1): that bounds the error derived above,
-// 5u D + 2 sqrt(3) eq sqrt(D) + 3 eq^2, the square-root term by
-// 2 sqrt(3) eq sqrt(key) <= 2 sqrt(1.001 eq * 3.003 eq key) <= 1.001 eq + 3.003 eq key.
+// distance of its point (dist2f), within ke0 + kKe1 key of the reference's
+// double value: that bounds the error derived above, 7u D + 2 sqrt(3) eq
+// sqrt(D) + 3 eq^2, the square-root term by
+// 2 sqrt(3) eq sqrt(D) <= sqrt(3) (1e7 eq^2 + 1e-7 D).
 // Heap comparisons are decided on the keys and their bounds, and only when
 // two keys' intervals overlap are the exact doubles of both points computed
 // (GB300 runs a double operation at ~1/64 of the float rate, and divergent
@@ -291,19 +342,19 @@ __host__ __device__ __forceinline__ int64_t knn_heap_stride(int k) { return ((in
 
 // (d2, idx) lexicographic on the exact distances, decided on the keys when
 // their bounds do not overlap.
-__device__ __forceinline__ bool fcand_less(const float4 *__restrict__ nodes, const Query &Q, const FCand &a,
+__device__ __forceinline__ bool fcand_less(const Tree &T, const Query &Q, const FCand &a,
                                            const FCand &b) {
   // decided when |a - b| exceeds both bounds (with a margin for this float arithmetic)
-  const float d = a.key - b.key, tol = 1.0001f * fmaf(Q.ke1, a.key + b.key, 2.0f * Q.ke0);
+  const float d = a.key - b.key, tol = 1.0001f * fmaf(kKe1, a.key + b.key, 2.0f * Q.ke0);
   if (d < -tol) return true;
   if (d > tol) return false;
-  const double da = point_d2(__ldg(nodes + a.idx), Q), db = point_d2(__ldg(nodes + b.idx), Q);
+  const double da = point_d2(T.at(a.idx), Q), db = point_d2(T.at(b.idx), Q);
   return da == db ? a.idx < b.idx : da < db;
 }
 
-__device__ __forceinline__ void fheap_push_up(const float4 *__restrict__ nodes, const Query &Q, FCand *h, int hole, int top, FCand value) {
+__device__ __forceinline__ void fheap_push_up(const Tree &T, const Query &Q, FCand *h, int hole, int top, FCand value) {
   int parent = (hole - 1) / 2;
-  while (hole > top && fcand_less(nodes, Q, h[parent], value)) {
+  while (hole > top && fcand_less(T, Q, h[parent], value)) {
     h[hole] = h[parent];
     hole = parent;
     parent = (hole - 1) / 2;
@@ -314,7 +365,7 @@ __device__ __forceinline__ void fheap_push_up(const float4 *__restrict__ nodes, 
 // PAIR: h[1] is 16-byte aligned, so that the children 2j+1, 2j+2 of every
 // entry j share one 16-byte load.
 template <bool PAIR = false>
-__device__ __forceinline__ void fheap_adjust(const float4 *__restrict__ nodes, const Query &Q, FCand *h, int hole, int len, FCand value) {
+__device__ __forceinline__ void fheap_adjust(const Tree &T, const Query &Q, FCand *h, int hole, int len, FCand value) {
   const int top = hole;
   int second = hole;
   while (second < (len - 1) / 2) {
@@ -322,11 +373,11 @@ __device__ __forceinline__ void fheap_adjust(const float4 *__restrict__ nodes, c
     if (PAIR) {
       const uint4 two = *reinterpret_cast<const uint4 *>(h + second - 1);
       const FCand a{__uint_as_float(two.x), (int32_t)two.y}, b{__uint_as_float(two.z), (int32_t)two.w};
-      const bool left = fcand_less(nodes, Q, b, a);
+      const bool left = fcand_less(T, Q, b, a);
       second -= left ? 1 : 0;
       h[hole] = left ? a : b;
     } else {
-      if (fcand_less(nodes, Q, h[second], h[second - 1])) second--;
+      if (fcand_less(T, Q, h[second], h[second - 1])) second--;
       h[hole] = h[second];
     }
     hole = second;
@@ -336,33 +387,23 @@ __device__ __forceinline__ void fheap_adjust(const float4 *__restrict__ nodes, c
     h[hole] = h[second - 1];
     hole = second - 1;
   }
-  fheap_push_up(nodes, Q, h, hole, top, value);
+  fheap_push_up(T, Q, h, hole, top, value);
 }
 
-__device__ __forceinline__ void fheap_make(const float4 *__restrict__ nodes, const Query &Q, FCand *h, int len) {
+__device__ __forceinline__ void fheap_make(const Tree &T, const Query &Q, FCand *h, int len) {
   if (len < 2) return;
   for (int parent = (len - 2) / 2;; --parent) {
-    fheap_adjust(nodes, Q, h, parent, len, h[parent]);
+    fheap_adjust(T, Q, h, parent, len, h[parent]);
     if (parent == 0) return;
   }
 }
 
 __device__ __forceinline__ void load_query(Query &Q, const double *__restrict__ q, const double *__restrict__ qn,
                                            int64_t i, double cos_t) {
-  Q.q[0] = q[3 * i];
-  Q.q[1] = q[3 * i + 1];
-  Q.q[2] = q[3 * i + 2];
+  Q.q = q + 3 * i;
   Q.filter = cos_t >= 0.0;
-  if (Q.filter) {
-    Q.n[0] = qn[3 * i];
-    Q.n[1] = qn[3 * i + 1];
-    Q.n[2] = qn[3 * i + 2];
-    Q.cos_t = cos_t;
-    Q.sin_t = __dsqrt_rn(__dsub_rn(1.0, __dmul_rn(cos_t, cos_t)));
-  } else {
-    Q.n[0] = Q.n[1] = Q.n[2] = 0.0;
-    Q.cos_t = Q.sin_t = 0.0;
-  }
+  Q.n = Q.filter ? qn + 3 * i : nullptr;
+  Q.cos_t = cos_t;
   query_float(Q);
 }
 
@@ -379,15 +420,15 @@ __device__ __forceinline__ void load_query(Query &Q, const double *__restrict__ 
 struct GlobalHeap {
   FCand *h;
   __device__ __forceinline__ void add(int i, float key, int32_t photon) { h[i] = FCand{key, photon}; }
-  __device__ __forceinline__ void make(const float4 *__restrict__ nodes, const Query &Q, int k) {
-    fheap_make(nodes, Q, h, k);
+  __device__ __forceinline__ void make(const Tree &T, const Query &Q, int k) {
+    fheap_make(T, Q, h, k);
   }
-  __device__ __forceinline__ void replace(const float4 *__restrict__ nodes, const Query &Q, int k, float key,
+  __device__ __forceinline__ void replace(const Tree &T, const Query &Q, int k, float key,
                                           int32_t photon) {
     const FCand back = h[k - 1];
     h[k - 1] = h[0];
-    fheap_adjust<true>(nodes, Q, h, 0, k - 1, back);
-    fheap_push_up(nodes, Q, h, k - 1, 0, FCand{key, photon});
+    fheap_adjust<true>(T, Q, h, 0, k - 1, back);
+    fheap_push_up(T, Q, h, k - 1, 0, FCand{key, photon});
   }
   __device__ __forceinline__ int32_t photon(int i) const { return h[i].idx; }
   __device__ __forceinline__ void top(const Query &Q, Radius &r) const { r.set(Q, h[0].idx, h[0].key, 0.0f); }
@@ -395,81 +436,96 @@ struct GlobalHeap {
 
 // Heaps in shared memory (k <= 128), one word per entry: the key with its low
 // 7 bits replaced by the entry's slot, the place in `ids` that holds its tree
-// position.  A heap operation moves words only -- two loads and a store per
-// level, [entry][thread] so that lanes never share a bank -- and a photon's
-// position is written once, into local memory.  The word is compared as the
-// float it is, within 2^-16 of the photon's key, which joins the error bounds:
-// two keys that close are compared in double.  What bounds the lookup is the
-// latency of its chains of moves and node reads at 14 warps per SM (ncu: issue
-// 34 %): the k = 100 lookups of 669,824 queries took 9.91 ms with 8-byte
-// entries in local memory (1 KB per query, which L1 cannot hold) and took 9.17
-// ms here; 7.64 ms with far children dropped at the push when their plane is
-// outside by then, 7.29 ms with the normals read in one load.
+// position.  A heap operation moves words only, one load and a store per level
+// ([row][thread], so that lanes never share a bank), and a photon's position is
+// written once, into local memory.  As a float the word is within 2^-16 of the
+// photon's key, which joins the error bounds; two words that close are compared
+// by their photons' distances in double, out of line.  What bounds the lookup is
+// the latency of its chains of moves and node reads at 12 to 14 warps per SM
+// (ncu: issue 36 %).  The k = 100 lookups of 669,824 queries took 9.91 ms with
+// 8-byte entries in local memory (1 KB per query, which L1 cannot hold), 9.17 ms
+// with words here, 7.64 ms with far children dropped at the push when their
+// plane is outside by then, 7.29 ms with the normals read in one load, 6.48 ms
+// with records, words compared as integers and lanes that wait for one another
+// (k_knn_gang), 6.12 ms with the heaps made together.
 struct SharedHeap {
   static constexpr uint32_t kSlot = 127u;
   static constexpr float kCut = 1.5262e-5f;  // 128 units in the last place: 2^-16, rounded up
-  uint32_t *h;                               // entry i of this thread: h[i * kKnnBlock]
+  char *h;  // this thread's 8 bytes of row 0
   int32_t *ids;
-  __device__ __forceinline__ uint32_t at(int i) const { return h[i * kKnnBlock]; }
-  __device__ __forceinline__ void put(int i, uint32_t v) { h[i * kKnnBlock] = v; }
+  // Entries 2r - 1 and 2r share the 8 bytes of row r, so that the children of
+  // entry i are one load, of row i + 1 (the root is the second word of row 0).
+  static constexpr int kRow = kKnnBlock * 8;
+  __host__ __device__ static __forceinline__ size_t bytes(int k) { return (size_t)(k / 2 + 1) * kRow; }
+  __device__ __forceinline__ uint32_t *slot(int i) const {
+    return reinterpret_cast<uint32_t *>(h + ((i + 1) >> 1) * kRow + ((i + 1) & 1) * 4);
+  }
+  __device__ __forceinline__ uint2 children(int i) const { return *reinterpret_cast<const uint2 *>(h + (i + 1) * kRow); }
+  __device__ __forceinline__ uint32_t at(int i) const { return *slot(i); }
   static __device__ __forceinline__ uint32_t entry(float key, uint32_t slot) {
     return (__float_as_uint(key) & ~kSlot) | slot;
   }
-  // as fcand_less
-  __device__ __forceinline__ bool less(const float4 *__restrict__ nodes, const Query &Q, uint32_t a, uint32_t b) const {
-    const float ka = __uint_as_float(a), kb = __uint_as_float(b), d = ka - kb;
-    const float tol = 1.0001f * fmaf(Q.ke1 + kCut, ka + kb, 2.0f * Q.ke0);
-    if (d < -tol) return true;
-    if (d > tol) return false;
-    const int32_t ia = ids[a & kSlot], ib = ids[b & kSlot];
-    const double da = point_d2(__ldg(nodes + ia), Q), db = point_d2(__ldg(nodes + ib), Q);
+  // (d2, position) lexicographic, as fcand_less.  Words that differ by more
+  // than kApart are in the order of their photons' exact distances if the
+  // smaller is not below `tiny`: floats a > b that are n words apart have
+  // a - b >= n 2^-24 b, and what must be exceeded is 2 (kKe1 + kCut) of their
+  // mean and 2 ke0, 4.18e-5 b for b >= tiny = 2e5 ke0 -- 702 words.  Infinite
+  // keys and NaN (all of a query's, then) lie within kApart of each other.
+  static constexpr uint32_t kApart = 720u;
+  uint32_t tiny;
+  static __device__ __noinline__ bool less_exact(Tree T, const double *q, int32_t ia, int32_t ib) {
+    const double da = point_d2(T.at(ia), q), db = point_d2(T.at(ib), q);
     return da == db ? ia < ib : da < db;
   }
-  __device__ __forceinline__ void push_up(const float4 *__restrict__ nodes, const Query &Q, int hole, int top,
-                                          uint32_t value) {
-    int parent = (hole - 1) / 2;
-    while (hole > top) {
-      const uint32_t p = at(parent);
-      if (!less(nodes, Q, p, value)) break;
-      put(hole, p);
-      hole = parent;
-      parent = (hole - 1) / 2;
-    }
-    put(hole, value);
+  __device__ __forceinline__ bool less(const Tree &T, const Query &Q, uint32_t a, uint32_t b) const {
+    if (a - b + kApart > 2u * kApart && min(a, b) >= tiny) return a < b;
+    return less_exact(T, Q.q, ids[a & kSlot], ids[b & kSlot]);
   }
-  __device__ __forceinline__ void adjust(const float4 *__restrict__ nodes, const Query &Q, int hole, int len,
+  // to: the slot of `hole`
+  __device__ __forceinline__ void push_up(const Tree &T, const Query &Q, int hole, uint32_t *to,
+                                          int top, uint32_t value) {
+    while (hole > top) {
+      const int parent = (hole - 1) >> 1;
+      uint32_t *from = slot(parent);
+      const uint32_t p = *from;
+      if (!less(T, Q, p, value)) break;
+      *to = p;
+      hole = parent;
+      to = from;
+    }
+    *to = value;
+  }
+  __device__ __forceinline__ void adjust(const Tree &T, const Query &Q, int hole, int len,
                                          uint32_t value) {
-    const int top = hole;
-    int second = hole;
-    while (second < (len - 1) / 2) {
-      second = 2 * (second + 1);
-      const uint32_t a = at(second - 1), b = at(second);
-      const bool left = less(nodes, Q, b, a);
-      second -= left ? 1 : 0;
-      put(hole, left ? a : b);
-      hole = second;
+    const int top = hole, two = (len - 1) / 2;
+    uint32_t *to = slot(hole);
+    while (hole < two) {
+      const uint2 c = children(hole);
+      const bool left = less(T, Q, c.y, c.x);
+      *to = left ? c.x : c.y;
+      to = reinterpret_cast<uint32_t *>(h + (hole + 1) * kRow + (left ? 0 : 4));
+      hole = 2 * hole + (left ? 1 : 2);
     }
-    if ((len & 1) == 0 && second == (len - 2) / 2) {
-      second = 2 * (second + 1);
-      put(hole, at(second - 1));
-      hole = second - 1;
+    if ((len & 1) == 0 && hole == (len - 2) / 2) {
+      *to = children(hole).x;
+      to = reinterpret_cast<uint32_t *>(h + (hole + 1) * kRow);
+      hole = 2 * hole + 1;
     }
-    push_up(nodes, Q, hole, top, value);
+    push_up(T, Q, hole, to, top, value);
   }
   __device__ __forceinline__ void add(int i, float key, int32_t photon) {
     ids[i] = photon;
-    put(i, entry(key, (uint32_t)i));
+    *slot(i) = entry(key, (uint32_t)i);
   }
-  __device__ __forceinline__ void make(const float4 *__restrict__ nodes, const Query &Q, int k) {
-    for (int parent = (k - 2) / 2; parent >= 0 && k >= 2; --parent) adjust(nodes, Q, parent, k, at(parent));
+  __device__ __forceinline__ void make(const Tree &T, const Query &Q, int k) {
+    for (int parent = (k - 2) / 2; parent >= 0 && k >= 2; --parent) adjust(T, Q, parent, k, at(parent));
   }
-  __device__ __forceinline__ void replace(const float4 *__restrict__ nodes, const Query &Q, int k, float key,
+  __device__ __forceinline__ void replace(const Tree &T, const Query &Q, int k, float key,
                                           int32_t photon) {
     const uint32_t back = at(k - 1), top = at(0);
-    put(k - 1, top);
-    adjust(nodes, Q, 0, k - 1, back);
+    adjust(T, Q, 0, k - 1, back);
     ids[top & kSlot] = photon;
-    push_up(nodes, Q, k - 1, 0, entry(key, top & kSlot));
+    push_up(T, Q, k - 1, slot(k - 1), 0, entry(key, top & kSlot));
   }
   __device__ __forceinline__ int32_t photon(int i) const { return ids[at(i) & kSlot]; }
   __device__ __forceinline__ void top(const Query &Q, Radius &r) const {
@@ -478,17 +534,45 @@ struct SharedHeap {
   }
 };
 
+// A query's output: its heap's photons and their exact squared distances, four
+// independent chains at a time.
+template <class Heap>
+__device__ __forceinline__ void write_found(const Tree &T, const Query &Q, const Heap &heap, int64_t i, int size, int k,
+                                            int32_t *__restrict__ out_idx, double *__restrict__ out_d2) {
+  int j = 0;
+  for (; j + 4 <= size; j += 4) {
+    const int32_t a0 = heap.photon(j), a1 = heap.photon(j + 1), a2 = heap.photon(j + 2), a3 = heap.photon(j + 3);
+    const double d0 = point_d2(T.at(a0), Q), d1 = point_d2(T.at(a1), Q),
+                 d2 = point_d2(T.at(a2), Q), d3 = point_d2(T.at(a3), Q);
+    out_idx[i * k + j] = a0;
+    out_idx[i * k + j + 1] = a1;
+    out_idx[i * k + j + 2] = a2;
+    out_idx[i * k + j + 3] = a3;
+    out_d2[i * k + j] = d0;
+    out_d2[i * k + j + 1] = d1;
+    out_d2[i * k + j + 2] = d2;
+    out_d2[i * k + j + 3] = d3;
+  }
+  for (; j < size; ++j) {
+    const int32_t a = heap.photon(j);
+    out_idx[i * k + j] = a;
+    out_d2[i * k + j] = point_d2(T.at(a), Q);
+  }
+  for (; j < k; ++j) {
+    out_idx[i * k + j] = -1;
+    out_d2[i * k + j] = 0.0;
+  }
+}
+
 // KMAX > 0: heaps of k <= KMAX entries in shared memory; KMAX == 0: global
 // heaps.
 template <int KMAX, int S>
-__global__ void __launch_bounds__(kKnnBlock, KMAX == 128 ? SKW_KNN_MINB / 2 : SKW_KNN_MINB) k_knn(const float4 *__restrict__ nodes, const uint16_t *__restrict__ nids,
-                                             const double *__restrict__ dirs, int n, const double *__restrict__ q,
-                                             const double *__restrict__ qn, int64_t nq, int k, double max_dist,
-                                             double cos_t, int32_t *__restrict__ out_idx,
-                                             double *__restrict__ out_d2, int32_t *__restrict__ out_count,
-                                             int32_t *__restrict__ out_visited, FCand *__restrict__ scratch,
-                                             unsigned *__restrict__ status, const int *__restrict__ nq_dev,
-                                             const int32_t *__restrict__ order, int per_warp) {
+__global__ void __launch_bounds__(kKnnBlock, knn_min_blocks(KMAX)) k_knn(
+    Tree T, const uint16_t *__restrict__ nids, const double *__restrict__ dirs, const double *__restrict__ q,
+    const double *__restrict__ qn, int64_t nq, int k, double max_dist, double cos_t, int32_t *__restrict__ out_idx,
+    double *__restrict__ out_d2, int32_t *__restrict__ out_count, int32_t *__restrict__ out_visited,
+    FCand *__restrict__ scratch, unsigned *__restrict__ status, const int *__restrict__ nq_dev,
+    const int32_t *__restrict__ order, int per_warp) {
   __shared__ uint32_t stk[S][kKnnBlock];
   const int lane = threadIdx.x & 31;
   if (lane >= per_warp) return;
@@ -496,39 +580,38 @@ __global__ void __launch_bounds__(kKnnBlock, KMAX == 128 ? SKW_KNN_MINB / 2 : SK
   if (nq_dev && *nq_dev < nq) nq = *nq_dev;
   if (i >= nq) return;
   if (order) i = order[i];
-  const float4 *nrm = node_normals(nids, n);
   Query Q;
   load_query(Q, q, qn, i, cos_t);
   int32_t ids[KMAX > 0 ? KMAX : 1];
-  extern __shared__ uint32_t s_heap[];
+  extern __shared__ __align__(16) char s_mem[];
   typename std::conditional<(KMAX > 0), SharedHeap, GlobalHeap>::type heap = [&]() {
-    if constexpr (KMAX > 0) return SharedHeap{s_heap + threadIdx.x, ids};
+    if constexpr (KMAX > 0) return SharedHeap{s_mem + threadIdx.x * 8, ids, __float_as_uint(2.0e5f * Q.ke0)};
     else return GlobalHeap{scratch + i * (int64_t)knn_heap_stride(k) + 1};
   }();
   int size = 0, visited = 0;
-  if (k > 0 && n > 0) {
+  if (k > 0 && T.n > 0) {
     Radius rad;  // max_dist until the heap is full, then its top
     rad.start(Q, max_dist);
     int sp = 0, cur = 0;
     bool overflow = false;
-    float4 p = __ldg(nodes);
+    float4 p = T.at(0);
     for (;;) {
       ++visited;
       int near, far;
       float s2;
-      node_children(p, cur, n, Q, near, far, s2);
+      node_children(p, cur, T.n, Q, near, far, s2);
       {
         const float d2f = dist2f(p, Q);
-        if ((d2f < rad.tin || (!(d2f >= rad.tout) && point_d2(p, Q) < rad.get(nodes, Q, KMAX > 0 ? ids : nullptr))) &&
-            (!Q.filter || photon_filter(Q, p, cur, nids, nrm, dirs))) {
+        if ((d2f < rad.tin || (!(d2f >= rad.tout) && point_d2(p, Q) < rad.get(T, Q, KMAX > 0 ? ids : nullptr))) &&
+            (!Q.filter || photon_filter(Q, NodeN{p, T.normal(cur)}, cur, nids, dirs))) {
           if (size < k) {
             heap.add(size++, d2f, cur);
             if (size == k) {
-              heap.make(nodes, Q, k);
+              heap.make(T, Q, k);
               heap.top(Q, rad);
             }
           } else {
-            heap.replace(nodes, Q, k, d2f, cur);
+            heap.replace(T, Q, k, d2f, cur);
             heap.top(Q, rad);
           }
         }
@@ -545,7 +628,7 @@ __global__ void __launch_bounds__(kKnnBlock, KMAX == 128 ? SKW_KNN_MINB / 2 : SK
       }
       if (near >= 0) {
         cur = near;
-        p = __ldg(nodes + near);
+        p = T.at(near);
         continue;
       }
       int next = -1;
@@ -555,67 +638,155 @@ __global__ void __launch_bounds__(kKnnBlock, KMAX == 128 ? SKW_KNN_MINB / 2 : SK
         const uint32_t par = stk[sp][threadIdx.x];
         int pnear, pfar;
         float ps2;
-        const float4 pp = __ldg(nodes + par);
-        node_children(pp, (int)par, n, Q, pnear, pfar, ps2);
-        if (ps2 < rad.tin || (!(ps2 >= rad.tout) && plane_d2(pp, Q) < rad.get(nodes, Q, KMAX > 0 ? ids : nullptr))) {
+        const float4 pp = T.at((int)par);
+        node_children(pp, (int)par, T.n, Q, pnear, pfar, ps2);
+        if (ps2 < rad.tin || (!(ps2 >= rad.tout) && plane_d2(pp, Q) < rad.get(T, Q, KMAX > 0 ? ids : nullptr))) {
           next = pfar;
           break;
         }
       }
       if (next < 0) break;
       cur = next;
-      p = __ldg(nodes + cur);
+      p = T.at(cur);
     }
     if (overflow) atomicOr(status, 2u);
   }
   out_count[i] = size;
-  // the exact squared distances of the output, four chains at a time
-  int j = 0;
-  for (; j + 4 <= size; j += 4) {
-    const int32_t a0 = heap.photon(j), a1 = heap.photon(j + 1), a2 = heap.photon(j + 2), a3 = heap.photon(j + 3);
-    const double d0 = point_d2(__ldg(nodes + a0), Q), d1 = point_d2(__ldg(nodes + a1), Q),
-                 d2 = point_d2(__ldg(nodes + a2), Q), d3 = point_d2(__ldg(nodes + a3), Q);
-    out_idx[i * k + j] = a0;
-    out_idx[i * k + j + 1] = a1;
-    out_idx[i * k + j + 2] = a2;
-    out_idx[i * k + j + 3] = a3;
-    out_d2[i * k + j] = d0;
-    out_d2[i * k + j + 1] = d1;
-    out_d2[i * k + j + 2] = d2;
-    out_d2[i * k + j + 3] = d3;
+  write_found(T, Q, heap, i, size, k, out_idx, out_d2);
+  if (out_visited) out_visited[i] = visited;
+}
+
+// A heap operation is a chain of some 15 levels (the make_heap of a full heap,
+// of 100), which a warp walks for whichever of its lanes are at one.  So in
+// full warps a lane that has a point for its heap waits with it until a third
+// of the lanes with full heaps do (kReplaceShare / 3), and one whose heap is
+// full for the first time until seven eighths of those still filling are
+// (kMakeShare / 8); what the lookups visit and find is the same, as a lane
+// takes no step with a radius that is not up to date.  k = 100, 669,824
+// queries: at once 6.98 ms, a third 6.53, half 6.48, two thirds 7.23; with the
+// heaps made at three quarters 6.28, seven eighths 6.19, all 6.08 (but queries
+// that never fill theirs would then hold up the others).  A waiting walk's
+// stack keeps a far child with its plane's distance, which spares the parent's
+// load at a pop.  Heaps of 32 entries are too short for it (gather lookups 2.82
+// -> 3.50 ms), at 33 to 40 it depends on the number of queries (669,824: 2.19
+// -> 2.37 ms, 100,000: 0.54 -> 0.50), from 50 on both gain (3.21 -> 2.92 ms,
+// 0.84 -> 0.59); and in warps with few queries (irradiance estimates 3.51 ->
+// 4.25 ms) no lane waits either.
+constexpr int kReplaceShare = 1, kMakeShare = 7, kGangEntries = 48;
+
+template <int KMAX>
+__global__ void __launch_bounds__(kKnnBlock, KMAX == 128 ? 16 : 24) k_knn_gang(
+    Tree T, const uint16_t *__restrict__ nids, const double *__restrict__ dirs, const double *__restrict__ q,
+    const double *__restrict__ qn, int64_t nq, int k, double max_dist, double cos_t, int32_t *__restrict__ out_idx,
+    double *__restrict__ out_d2, int32_t *__restrict__ out_count, int32_t *__restrict__ out_visited,
+    FCand *__restrict__ scratch, unsigned *__restrict__ status, const int *__restrict__ nq_dev,
+    const int32_t *__restrict__ order, int depth) {
+  static_assert(kKnnBlock == 32, "one warp per block");
+  // the heaps' rows, then the walk stacks: `depth` entries each
+  extern __shared__ __align__(16) char s_mem[];
+  uint2 *stk = reinterpret_cast<uint2 *>(s_mem + (KMAX > 0 ? SharedHeap::bytes(k) : 0)) + threadIdx.x;
+  const int lane = threadIdx.x & 31;
+  int64_t i = ((int64_t)blockIdx.x * (kKnnBlock / 32) + (threadIdx.x >> 5)) * 32 + lane;
+  if (nq_dev && *nq_dev < nq) nq = *nq_dev;
+  const bool mine = i < nq;
+  if (mine && order) i = order[i];
+  Query Q{};
+  if (mine) load_query(Q, q, qn, i, cos_t);
+  int32_t ids[KMAX > 0 ? KMAX : 1];
+  typename std::conditional<(KMAX > 0), SharedHeap, GlobalHeap>::type heap = [&]() {
+    if constexpr (KMAX > 0) return SharedHeap{s_mem + threadIdx.x * 8, ids, __float_as_uint(2.0e5f * Q.ke0)};
+    else return GlobalHeap{scratch + i * (int64_t)knn_heap_stride(k) + 1};
+  }();
+  int size = 0, visited = 0;
+  Radius rad;  // max_dist until the heap is full, then its top
+  if (mine) rad.start(Q, max_dist);
+  // A point for the heap waits in (key, photon), and its lane with it, until
+  // enough lanes have one.
+  bool walks = mine && k > 0 && T.n > 0, waits = false, made = false;
+  float key = 0.0f;
+  int photon = 0, sp = 0, cur = 0;  // cur < 0: the next node comes from the stack
+  NodeN p{};
+  if (walks) p = T.load(0, Q.filter);
+  for (;;) {
+    if (walks && !waits) {
+      while (cur < 0 && sp > 0) {
+        --sp;
+        // the reference's pop test: (qa - split)^2 < radius, in double
+        const uint2 top = stk[sp * kKnnBlock];
+        const float s2 = __uint_as_float(top.y);
+        if (s2 < rad.tin || (!(s2 >= rad.tout) && plane_d2(T.at(node_parent(T, (int)top.x)), Q) <
+                                                      rad.get(T, Q, KMAX > 0 ? ids : nullptr))) {
+          cur = (int)top.x;
+          p = T.load(cur, Q.filter);
+        }
+      }
+      walks = cur >= 0;
+      if (walks) {
+        ++visited;
+        int near, far;
+        float s2;
+        node_children(p.p, cur, T.n, Q, near, far, s2);
+        const float d2f = dist2f(p.p, Q);
+        if ((d2f < rad.tin || (!(d2f >= rad.tout) && point_d2(p.p, Q) < rad.get(T, Q, KMAX > 0 ? ids : nullptr))) &&
+            (!Q.filter || photon_filter(Q, p, cur, nids, dirs))) {
+          key = d2f;
+          photon = cur;
+          waits = size >= k - 1;
+          if (size < k) heap.add(size++, d2f, cur);
+        }
+        // The far child waits on the stack, unless its plane is certainly outside
+        // already (the radius only shrinks, so it would be when popped).
+        if (far >= 0 && !(s2 >= rad.tout)) {
+          if (sp >= depth) {
+            atomicOr(status, 2u);
+            walks = waits = false;
+          } else {
+            stk[sp * kKnnBlock] = make_uint2((uint32_t)far, __float_as_uint(s2));
+            ++sp;
+          }
+        }
+        cur = near;
+        if (near >= 0) p = T.load(near, Q.filter);
+      }
+    }
+    if (!__any_sync(0xffffffffu, walks)) break;
+    const int filling = __popc(__ballot_sync(0xffffffffu, walks && !made)),
+              full = __popc(__ballot_sync(0xffffffffu, walks && made)),
+              to_make = __popc(__ballot_sync(0xffffffffu, waits && !made)),
+              to_replace = __popc(__ballot_sync(0xffffffffu, waits && made));
+    if (waits && (made ? 3 * to_replace >= kReplaceShare * full : 8 * to_make >= kMakeShare * filling)) {
+      if (made) heap.replace(T, Q, k, key, photon);
+      else heap.make(T, Q, k);
+      heap.top(Q, rad);
+      made = true;
+      waits = false;
+    }
   }
-  for (; j < size; ++j) {
-    const int32_t a = heap.photon(j);
-    out_idx[i * k + j] = a;
-    out_d2[i * k + j] = point_d2(__ldg(nodes + a), Q);
-  }
-  for (; j < k; ++j) {
-    out_idx[i * k + j] = -1;
-    out_d2[i * k + j] = 0.0;
-  }
+  if (!mine) return;
+  out_count[i] = size;
+  write_found(T, Q, heap, i, size, k, out_idx, out_d2);
   if (out_visited) out_visited[i] = visited;
 }
 
 // GetNearestPoint (KDTree.h:495-503) with NearestPointProc (:293-323):
 // every accepted point becomes the nearest and shrinks the radius.
 template <int S>
-__device__ __forceinline__ int nearest_walk(const float4 *__restrict__ nodes, const uint16_t *__restrict__ nids,
-                                            const float4 *__restrict__ nrm, const double *__restrict__ dirs, int n,
-                                            const Query &Q, double max_dist, uint32_t (*stk)[kKnnBlock],
+__device__ __forceinline__ int nearest_walk(Tree T, const uint16_t *__restrict__ nids,
+                                            const double *__restrict__ dirs, const Query &Q, double max_dist, uint2 (*stk)[kKnnBlock],
                                             unsigned *__restrict__ status) {
   int best = -1;
-  if (n <= 0) return best;
+  if (T.n <= 0) return best;
   Radius rad;
   rad.start(Q, max_dist);
   int sp = 0, cur = 0;
-  float4 p = __ldg(nodes);
+  NodeN p = T.load(0, Q.filter);
   for (;;) {
     int near, far;
     float s2;
-    node_children(p, cur, n, Q, near, far, s2);
-    const float d2f = dist2f(p, Q);
-    if ((d2f < rad.tin || (!(d2f >= rad.tout) && point_d2(p, Q) < rad.get(nodes, Q))) &&
-        (!Q.filter || photon_filter(Q, p, cur, nids, nrm, dirs))) {
+    node_children(p.p, cur, T.n, Q, near, far, s2);
+    const float d2f = dist2f(p.p, Q);
+    if ((d2f < rad.tin || (!(d2f >= rad.tout) && point_d2(p.p, Q) < rad.get(T, Q))) &&
+        (!Q.filter || photon_filter(Q, p, cur, nids, dirs))) {
       best = cur;
       rad.set(Q, cur, d2f, 0.0f);
     }
@@ -626,44 +797,42 @@ __device__ __forceinline__ int nearest_walk(const float4 *__restrict__ nodes, co
         atomicOr(status, 2u);
         return best;
       }
-      stk[sp][threadIdx.x] = (uint32_t)cur;
+      stk[sp][threadIdx.x] = make_uint2((uint32_t)far, __float_as_uint(s2));
       ++sp;
     }
     if (near >= 0) {
       cur = near;
-      p = __ldg(nodes + near);
+      p = T.load(near, Q.filter);
       continue;
     }
     int next = -1;
     while (sp > 0) {
       --sp;
       // the reference's pop test: (qa - split)^2 < radius, in double
-      const uint32_t par = stk[sp][threadIdx.x];
-      int pnear, pfar;
-      float ps2;
-      const float4 pp = __ldg(nodes + par);
-      node_children(pp, (int)par, n, Q, pnear, pfar, ps2);
-      if (ps2 < rad.tin || (!(ps2 >= rad.tout) && plane_d2(pp, Q) < rad.get(nodes, Q))) {
-        next = pfar;
+      const uint2 top = stk[sp][threadIdx.x];
+      const float s2 = __uint_as_float(top.y);
+      if (s2 < rad.tin || (!(s2 >= rad.tout) &&
+                           plane_d2(T.at(node_parent(T, (int)top.x)), Q) < rad.get(T, Q))) {
+        next = (int)top.x;
         break;
       }
     }
     if (next < 0) break;
     cur = next;
-    p = __ldg(nodes + cur);
+    p = T.load(cur, Q.filter);
   }
   return best;
 }
 
 template <int S>
-__global__ void __launch_bounds__(kKnnBlock, SKW_KNN_MINB) k_nearest(const float4 *__restrict__ nodes, const uint16_t *__restrict__ nids,
-                                                 const double *__restrict__ dirs, int n,
+__global__ void __launch_bounds__(kKnnBlock, SKW_KNN_MINB) k_nearest(Tree T, const uint16_t *__restrict__ nids,
+                                                 const double *__restrict__ dirs,
                                                  const double *__restrict__ q, const double *__restrict__ qn,
                                                  int64_t nq, double max_dist, double cos_t,
                                                  int32_t *__restrict__ out_idx, unsigned *__restrict__ status,
                                                  const int *__restrict__ nq_dev, const int32_t *__restrict__ order,
                                                  int per_warp) {
-  __shared__ uint32_t stk[S][kKnnBlock];
+  __shared__ uint2 stk[S][kKnnBlock];
   const int lane = threadIdx.x & 31;
   if (lane >= per_warp) return;
   int64_t i = ((int64_t)blockIdx.x * (kKnnBlock / 32) + (threadIdx.x >> 5)) * per_warp + lane;
@@ -672,7 +841,7 @@ __global__ void __launch_bounds__(kKnnBlock, SKW_KNN_MINB) k_nearest(const float
   if (order) i = order[i];
   Query Q;
   load_query(Q, q, qn, i, cos_t);
-  out_idx[i] = nearest_walk<S>(nodes, nids, node_normals(nids, n), dirs, n, Q, max_dist, stk, status);
+  out_idx[i] = nearest_walk<S>(T, nids, dirs, Q, max_dist, stk, status);
 }
 
 // The same by looking at every point, one warp per query: for launches of few
@@ -682,37 +851,36 @@ __global__ void __launch_bounds__(kKnnBlock, SKW_KNN_MINB) k_nearest(const float
 // stays), and so is the answer wherever one is met.
 template <int S>
 __global__ void __launch_bounds__(kKnnBlock, SKW_KNN_MINB) k_nearest_scan(
-    const float4 *__restrict__ nodes, const uint16_t *__restrict__ nids, const double *__restrict__ dirs, int n,
+    Tree T, const uint16_t *__restrict__ nids, const double *__restrict__ dirs,
     const double *__restrict__ q, const double *__restrict__ qn, int64_t nq, double max_dist, double cos_t,
     int32_t *__restrict__ out_idx, unsigned *__restrict__ status) {
   static_assert(kKnnBlock == 32, "one query per block");
-  __shared__ uint32_t stk[S][kKnnBlock];
+  __shared__ uint2 stk[S][kKnnBlock];
   const int64_t i = blockIdx.x;
   const int lane = threadIdx.x;
-  const float4 *nrm = node_normals(nids, n);
   Query Q;
   load_query(Q, q, qn, i, cos_t);
   Radius rad;
   rad.start(Q, max_dist);
   int best = -1;
   bool tie = false;
-  for (int t0 = lane; t0 < n; t0 += 128) {
+  for (int t0 = lane; t0 < T.n; t0 += 128) {
     float4 ps[4];
 #pragma unroll
-    for (int u = 0; u < 4; ++u) ps[u] = __ldg(nodes + min(t0 + 32 * u, n - 1));
+    for (int u = 0; u < 4; ++u) ps[u] = T.at(min(t0 + 32 * u, T.n - 1));
 #pragma unroll
     for (int u = 0; u < 4; ++u) {
       const int t = t0 + 32 * u;
       const float4 p = ps[u];
       const float d2f = dist2f(p, Q);
-      if (t >= n || d2f >= rad.tout) continue;
+      if (t >= T.n || d2f >= rad.tout) continue;
       bool equal = false;
       if (!(d2f < rad.tin)) {
-        const double d = point_d2(p, Q), r = rad.get(nodes, Q);
+        const double d = point_d2(p, Q), r = rad.get(T, Q);
         if (!(d <= r)) continue;
         equal = d == r;
       }
-      if (Q.filter && !photon_filter(Q, p, t, nids, nrm, dirs)) continue;
+      if (Q.filter && !photon_filter(Q, NodeN{p, T.normal(t)}, t, nids, dirs)) continue;
       if (equal) {
         tie = true;
       } else {
@@ -722,13 +890,13 @@ __global__ void __launch_bounds__(kKnnBlock, SKW_KNN_MINB) k_nearest_scan(
       }
     }
   }
-  const double mine = best >= 0 ? point_d2(__ldg(nodes + best), Q) : INFINITY;
+  const double mine = best >= 0 ? point_d2(T.at(best), Q) : INFINITY;
   double least = mine;
   for (int o = 16; o > 0; o >>= 1) least = fmin(least, __shfl_xor_sync(0xffffffffu, least, o));
   const unsigned who = __ballot_sync(0xffffffffu, best >= 0 && mine == least);
   const bool ties = __ballot_sync(0xffffffffu, tie) != 0u || __popc(who) > 1;
   if (ties) {
-    if (lane == 0) out_idx[i] = nearest_walk<S>(nodes, nids, nrm, dirs, n, Q, max_dist, stk, status);
+    if (lane == 0) out_idx[i] = nearest_walk<S>(T, nids, dirs, Q, max_dist, stk, status);
   } else if (who == 0u) {
     if (lane == 0) out_idx[i] = -1;
   } else if (lane == __ffs(who) - 1) {
@@ -768,23 +936,45 @@ inline bool nearest_by_scan(int64_t nq, int64_t n, bool filter) {
          (filter || nq * n <= kScanPairs);
 }
 
+// Levels of the median-split tree of n points: as many entries as a walk's
+// stack can hold.
+inline int tree_levels(int n) {
+  int levels = 1;
+  for (int64_t m = n; m > 1; m >>= 1) ++levels;
+  return levels;
+}
+
+// Full warps with heaps of more than 32 entries: k_knn_gang.  The others:
 // k_knn<KMAX, S> with S chosen by the tree's depth.
 template <int KMAX>
-void knn_kernel(cudaStream_t stream, const float4 *nodes, const uint16_t *nids, const double *dirs,
-                int n, const double *q, const double *qn, int64_t nq, int k, double max_dist, double cos_t,
-                int32_t *out_idx, double *out_d2, int32_t *out_count, int32_t *out_visited, FCand *scratch,
-                unsigned *status, const int *nq_dev, const int32_t *order) {
+void knn_kernel(cudaStream_t stream, const Tree &T, const uint16_t *nids, const double *dirs, const double *q,
+                const double *qn, int64_t nq, int k, double max_dist, double cos_t, int32_t *out_idx, double *out_d2,
+                int32_t *out_count, int32_t *out_visited, FCand *scratch, unsigned *status, const int *nq_dev,
+                const int32_t *order) {
   const int per_warp = queries_per_warp(nq);
   const unsigned grid = knn_grid(nq, per_warp);
-  const size_t smem = KMAX > 0 ? (size_t)k * kKnnBlock * sizeof(uint32_t) : 0;
-  if (shallow_tree(n))
-    k_knn<KMAX, kShallowStack><<<grid, kKnnBlock, smem, stream>>>(nodes, nids, dirs, n, q, qn, nq, k, max_dist, cos_t,
-                                                               out_idx, out_d2, out_count, out_visited, scratch,
-                                                               status, nq_dev, order, per_warp);
+  const size_t smem = KMAX > 0 ? SharedHeap::bytes(k) : 0;
+  if constexpr (KMAX != 32) {
+    if (per_warp == 32 && k > kGangEntries) {
+      const int depth = tree_levels(T.n);
+      k_knn_gang<KMAX><<<grid, kKnnBlock, smem + (size_t)depth * kKnnBlock * sizeof(uint2), stream>>>(
+          T, nids, dirs, q, qn, nq, k, max_dist, cos_t, out_idx, out_d2, out_count, out_visited, scratch, status, nq_dev,
+          order, depth);
+      return;
+    }
+  }
+  if (shallow_tree(T.n))
+    k_knn<KMAX, kShallowStack><<<grid, kKnnBlock, smem, stream>>>(T, nids, dirs, q, qn, nq, k, max_dist, cos_t, out_idx,
+                                                               out_d2, out_count, out_visited, scratch, status, nq_dev,
+                                                               order, per_warp);
   else
-    k_knn<KMAX, 32><<<grid, kKnnBlock, smem, stream>>>(nodes, nids, dirs, n, q, qn, nq, k, max_dist, cos_t, out_idx,
-                                                    out_d2, out_count, out_visited, scratch, status, nq_dev, order,
-                                                    per_warp);
+    k_knn<KMAX, 32><<<grid, kKnnBlock, smem, stream>>>(T, nids, dirs, q, qn, nq, k, max_dist, cos_t, out_idx, out_d2,
+                                                    out_count, out_visited, scratch, status, nq_dev, order, per_warp);
+}
+
+inline Tree tree_of(const void *nodes, const uint16_t *nids, int n) {
+  return Tree{(const float4 *)nodes,
+              reinterpret_cast<const float4 *>(reinterpret_cast<const char *>(nids) + nids_offset(n)), n};
 }
 
 // Spatial bins of queries: a box cut into 64^3 cells, each query's cell as
@@ -916,20 +1106,21 @@ __global__ void __launch_bounds__(kSortBlock) k_sort_scatter(const uint32_t *__r
   val2[dst] = val ? val[i] : (int32_t)i;
 }
 
-__global__ void k_normals(const uint16_t *__restrict__ nids, int64_t n, const float *__restrict__ dirs_f,
-                          float4 *__restrict__ out) {
+__global__ void k_node_records(const float4 *__restrict__ nodes, const uint16_t *__restrict__ nids, int64_t n,
+                               const float *__restrict__ dirs_f, float4 *__restrict__ out) {
   const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= n) return;
   const float *d = dirs_f + 3 * (int)nids[i];
-  out[i] = make_float4(d[0], d[1], d[2], 0.0f);
+  out[2 * i] = nodes[i];
+  out[2 * i + 1] = make_float4(d[0], d[1], d[2], 0.0f);
 }
 
 }  // namespace
 
-cudaError_t launch_normals(uint16_t *nids, int64_t n, const double *dirs, cudaStream_t st) {
+cudaError_t launch_node_records(const void *nodes, uint16_t *nids, int64_t n, const double *dirs, cudaStream_t st) {
   if (n <= 0) return cudaSuccess;
-  k_normals<<<(unsigned)((n + 255) / 256), 256, 0, st>>>(
-      nids, n, reinterpret_cast<const float *>(dirs + (3 << 16)),
+  k_node_records<<<(unsigned)((n + 255) / 256), 256, 0, st>>>(
+      (const float4 *)nodes, nids, n, reinterpret_cast<const float *>(dirs + (3 << 16)),
       reinterpret_cast<float4 *>(reinterpret_cast<char *>(nids) + nids_offset(n)));
   return cudaGetLastError();
 }
@@ -1006,19 +1197,19 @@ cudaError_t launch_knn(const void *nodes, const uint16_t *nids, const double *di
                        double *out_d2, int32_t *out_count, int32_t *out_visited, void *scratch, unsigned *status,
                        cudaStream_t stream, const int *nq_dev, const int32_t *order) {
   if (nq <= 0) return cudaSuccess;
-  const float4 *nd = (const float4 *)nodes;
+  const Tree T = tree_of(nodes, nids, n);
   if (scratch && k >= SKW_KNN_GHEAP) {
-    knn_kernel<0>(stream, nd, nids, dirs, n, q, qn, nq, k, max_dist, cos_t, out_idx, out_d2, out_count,
+    knn_kernel<0>(stream, T, nids, dirs, q, qn, nq, k, max_dist, cos_t, out_idx, out_d2, out_count,
                   out_visited, (FCand *)scratch, status, nq_dev, order);
   } else if (k <= 32) {
-    knn_kernel<32>(stream, nd, nids, dirs, n, q, qn, nq, k, max_dist, cos_t, out_idx, out_d2, out_count,
+    knn_kernel<32>(stream, T, nids, dirs, q, qn, nq, k, max_dist, cos_t, out_idx, out_d2, out_count,
                    out_visited, nullptr, status, nq_dev, order);
   } else if (k <= 128) {
-    knn_kernel<128>(stream, nd, nids, dirs, n, q, qn, nq, k, max_dist, cos_t, out_idx, out_d2, out_count,
+    knn_kernel<128>(stream, T, nids, dirs, q, qn, nq, k, max_dist, cos_t, out_idx, out_d2, out_count,
                     out_visited, nullptr, status, nq_dev, order);
   } else {
     if (!scratch) return cudaErrorInvalidValue;
-    knn_kernel<0>(stream, nd, nids, dirs, n, q, qn, nq, k, max_dist, cos_t, out_idx, out_d2, out_count,
+    knn_kernel<0>(stream, T, nids, dirs, q, qn, nq, k, max_dist, cos_t, out_idx, out_d2, out_count,
                   out_visited, (FCand *)scratch, status, nq_dev, order);
   }
   return cudaGetLastError();
@@ -1083,7 +1274,7 @@ cudaError_t launch_knn_noalloc(const void *nodes, const uint16_t *nids, const do
   if (e != cudaSuccess) return e;
   // Every heap slot is written before it is read, so the array needs no
   // clearing between calls.
-  knn_kernel<0>(stream, (const float4 *)nodes, nids, dirs, n, q, qn, nq, k, max_dist, cos_t, out_idx, out_d2,
+  knn_kernel<0>(stream, tree_of(nodes, nids, n), nids, dirs, q, qn, nq, k, max_dist, cos_t, out_idx, out_d2,
                 out_count, nullptr, (FCand *)scratch, status, nullptr, nullptr);
   return cudaGetLastError();
 }
@@ -1092,18 +1283,19 @@ cudaError_t launch_nearest(const void *nodes, const uint16_t *nids, const double
                            const double *qn, int64_t nq, double max_dist, double cos_t, int32_t *out_idx,
                            unsigned *status, cudaStream_t stream, const int *nq_dev, const int32_t *order) {
   if (nq <= 0) return cudaSuccess;
+  const Tree T = tree_of(nodes, nids, n);
   if (!nq_dev && !order && nearest_by_scan(nq, n, cos_t >= 0.0)) {
     k_nearest_scan<kShallowStack><<<(unsigned)nq, kKnnBlock, 0, stream>>>(
-        (const float4 *)nodes, nids, dirs, n, q, qn, nq, max_dist, cos_t, out_idx, status);
+        T, nids, dirs, q, qn, nq, max_dist, cos_t, out_idx, status);
     return cudaGetLastError();
   }
   const int per_warp = queries_per_warp(nq);
   const unsigned grid = knn_grid(nq, per_warp);
   if (shallow_tree(n))
-    k_nearest<kShallowStack><<<grid, kKnnBlock, 0, stream>>>((const float4 *)nodes, nids, dirs, n, q, qn, nq, max_dist,
+    k_nearest<kShallowStack><<<grid, kKnnBlock, 0, stream>>>(T, nids, dirs, q, qn, nq, max_dist,
                                                          cos_t, out_idx, status, nq_dev, order, per_warp);
   else
-    k_nearest<32><<<grid, kKnnBlock, 0, stream>>>((const float4 *)nodes, nids, dirs, n, q, qn, nq, max_dist, cos_t,
+    k_nearest<32><<<grid, kKnnBlock, 0, stream>>>(T, nids, dirs, q, qn, nq, max_dist, cos_t,
                                               out_idx, status, nq_dev, order, per_warp);
   return cudaGetLastError();
 }

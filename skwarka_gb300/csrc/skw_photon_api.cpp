@@ -176,7 +176,7 @@ int skw_kdtree_create(skw_ctx *ctx, const float *positions, const uint16_t *norm
   if (e == cudaSuccess) e = cudaMemcpy(t->d_nids, nids.data(), nids.size() * sizeof(uint16_t), cudaMemcpyHostToDevice);
   if (e == cudaSuccess) e = cudaMemcpy(t->d_dirs, dirs.data(), dirs.size() * sizeof(double), cudaMemcpyHostToDevice);
   if (e == cudaSuccess) e = cudaMemset(t->d_status, 0, sizeof(unsigned));
-  if (e == cudaSuccess) e = skw::launch_normals(t->d_nids, n, t->d_dirs, nullptr);
+  if (e == cudaSuccess) e = skw::launch_node_records(t->d_nodes, t->d_nids, n, t->d_dirs, nullptr);
   if (e == cudaSuccess) e = cudaStreamSynchronize(nullptr);  // lookups may come on any stream
   if (e != cudaSuccess) {
     skw_kdtree_destroy(t);

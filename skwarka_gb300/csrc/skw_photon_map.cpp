@@ -43,12 +43,13 @@ cudaError_t upload(const std::vector<T> &v, T **out) {
   return e;
 }
 
-// Normal ids with their normals behind them (nids_bytes).
-cudaError_t upload_nids(const std::vector<uint16_t> &v, const double *dirs, cudaStream_t st, uint16_t **out) {
+// Normal ids with the tree's node records behind them (nids_bytes).
+cudaError_t upload_nids(const void *nodes, const std::vector<uint16_t> &v, const double *dirs, cudaStream_t st,
+                        uint16_t **out) {
   const int64_t n = (int64_t)v.size();
   cudaError_t e = cudaMalloc((void **)out, skw::nids_bytes(n));
   if (e == cudaSuccess && n > 0) e = cudaMemcpy(*out, v.data(), (size_t)n * 2, cudaMemcpyHostToDevice);
-  if (e == cudaSuccess) e = skw::launch_normals(*out, n, dirs, st);
+  if (e == cudaSuccess) e = skw::launch_node_records(nodes, *out, n, dirs, st);
   return e == cudaSuccess ? cudaStreamSynchronize(st) : e;  // lookups on other streams follow
 }
 
@@ -95,7 +96,7 @@ cudaError_t build_map(Map &m, const double *dirs, cudaStream_t st) {
         (e = cudaMalloc(&m.d_dirid, n * 2)) == cudaSuccess && (e = cudaMalloc(&m.d_weight, n * 12)) == cudaSuccess &&
         (e = skw::gather_tree_order(d_perm, m.n, nin, din, win, m.d_nids, m.d_dirid, m.d_weight, st)) ==
             cudaSuccess &&
-        (e = skw::launch_normals(m.d_nids, m.n, dirs, st)) == cudaSuccess)
+        (e = skw::launch_node_records(m.d_nodes, m.d_nids, m.n, dirs, st)) == cudaSuccess)
       e = cudaStreamSynchronize(st);
     cudaFree(nin);
     cudaFree(din);
@@ -113,7 +114,7 @@ cudaError_t build_map(Map &m, const double *dirs, cudaStream_t st) {
     dt[t] = dirid[i];
     for (int k = 0; k < 3; ++k) wt[3 * t + k] = w[3 * i + k];
   }
-  if (e == cudaSuccess) e = upload_nids(nt, dirs, st, &m.d_nids);
+  if (e == cudaSuccess) e = upload_nids(m.d_nodes, nt, dirs, st, &m.d_nids);
   if (e == cudaSuccess) e = upload(dt, &m.d_dirid);
   if (e == cudaSuccess) e = upload(wt, &m.d_weight);
   return e;
@@ -287,7 +288,7 @@ int build_maps(skw_photon_map *pm, cudaStream_t st) {
       skw::KdNode *dn = nullptr;
       e = upload(nodes, &dn);
       pm->d_irr_nodes = dn;
-      if (e == cudaSuccess) e = upload_nids(nrm_t, pm->d_dirs, st, &pm->d_irr_nids);
+      if (e == cudaSuccess) e = upload_nids(pm->d_irr_nodes, nrm_t, pm->d_dirs, st, &pm->d_irr_nids);
       if (e == cudaSuccess)
         e = skw::launch_nearest(pm->d_irr_nodes, pm->d_irr_nids, pm->d_dirs, (int)nq, B.sq, B.sqn, ns,
                                 std::numeric_limits<double>::infinity(), kMaxNormalDeviationCos, B.near,

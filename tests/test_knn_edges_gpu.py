@@ -97,3 +97,27 @@ def test_radius_at_a_point(trees):
             got = tree.get_nearest_point(_dev(q), _dev(qn), radius, -1.0).cpu().numpy()
             assert np.array_equal(got, want.nearest(q, qn, radius, -1.0))
             _check_knn(trees, n, True, 300, 40, radius, -1.0)
+
+
+@pytest.mark.parametrize("k,radius", [(48, 0.25), (49, 0.25), (64, 0.2), (128, 0.45), (129, 0.35)])
+@pytest.mark.parametrize("lattice", [False, True])
+def test_full_warps(trees, k, radius, lattice):
+    """From 63,489 queries on the warps are full and lanes wait for one another at their heaps (k > 48): with heaps
+    that some queries of a warp fill and others do not, with the filter and without, and a last warp in part."""
+    _check_knn(trees, 6000, lattice, 63_489 + k, k, radius, 0.3 if k % 2 else -1.0)
+
+
+def test_far_from_the_origin(trees, oracle):
+    """Coordinates whose float spacing is large against the distances: what float cannot tell apart is decided in
+    double."""
+    pos, nid = _points(4000, 3, False)
+    for shift in (1e3, 3e7):
+        p = (pos.astype(np.float64) + shift).astype(np.float32)
+        tree, want = PhotonKDTree(p, nid), oracle.kdtree(p, nid)
+        q, qn = _queries(500, 4, False)
+        q = q + shift
+        for k, cos in ((10, 0.3), (60, -1.0)):
+            got = tree.get_nearest_points(_dev(q), _dev(qn), k, 2.0 if shift < 1e6 else 40.0, cos)
+            ref = want.knn(q, qn, k, 2.0 if shift < 1e6 else 40.0, cos)
+            for key in ("count", "idx", "d2"):
+                assert np.array_equal(got[key].cpu().numpy(), ref[key]), (shift, k, key)
