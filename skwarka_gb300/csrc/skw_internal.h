@@ -61,6 +61,13 @@ namespace skw {
 int fail(skw_ctx *ctx, int code, const std::string &msg);
 // Maps a CUDA error to SKW_ERR_OOM / SKW_ERR_CUDA with a message.
 int cuda_fail(skw_ctx *ctx, cudaError_t e, const char *what);
+// Copies host memory in and waits: a plain cudaMemcpy from pageable memory
+// returns when the source may be reused, and a kernel on a non-blocking stream
+// could still run before the bytes have arrived.
+inline cudaError_t copy_in(void *dst, const void *src, size_t bytes) {
+  const cudaError_t e = cudaMemcpy(dst, src, bytes, cudaMemcpyHostToDevice);
+  return e == cudaSuccess ? cudaStreamSynchronize(nullptr) : e;
+}
 // Creates the context's workspace pool on first use.
 cudaError_t ctx_pool(skw_ctx *ctx, cudaMemPool_t *pool);
 

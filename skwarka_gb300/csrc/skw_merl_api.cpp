@@ -37,8 +37,8 @@ int skw_merl_create(skw_ctx *ctx, const void *bytes, int64_t n_bytes, skw_merl *
   void *t = nullptr, *sg = nullptr;
   if (e == cudaSuccess) e = cudaMalloc(&t, m->host.table.size() * 2);
   if (e == cudaSuccess) e = cudaMalloc(&sg, m->host.seg.size() * 4);
-  if (e == cudaSuccess) e = cudaMemcpy(t, m->host.table.data(), m->host.table.size() * 2, cudaMemcpyHostToDevice);
-  if (e == cudaSuccess) e = cudaMemcpy(sg, m->host.seg.data(), m->host.seg.size() * 4, cudaMemcpyHostToDevice);
+  if (e == cudaSuccess) e = skw::copy_in(t, m->host.table.data(), m->host.table.size() * 2);
+  if (e == cudaSuccess) e = skw::copy_in(sg, m->host.seg.data(), m->host.seg.size() * 4);
   if (e != cudaSuccess) {
     cudaFree(t);
     cudaFree(sg);

@@ -39,7 +39,7 @@ cudaError_t upload(const std::vector<T> &v, T **out) {
   *out = nullptr;
   const size_t b = std::max<size_t>(v.size(), 1) * sizeof(T);
   cudaError_t e = cudaMalloc((void **)out, b);
-  if (e == cudaSuccess && !v.empty()) e = cudaMemcpy(*out, v.data(), v.size() * sizeof(T), cudaMemcpyHostToDevice);
+  if (e == cudaSuccess && !v.empty()) e = skw::copy_in(*out, v.data(), v.size() * sizeof(T));
   return e;
 }
 
@@ -48,7 +48,7 @@ cudaError_t upload_nids(const void *nodes, const std::vector<uint16_t> &v, const
                         uint16_t **out) {
   const int64_t n = (int64_t)v.size();
   cudaError_t e = cudaMalloc((void **)out, skw::nids_bytes(n));
-  if (e == cudaSuccess && n > 0) e = cudaMemcpy(*out, v.data(), (size_t)n * 2, cudaMemcpyHostToDevice);
+  if (e == cudaSuccess && n > 0) e = skw::copy_in(*out, v.data(), (size_t)n * 2);
   if (e == cudaSuccess) e = skw::launch_node_records(nodes, *out, n, dirs, st);
   return e == cudaSuccess ? cudaStreamSynchronize(st) : e;  // lookups on other streams follow
 }
@@ -253,10 +253,10 @@ int build_maps(skw_photon_map *pm, cudaStream_t st) {
     if ((e = cudaStreamCreateWithFlags(&B.side[i], cudaStreamNonBlocking)) == cudaSuccess)
       e = cudaEventCreateWithFlags(&B.join[i], cudaEventDisableTiming);
   if (e == cudaSuccess) e = cudaEventCreateWithFlags(&B.fork, cudaEventDisableTiming);
-  if (e == cudaSuccess) e = cudaMemcpy(B.q, q.data(), (size_t)nq * 24, cudaMemcpyHostToDevice);
-  if (e == cudaSuccess) e = cudaMemcpy(B.qn, qn.data(), (size_t)nq * 24, cudaMemcpyHostToDevice);
-  if (e == cudaSuccess) e = cudaMemcpy(B.sq, sq.data(), (size_t)ns * 24, cudaMemcpyHostToDevice);
-  if (e == cudaSuccess) e = cudaMemcpy(B.sqn, sqn.data(), (size_t)ns * 24, cudaMemcpyHostToDevice);
+  if (e == cudaSuccess) e = skw::copy_in(B.q, q.data(), (size_t)nq * 24);
+  if (e == cudaSuccess) e = skw::copy_in(B.qn, qn.data(), (size_t)nq * 24);
+  if (e == cudaSuccess) e = skw::copy_in(B.sq, sq.data(), (size_t)ns * 24);
+  if (e == cudaSuccess) e = skw::copy_in(B.sqn, sqn.data(), (size_t)ns * 24);
   if (e != cudaSuccess) return cuda_fail(ctx, e, "irradiance photon buffers");
   std::vector<float> ext((size_t)nq * 3), intr((size_t)nq * 3);
   std::vector<int32_t> nearest((size_t)ns);

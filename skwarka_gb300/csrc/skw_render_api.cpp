@@ -33,7 +33,7 @@ cudaError_t upload(skw_scene *s, const std::vector<T> &v, const T **out) {
   cudaError_t e = cudaMalloc(&p, v.size() * sizeof(T));
   if (e != cudaSuccess) return e;
   s->buffers.push_back(p);
-  e = cudaMemcpy(p, v.data(), v.size() * sizeof(T), cudaMemcpyHostToDevice);
+  e = skw::copy_in(p, v.data(), v.size() * sizeof(T));
   *out = (const T *)p;
   return e;
 }
@@ -1272,8 +1272,7 @@ int skw_render_batch_create(skw_scene *s, const skw_camera *cams, int32_t n_view
   int rc = batch_configure(b, to_pass_config(cfg));
   if (rc == SKW_OK) {
     if ((e = cudaMalloc((void **)&b->d_views, sizeof(skw::ViewDev) * (size_t)n_views)) != cudaSuccess ||
-        (e = cudaMemcpy(b->d_views, b->plan.views.data(), sizeof(skw::ViewDev) * (size_t)n_views,
-                        cudaMemcpyHostToDevice)) != cudaSuccess ||
+        (e = skw::copy_in(b->d_views, b->plan.views.data(), sizeof(skw::ViewDev) * (size_t)n_views)) != cudaSuccess ||
         (e = cudaStreamCreateWithFlags(&b->own, cudaStreamNonBlocking)) != cudaSuccess ||
         (e = cudaStreamCreateWithFlags(&b->side, cudaStreamNonBlocking)) != cudaSuccess ||
         (e = cudaEventCreateWithFlags(&b->ev_in, cudaEventDisableTiming)) != cudaSuccess ||
