@@ -223,10 +223,10 @@ typedef struct skw_hit_d {
  * IntersectTest on the reference's own ray type (TriangleAccelerator.cpp:
  * 154-352, 354-468).  Nodes are culled in float with bounds that cover the
  * rounding of the ray to float, so a node is skipped only if the reference
- * skips it; every triangle of a reached leaf is tested with the reference's
- * double Moller-Trumbore on the double ray, so the hit ids and t are the
- * reference's, bit for bit.  Slower than the float entry points (every
- * triangle test runs in double). */
+ * skips it; a triangle of a reached leaf is decided in float where a bound that
+ * covers that rounding allows it, else with the reference's double
+ * Moller-Trumbore on the double ray, which also gives every hit's t, so the hit
+ * ids and t are the reference's, bit for bit. */
 int skw_intersect_d(skw_accel *accel, const skw_ray_d *rays, int64_t n, skw_hit_d *hits, void *stream);
 int skw_intersect_test_d(skw_accel *accel, const skw_ray_d *rays, int64_t n, uint8_t *occluded, void *stream);
 /* The same with host buffers; waits for completion. */
