@@ -226,14 +226,15 @@ __device__ __forceinline__ void add_albedo_grad(float4 *g, V3 v) {
                : "memory");
 }
 
-// g_albedo (3 floats per triangle) += the sums.
-__global__ void k_albedo_grad(const float4 *__restrict__ sum, int64_t n, float *__restrict__ g_albedo) {
+// g_albedo (3 floats per triangle) += the sums, atomically: adjoints on other
+// streams may be adding to the same gradient.
+__global__ void k_albedo_grad(const float4 *__restrict__ sum, int64_t n, float *g_albedo) {
   const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= n) return;
   const float4 v = sum[i];
-  g_albedo[3 * i] += v.x;
-  g_albedo[3 * i + 1] += v.y;
-  g_albedo[3 * i + 2] += v.z;
+  if (v.x != 0.0f) atomicAdd(g_albedo + 3 * i, v.x);
+  if (v.y != 0.0f) atomicAdd(g_albedo + 3 * i + 1, v.y);
+  if (v.z != 0.0f) atomicAdd(g_albedo + 3 * i + 2, v.z);
 }
 
 // A warp's part of the emission gradient over a kernel's strides: the warp
