@@ -114,15 +114,17 @@ struct SlabRay {
   uint32_t bits;
 };
 
-// widen_u: the widening in units of u -- 6 for a float ray; 9 for a double
-// ray rounded to float, whose rounding moves a plane distance by at most
-// u |o| |1/d| (origin) + u |b - o| |1/d| (direction) more.
-__device__ __forceinline__ SlabRay make_slab_ray(const RayF &r, float scene_abs, float widen_u = 6.0f) {
+// The widening is 6u for a float ray; 9u for a double ray rounded to float
+// (ROUNDED), whose rounding moves a plane distance by at most
+// u |o| |1/d| (origin) + u |b - o| |1/d| (direction) more, and whose plane
+// distances, beyond a float's range on an axis, leave that axis out.
+template <bool ROUNDED>
+__device__ __forceinline__ SlabRay make_slab_ray(const RayF &r, float scene_abs) {
   SlabRay s;
   s.ix = 1.0f / r.dx;
   s.iy = 1.0f / r.dy;
   s.iz = 1.0f / r.dz;
-  const float c = widen_u * 5.9604645e-8f;
+  constexpr float c = (ROUNDED ? 9.0f : 6.0f) * 5.9604645e-8f;
   const float wx = c * (scene_abs + fabsf(r.ox)) * fabsf(s.ix);
   const float wy = c * (scene_abs + fabsf(r.oy)) * fabsf(s.iy);
   const float wz = c * (scene_abs + fabsf(r.oz)) * fabsf(s.iz);
@@ -133,6 +135,13 @@ __device__ __forceinline__ SlabRay make_slab_ray(const RayF &r, float scene_abs,
   s.fx = ox + wx;
   s.fy = oy + wy;
   s.fz = oz + wz;
+  if (ROUNDED) {  // the distances are within w / c
+    constexpr float most = c * 1.0e38f;
+    const float inf = __int_as_float(0x7f800000);
+    if (!(wx < most)) s.ix = 0.0f, s.nx = -inf, s.fx = inf;
+    if (!(wy < most)) s.iy = 0.0f, s.ny = -inf, s.fy = inf;
+    if (!(wz < most)) s.iz = 0.0f, s.nz = -inf, s.fz = inf;
+  }
   s.tmin = r.tmin;
   s.tmax = r.tmax;
   s.bits = (r.dx > 0.0f ? 0u : 1u) | (r.dy > 0.0f ? 0u : 2u) | (r.dz > 0.0f ? 0u : 4u) |
@@ -374,7 +383,6 @@ __global__ void __launch_bounds__(SKW_TRAV_BLOCK, SKW_TRAV_MINB)
   bool fin = true;   // its walk is over; its result waits while ray_i >= 0
   bool hit = false;  // any hit: the result
   RayF r{};          // read only by the triangle tests
-  constexpr float kSlabWiden = DRAY ? 9.0f : 6.0f;
   uint32_t cur_a = 0, cur_b = 0;
   float cur_lo = 0.0f;
   int best_slot = -1;
@@ -436,7 +444,7 @@ __global__ void __launch_bounds__(SKW_TRAV_BLOCK, SKW_TRAV_MINB)
             lo_t = r.tmax;
           }
           hi_t = r.tmax;
-          const SlabRay s = make_slab_ray(r, scene_abs, kSlabWiden);
+          const SlabRay s = make_slab_ray<DRAY>(r, scene_abs);
           best_slot = -1;
           flags = 8u;
           hit = false;
@@ -461,7 +469,7 @@ __global__ void __launch_bounds__(SKW_TRAV_BLOCK, SKW_TRAV_MINB)
     // The slab data (14 words) is made from the ray in every round instead of
     // being held through the triangle tests (measured at 80 registers, 4M
     // closest hits: 3.69 -> 3.50 ms).
-    const SlabRay s = make_slab_ray(r, scene_abs, kSlabWiden);
+    const SlabRay s = make_slab_ray<DRAY>(r, scene_abs);
 
     // Node steps continue past a lane's first leaf (postponed) until all but
     // SKW_TRAV_LAG walking lanes hold one, or the lane reaches a second leaf;
