@@ -762,7 +762,7 @@ __device__ bool own_light_leaf_occludes(const SceneDev &S, int j, D3 x, const Me
       return false;
   }
   const int first = __float_as_int(lb[6]), count = __float_as_int(lb[7]);
-  const float pf[3] = {(float)p.x, (float)p.y, (float)p.z};
+  const float pf[3] = {(float)p.x, (float)p.y, (float)p.z}, under = tri_under(rf, S.scene_abs);
   for (int k = 0; k < count; ++k) {
     const float4 ta = S.accel_tris[3 * (first + k)], tb = S.accel_tris[3 * (first + k) + 1],
                  tc = S.accel_tris[3 * (first + k) + 2];
@@ -777,7 +777,7 @@ __device__ bool own_light_leaf_occludes(const SceneDev &S, int j, D3 x, const Me
     if (!near) continue;
     float tt, et;
     const int res = tri_test32<true>(rf, make_float3(va[0], va[1], va[2]), make_float3(vb[0], vb[1], vb[2]),
-                                     make_float3(vc[0], vc[1], vc[2]), tt, et);
+                                     make_float3(vc[0], vc[1], vc[2]), tt, et, under);
     if (res == kMiss) continue;
     // Moller-Trumbore in double (TriangleAccelerator.cpp:419-452)
     const D3 w0{(double)ta.x, (double)ta.y, (double)ta.z};

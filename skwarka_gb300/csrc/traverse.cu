@@ -509,13 +509,14 @@ __global__ void __launch_bounds__(SKW_TRAV_BLOCK, SKW_TRAV_MINB)
     }
     __syncwarp(busy);
     if (has_post) {
+      const float under = DRAY ? tri_under(r, scene_abs) : 0.0f;
       for (uint32_t k = 0; k < post_cnt; ++k) {
         const int slot = (int)(post_a + k);
         float3 v0, v1, v2;
         int prim, tri;
         load_tri(tris, (uint32_t)slot, v0, v1, v2, prim, tri);
         float t, et;
-        const int res = tri_test32<DRAY>(r, v0, v1, v2, t, et);
+        const int res = tri_test32<DRAY>(r, v0, v1, v2, t, et, under);
         if (res == kMiss) continue;
         // A ray leaving a surface (surf) starts at an upper bound of the
         // reference's GetNextMinT: a triangle whose t cannot be told apart
