@@ -511,9 +511,10 @@ __global__ void __launch_bounds__(kSmallWarps * 32) k_split_small(Dev D) {
         x.lo[0] = p.x, x.lo[1] = p.y, x.lo[2] = p.z;
         x.hi[0] = q.x, x.hi[1] = q.y, x.hi[2] = q.z;
         x.n = 1u;
-        if (i >= __float_as_int(p.w)) box_unite(L, x);
-        else if (i < __float_as_int(q.w)) box_unite(R, x);
-        else box_unite(M, x);
+        const bool left = i >= __float_as_int(p.w), right = i < __float_as_int(q.w);
+        if (left) box_unite(L, x);
+        if (right) box_unite(R, x);  // (both: only where the planes per unit of length are infinite)
+        if (!left && !right) box_unite(M, x);
       }
       float cl = INFINITY, ch = INFINITY;
       if (i < tries) plane_cost_bounds(L, M, R, inv_f, cl, ch);
