@@ -239,6 +239,11 @@ int skw_flat_tree_leaf_ranges(const skw_flat_tree *t, uint32_t leaf_word_a, uint
   return SKW_OK;
 }
 
+// Accelerators of at least this many triangles (and no instancing) build
+// their tree on the GPU; below it the host build is as fast, and the tree
+// stays on the host too.
+constexpr int64_t kDeviceBuildMin = 16384;
+
 // An accelerator of a tree: uploaded, or (`dev` given) taken over from the
 // device tree, which is then empty.
 static int accel_from_tree(skw_ctx *ctx, const skw_flat_tree *tree, skw::DeviceTree *dev, skw_accel **out) {
@@ -297,6 +302,13 @@ static int accel_from_tree(skw_ctx *ctx, const skw_flat_tree *tree, skw::DeviceT
   info.build_ms = tree->build_ms;
   info.built_on_device = tree->on_device ? 1 : 0;
   info.device_bytes = (int64_t)(nb + tb + ib + eb);
+  if (!dev && (int64_t)n_tris < kDeviceBuildMin) {
+    a->h_nodes = ft.nodes;
+    for (const DevTri &t : ft.tris) {
+      a->h_prim.push_back(t.prim);
+      a->h_tri.push_back(t.tri);
+    }
+  }
   // instances need the stack of the top tree and of the deepest subtree at once
   if (a->d_inst) skw::register_instances(a->d_nodes, a->d_inst, a->d_leaf_ext);
   skw::register_ray_counter(a->d_nodes, a->d_traced);
@@ -309,10 +321,6 @@ int skw_accel_create_from_flat(skw_ctx *ctx, const skw_flat_tree *tree, skw_acce
   *out = nullptr;
   return accel_from_tree(ctx, tree, nullptr, out);
 }
-
-// Accelerators of at least this many triangles (and no instancing) build
-// their tree on the GPU; below it the host build is as fast.
-constexpr int64_t kDeviceBuildMin = 16384;
 
 int skw_accel_create(skw_ctx *ctx, const skw_mesh *meshes, int32_t n_meshes, const skw_primitive *prims,
                      int32_t n_prims, skw_accel **out) {
@@ -357,9 +365,9 @@ int skw_accel_get_info(const skw_accel *a, skw_accel_info *info) {
   return SKW_OK;
 }
 
-// Writes one word per page of a caller's buffer from several threads: a
-// copy into fresh pages otherwise takes their faults one by one (72 MB:
-// 3.5 ms against 2.1 with the writes).
+// Writes one byte per page of a caller's buffer, its own, from several
+// threads: a copy into fresh pages otherwise takes their faults one by one
+// (72 MB: 3.5 ms against 2.1 with the writes).
 static void touch_pages(void *p, size_t bytes) {
   constexpr size_t kStep = 4096, kMin = 4 << 20;
   const size_t nt = std::min<size_t>({bytes / kMin, 8, (size_t)std::max(1u, std::thread::hardware_concurrency())});
@@ -369,7 +377,7 @@ static void touch_pages(void *p, size_t bytes) {
     for (size_t w = 0; w < nt; ++w)
       pool[w] = std::thread([=]() {
         volatile char *c = (volatile char *)p;
-        for (size_t i = bytes / nt * w; i < (w + 1 == nt ? bytes : bytes / nt * (w + 1)); i += kStep) c[i] = 0;
+        for (size_t i = bytes / nt * w; i < (w + 1 == nt ? bytes : bytes / nt * (w + 1)); i += kStep) c[i] = c[i];
       });
   } catch (...) {  // no thread to be had: the copy takes the faults
   }
@@ -377,31 +385,69 @@ static void touch_pages(void *p, size_t bytes) {
     if (t.joinable()) t.join();
 }
 
-// Read straight from the device, on a stream of its own: a caller's capture
-// on another stream stays valid.
+// The primitive and mesh triangle of every slot, gathered on the device in a
+// workspace of the context's pool, or where there is no room for that, on the
+// host from the triangles, some at a time.
+static cudaError_t export_ids(const skw_accel *a, int32_t *tri_prim, int32_t *tri_index, cudaStream_t st) {
+  const size_t n = (size_t)a->info.n_triangles;
+  cudaMemPool_t pool;
+  int32_t *ids = nullptr;
+  if (skw::ctx_pool(a->ctx, &pool) == cudaSuccess &&
+      cudaMallocFromPoolAsync((void **)&ids, n * 8, pool, st) == cudaSuccess) {
+    cudaError_t e = skw::launch_slot_ids(a->d_tris, (int64_t)n, ids, ids + n, st);
+    if (e == cudaSuccess && tri_prim) e = cudaMemcpyAsync(tri_prim, ids, n * 4, cudaMemcpyDeviceToHost, st);
+    if (e == cudaSuccess && tri_index) e = cudaMemcpyAsync(tri_index, ids + n, n * 4, cudaMemcpyDeviceToHost, st);
+    cudaFreeAsync(ids, st);
+    return e;
+  }
+  cudaGetLastError();  // the refused workspace
+  constexpr size_t kSome = 256;
+  DevTri some[kSome];
+  for (size_t i = 0; i < n; i += kSome) {
+    const size_t c = std::min(kSome, n - i);
+    cudaError_t e = cudaMemcpyAsync(some, a->d_tris + i, c * sizeof(DevTri), cudaMemcpyDeviceToHost, st);
+    if (e == cudaSuccess) e = cudaStreamSynchronize(st);
+    if (e != cudaSuccess) return e;
+    for (size_t k = 0; k < c; ++k) {
+      if (tri_prim) tri_prim[i + k] = some[k].prim;
+      if (tri_index) tri_index[i + k] = some[k].tri;
+    }
+  }
+  return cudaSuccess;
+}
+
+// A small tree is on the host.  Others are read from the device, on a stream
+// of its own, so that a caller's capture on another stream stays valid and
+// nothing else on the GPU is waited for; the calling thread keeps its current
+// device.
 int skw_accel_export(const skw_accel *a, uint32_t *nodes, int32_t *tri_prim, int32_t *tri_index) {
   if (!a) return SKW_ERR_ARG;
   const size_t n = (size_t)a->info.n_triangles, nb = (size_t)a->info.n_nodes * sizeof(DevNode);
-  cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
-  cudaError_t e = cudaSetDevice(a->ctx->device);
-  if (e == cudaSuccess) e = cudaThreadExchangeStreamCaptureMode(&mode);
-  if (e != cudaSuccess) return cuda_fail(a->ctx, e, "export (accelerator)");
-  cudaStream_t st = nullptr;
-  int32_t *ids = nullptr;
-  e = cudaStreamCreateWithFlags(&st, cudaStreamNonBlocking);
-  if (e == cudaSuccess && n > 0 && (tri_prim || tri_index)) {
-    e = cudaMalloc(&ids, n * 8);
-    if (e == cudaSuccess) e = skw::launch_slot_ids(a->d_tris, (int64_t)n, ids, ids + n, st);
+  if (!a->h_nodes.empty()) {
+    if (nodes) std::memcpy(nodes, a->h_nodes.data(), nb);
+    if (tri_prim && n > 0) std::memcpy(tri_prim, a->h_prim.data(), n * 4);
+    if (tri_index && n > 0) std::memcpy(tri_index, a->h_tri.data(), n * 4);
+    return SKW_OK;
   }
+  int device = a->ctx->device;
+  cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
+  cudaStream_t st = nullptr;
+  cudaGetDevice(&device);
+  cudaError_t e = cudaThreadExchangeStreamCaptureMode(&mode);
+  if (e != cudaSuccess) return cuda_fail(a->ctx, e, "export (accelerator)");
+  e = cudaSetDevice(a->ctx->device);
+  if (e == cudaSuccess) e = cudaStreamCreateWithFlags(&st, cudaStreamNonBlocking);
+  if (e == cudaSuccess && n > 0 && (tri_prim || tri_index)) e = export_ids(a, tri_prim, tri_index, st);
   if (e == cudaSuccess && nodes) {
     touch_pages(nodes, nb);
     e = cudaMemcpyAsync(nodes, a->d_nodes, nb, cudaMemcpyDeviceToHost, st);
   }
-  if (e == cudaSuccess && ids && tri_prim) e = cudaMemcpyAsync(tri_prim, ids, n * 4, cudaMemcpyDeviceToHost, st);
-  if (e == cudaSuccess && ids && tri_index) e = cudaMemcpyAsync(tri_index, ids + n, n * 4, cudaMemcpyDeviceToHost, st);
-  if (e == cudaSuccess) e = cudaStreamSynchronize(st);
-  if (st) cudaStreamDestroy(st);
-  cudaFree(ids);
+  if (st) {
+    const cudaError_t done = cudaStreamSynchronize(st);
+    if (e == cudaSuccess) e = done;
+    cudaStreamDestroy(st);
+  }
+  if (device != a->ctx->device) cudaSetDevice(device);
   cudaThreadExchangeStreamCaptureMode(&mode);
   if (e != cudaSuccess) return cuda_fail(a->ctx, e, "export (accelerator)");
   return SKW_OK;

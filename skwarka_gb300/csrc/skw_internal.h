@@ -43,6 +43,9 @@ struct skw_accel {
   int stack_cap = 0;
   float scene_abs = 0.0f;  // largest absolute vertex coordinate
   skw_accel_info info{};
+  // A small host-built tree as exported (empty: it is read from the device).
+  std::vector<skw::DevNode> h_nodes;
+  std::vector<int32_t> h_prim, h_tri;
 };
 
 // A render scene (skw_scene_create): its accelerator plus the shading data.
