@@ -273,17 +273,18 @@ static int accel_from_tree(skw_ctx *ctx, const skw_flat_tree *tree, skw::DeviceT
   const size_t ib = ft.inst.size() * sizeof(skw::DevInst), eb = ft.leaf_ext.size() * sizeof(skw::LeafExt);
   if (!ft.inst.empty() && ((e = cudaMalloc(&a->d_inst, ib)) != cudaSuccess ||
                            (e = cudaMalloc(&a->d_leaf_ext, std::max<size_t>(eb, 16))) != cudaSuccess ||
-                           (e = skw::copy_in(a->d_inst, ft.inst.data(), ib)) != cudaSuccess ||
-                           (eb > 0 && (e = skw::copy_in(a->d_leaf_ext, ft.leaf_ext.data(), eb)) !=
+                           (e = cudaMemcpy(a->d_inst, ft.inst.data(), ib, cudaMemcpyHostToDevice)) != cudaSuccess ||
+                           (eb > 0 && (e = cudaMemcpy(a->d_leaf_ext, ft.leaf_ext.data(), eb, cudaMemcpyHostToDevice)) !=
                                           cudaSuccess))) {
     skw_accel_destroy(a);
     return cuda_fail(ctx, e, "instance tables");
   }
-  if ((!dev && ((e = skw::copy_in(a->d_nodes, ft.nodes.data(), nb)) != cudaSuccess ||
-                (n_tris > 0 && (e = skw::copy_in(a->d_tris, ft.tris.data(), n_tris * sizeof(DevTri))) != cudaSuccess))) ||
+  if ((!dev && ((e = cudaMemcpy(a->d_nodes, ft.nodes.data(), nb, cudaMemcpyHostToDevice)) != cudaSuccess ||
+                (n_tris > 0 && (e = cudaMemcpy(a->d_tris, ft.tris.data(), n_tris * sizeof(DevTri),
+                                               cudaMemcpyHostToDevice)) != cudaSuccess))) ||
       (e = cudaMemset(a->d_status, 0, sizeof(unsigned))) != cudaSuccess ||
       (e = cudaMemset(a->d_traced, 0, sizeof(unsigned long long))) != cudaSuccess ||
-      (e = cudaStreamSynchronize(nullptr)) != cudaSuccess) {  // queries may come on any stream
+      (e = cudaStreamSynchronize(nullptr)) != cudaSuccess) {  // queries may come on any stream (copy_in)
     skw_accel_destroy(a);
     return cuda_fail(ctx, e, "upload (accelerator)");
   }

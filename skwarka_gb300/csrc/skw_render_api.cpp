@@ -33,7 +33,7 @@ cudaError_t upload(skw_scene *s, const std::vector<T> &v, const T **out) {
   cudaError_t e = cudaMalloc(&p, v.size() * sizeof(T));
   if (e != cudaSuccess) return e;
   s->buffers.push_back(p);
-  e = skw::copy_in(p, v.data(), v.size() * sizeof(T));
+  e = cudaMemcpy(p, v.data(), v.size() * sizeof(T), cudaMemcpyHostToDevice);
   *out = (const T *)p;
   return e;
 }
@@ -468,8 +468,8 @@ int skw_scene_create(skw_ctx *ctx, const skw_mesh *meshes, int32_t n_meshes, con
     if (e == cudaSuccess)
       e = skw::launch_light_leaves(s->accel->d_nodes, s->accel->info.n_nodes, s->accel->d_leaf_ext, s->accel->d_tris,
                                    D.prim_tri_offset, keys, (int64_t)light_key.size(), (float *)D.light_leaf, nullptr);
-    if (e == cudaSuccess) e = cudaStreamSynchronize(nullptr);
   }
+  if (e == cudaSuccess) e = cudaStreamSynchronize(nullptr);  // renders may come on any stream (copy_in)
   if (e != cudaSuccess) {
     skw_scene_destroy(s);
     return cuda_fail(ctx, e, "render scene upload");
