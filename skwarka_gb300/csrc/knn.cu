@@ -769,11 +769,13 @@ __global__ void __launch_bounds__(kKnnBlock, KMAX == 128 ? 16 : 24) k_knn_gang(
 }
 
 // GetNearestPoint (KDTree.h:495-503) with NearestPointProc (:293-323):
-// every accepted point becomes the nearest and shrinks the radius.
-template <int S>
+// every accepted point becomes the nearest and shrinks the radius.  BOUNDED:
+// a walk that has not ended after `budget` nodes is given up (kUnfinished).
+constexpr int kUnfinished = -2;
+template <int S, bool BOUNDED>
 __device__ __forceinline__ int nearest_walk(Tree T, const uint16_t *__restrict__ nids,
                                             const double *__restrict__ dirs, const Query &Q, double max_dist, uint2 (*stk)[kKnnBlock],
-                                            unsigned *__restrict__ status) {
+                                            unsigned *__restrict__ status, int budget) {
   int best = -1;
   if (T.n <= 0) return best;
   Radius rad;
@@ -781,6 +783,7 @@ __device__ __forceinline__ int nearest_walk(Tree T, const uint16_t *__restrict__
   int sp = 0, cur = 0;
   NodeN p = T.load(0, Q.filter);
   for (;;) {
+    if (BOUNDED && budget-- == 0) return kUnfinished;
     int near, far;
     float s2;
     node_children(p.p, cur, T.n, Q, near, far, s2);
@@ -841,22 +844,28 @@ __global__ void __launch_bounds__(kKnnBlock, SKW_KNN_MINB) k_nearest(Tree T, con
   if (order) i = order[i];
   Query Q;
   load_query(Q, q, qn, i, cos_t);
-  out_idx[i] = nearest_walk<S>(T, nids, dirs, Q, max_dist, stk, status);
+  out_idx[i] = nearest_walk<S, false>(T, nids, dirs, Q, max_dist, stk, status, 0);
 }
 
-// The same by looking at every point, one warp per query: for launches of few
-// queries over few points, whose time is their longest walk -- a query whose
-// filter takes no point near it walks the whole tree, one node after the
-// other.  Equal exact distances are settled by the walk (the first visited
-// stays), and so is the answer wherever one is met.
+// The walk of lane 0 where a scan met equal distances.
 template <int S>
-__global__ void __launch_bounds__(kKnnBlock, SKW_KNN_MINB) k_nearest_scan(
-    Tree T, const uint16_t *__restrict__ nids, const double *__restrict__ dirs,
-    const double *__restrict__ q, const double *__restrict__ qn, int64_t nq, double max_dist, double cos_t,
-    int32_t *__restrict__ out_idx, unsigned *__restrict__ status) {
-  static_assert(kKnnBlock == 32, "one query per block");
-  __shared__ uint2 stk[S][kKnnBlock];
-  const int64_t i = blockIdx.x;
+__device__ __noinline__ int nearest_walk_alone(Tree T, const uint16_t *nids, const double *dirs, const double *q,
+                                               const double *qn, int64_t i, double max_dist, double cos_t,
+                                               uint2 (*stk)[kKnnBlock], unsigned *status) {
+  Query Q;
+  load_query(Q, q, qn, i, cos_t);
+  return nearest_walk<S, false>(T, nids, dirs, Q, max_dist, stk, status, 0);
+}
+
+// The nearest point of query i by looking at every point, one warp.  Equal
+// exact distances are settled by the walk (the first visited stays), and so
+// is the answer wherever one is met.
+template <int S>
+__device__ __forceinline__ void nearest_scan(Tree T, const uint16_t *__restrict__ nids,
+                                             const double *__restrict__ dirs, const double *__restrict__ q,
+                                             const double *__restrict__ qn, int64_t i, double max_dist, double cos_t,
+                                             int32_t *__restrict__ out_idx, uint2 (*stk)[kKnnBlock],
+                                             unsigned *__restrict__ status) {
   const int lane = threadIdx.x;
   Query Q;
   load_query(Q, q, qn, i, cos_t);
@@ -896,12 +905,36 @@ __global__ void __launch_bounds__(kKnnBlock, SKW_KNN_MINB) k_nearest_scan(
   const unsigned who = __ballot_sync(0xffffffffu, best >= 0 && mine == least);
   const bool ties = __ballot_sync(0xffffffffu, tie) != 0u || __popc(who) > 1;
   if (ties) {
-    if (lane == 0) out_idx[i] = nearest_walk<S>(T, nids, dirs, Q, max_dist, stk, status);
+    if (lane == 0) out_idx[i] = nearest_walk_alone<S>(T, nids, dirs, q, qn, i, max_dist, cos_t, stk, status);
   } else if (who == 0u) {
     if (lane == 0) out_idx[i] = -1;
   } else if (lane == __ffs(who) - 1) {
     out_idx[i] = best;
   }
+}
+
+// Launches of few queries over few points: their time is their longest walk,
+// and a query whose filter takes no point near it walks the whole tree, one
+// node after the other.  A walk is given up after `budget` nodes, and its warp
+// looks at every point instead.
+template <int S>
+__global__ void __launch_bounds__(kKnnBlock, 16) k_nearest_few(
+    Tree T, const uint16_t *__restrict__ nids, const double *__restrict__ dirs,
+    const double *__restrict__ q, const double *__restrict__ qn, int64_t nq, double max_dist, double cos_t,
+    int32_t *__restrict__ out_idx, unsigned *__restrict__ status, int per_warp, int budget) {
+  static_assert(kKnnBlock == 32, "one warp per block");
+  __shared__ uint2 stk[S][kKnnBlock];
+  const int lane = threadIdx.x;
+  const int64_t first = (int64_t)blockIdx.x * per_warp, i = first + lane;
+  int found = -1;
+  if (lane < per_warp && i < nq) {
+    Query Q;
+    load_query(Q, q, qn, i, cos_t);
+    found = nearest_walk<S, true>(T, nids, dirs, Q, max_dist, stk, status, budget);
+    if (found != kUnfinished) out_idx[i] = found;
+  }
+  for (unsigned left = __ballot_sync(0xffffffffu, found == kUnfinished); left != 0u; left &= left - 1u)
+    nearest_scan<S>(T, nids, dirs, q, qn, first + __ffs(left) - 1, max_dist, cos_t, out_idx, stk, status);
 }
 
 // Walk stack entries for a tree of n points (see walk).
@@ -922,18 +955,20 @@ inline unsigned knn_grid(int64_t nq, int per_warp) {
   return (unsigned)((nq + per_block - 1) / per_block);
 }
 
-// Nearest points by scan: the query's n / 128 rounds take what they take
-// whatever the filter does, about a usual walk's time at kScanPoints points,
-// but a few queries alone walk a tree of thousands faster than one warp scans
-// it, and unfiltered walks are short (scan against walk: 8,000 points, 100
-// filtered queries 115 / 646 us, 8,000 unfiltered 90 / 129 us, one unfiltered
-// 32 / 19 us; 1,000 points, one query 11 / 15 us; the photon maps' 5,848
-// filtered queries over 6,427 points 0.14 / 2.52 ms).
-constexpr int64_t kScanPoints = 8192, kScanFewPoints = 2048, kScanFewQueries = 64, kScanQueries = 16384,
-                  kScanPairs = (int64_t)1 << 26;
-inline bool nearest_by_scan(int64_t nq, int64_t n, bool filter) {
-  return n <= kScanPoints && nq <= kScanQueries && (n <= kScanFewPoints || nq >= kScanFewQueries) &&
-         (filter || nq * n <= kScanPairs);
+// Nearest points of few queries over few points: k_nearest_few, or with no
+// walk at all (budget 0) where looking at every point takes no longer than a
+// short walk.  Else a walk is given up after half as many nodes as its warp
+// would take rounds of 128 points to look at all of them for each of its
+// queries (a round takes about a node's time), so that a launch is never far
+// from the less of walking and looking.  16,384 queries over 8,000 points, us,
+// by full warps' walks / by looking alone / so: all points pass 76 / 84 / 38,
+// the normals alike 86 / 272 / 41, radii of a point or two 30 / 122 / 19, a
+// filter that no near point passes 6,850 / 286 / 665; 64 queries over 2,000
+// points, the same: 59 / 22 / 22, 65 / 28 / 28, 17 / 16 / 16, 1,600 / 33 / 33.
+constexpr int64_t kScanPoints = 8192, kScanQueries = 16384, kLookPoints = 2048, kLookQueries = 2048, kLookFrom = 16;
+inline int nearest_budget(int64_t nq, int n, int per_warp) {
+  if (n <= kLookPoints && nq >= kLookFrom && nq <= kLookQueries) return 0;
+  return n * per_warp / 256 + 24;
 }
 
 // Levels of the median-split tree of n points: as many entries as a walk's
@@ -1284,14 +1319,12 @@ cudaError_t launch_nearest(const void *nodes, const uint16_t *nids, const double
                            unsigned *status, cudaStream_t stream, const int *nq_dev, const int32_t *order) {
   if (nq <= 0) return cudaSuccess;
   const Tree T = tree_of(nodes, nids, n);
-  if (!nq_dev && !order && nearest_by_scan(nq, n, cos_t >= 0.0)) {
-    k_nearest_scan<kShallowStack><<<(unsigned)nq, kKnnBlock, 0, stream>>>(
-        T, nids, dirs, q, qn, nq, max_dist, cos_t, out_idx, status);
-    return cudaGetLastError();
-  }
   const int per_warp = queries_per_warp(nq);
   const unsigned grid = knn_grid(nq, per_warp);
-  if (shallow_tree(n))
+  if (!nq_dev && !order && n <= kScanPoints && nq <= kScanQueries)
+    k_nearest_few<kShallowStack><<<grid, kKnnBlock, 0, stream>>>(T, nids, dirs, q, qn, nq, max_dist, cos_t, out_idx,
+                                                                 status, per_warp, nearest_budget(nq, n, per_warp));
+  else if (shallow_tree(n))
     k_nearest<kShallowStack><<<grid, kKnnBlock, 0, stream>>>(T, nids, dirs, q, qn, nq, max_dist,
                                                          cos_t, out_idx, status, nq_dev, order, per_warp);
   else
