@@ -946,9 +946,18 @@ inline bool shallow_tree(int n) { return n < (1 << kShallowStack); }
 // resident at k = 100 -- spreads them (the photon maps' 6,427 irradiance
 // estimates: 3.90 -> 1.94 ms in 4s; 2s and 1s measure the same).
 constexpr int64_t kSpreadWarps = 2048;
-inline int queries_per_warp(int64_t nq) {
-  const int64_t per = (nq + kSpreadWarps - 1) / kSpreadWarps;
+inline int queries_per_warp(int64_t nq, int64_t warps = kSpreadWarps) {
+  const int64_t per = (nq + warps - 1) / warps;
   return (int)(per < 32 ? per : 32);
+}
+// Of heaps of more than 100 entries fewer fit into the SMs' shared memory
+// (k = 128: 11 a SM), and a launch of a few warps more than that takes a second
+// round of blocks (50,000 unfiltered queries of k = 128 with some 40 points
+// each: 337 us in 2,000 warps, 213 in 1,667).
+inline int64_t spread_warps(size_t smem) {
+  constexpr size_t kSms = 152, kPerSm = 228 << 10, kStack = kShallowStack * kKnnBlock * 4, kReserved = 1024;
+  const int64_t fit = (int64_t)(kSms * (kPerSm / (smem + kStack + kReserved)));
+  return fit < kSpreadWarps ? fit : kSpreadWarps;
 }
 inline unsigned knn_grid(int64_t nq, int per_warp) {
   const int64_t per_block = (int64_t)per_warp * (kKnnBlock / 32);
@@ -979,16 +988,16 @@ inline int tree_levels(int n) {
   return levels;
 }
 
-// Full warps with heaps of more than 32 entries: k_knn_gang.  The others:
+// Full warps with heaps of more than kGangEntries entries: k_knn_gang.  The others:
 // k_knn<KMAX, S> with S chosen by the tree's depth.
 template <int KMAX>
 void knn_kernel(cudaStream_t stream, const Tree &T, const uint16_t *nids, const double *dirs, const double *q,
                 const double *qn, int64_t nq, int k, double max_dist, double cos_t, int32_t *out_idx, double *out_d2,
                 int32_t *out_count, int32_t *out_visited, FCand *scratch, unsigned *status, const int *nq_dev,
                 const int32_t *order) {
-  const int per_warp = queries_per_warp(nq);
-  const unsigned grid = knn_grid(nq, per_warp);
   const size_t smem = KMAX > 0 ? SharedHeap::bytes(k) : 0;
+  const int per_warp = queries_per_warp(nq, spread_warps(smem));
+  const unsigned grid = knn_grid(nq, per_warp);
   if constexpr (KMAX != 32) {
     if (per_warp == 32 && k > kGangEntries) {
       const int depth = tree_levels(T.n);
