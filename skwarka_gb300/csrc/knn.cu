@@ -673,9 +673,10 @@ __global__ void __launch_bounds__(kKnnBlock, knn_min_blocks(KMAX)) k_knn(
 // 0.84 -> 0.59); and in warps with few queries (irradiance estimates 3.51 ->
 // 4.25 ms) no lane waits either.
 constexpr int kReplaceShare = 1, kMakeShare = 7, kGangEntries = 48;
+constexpr int kGangBlocks = 24;  // resident per SM with heaps in global memory
 
 template <int KMAX>
-__global__ void __launch_bounds__(kKnnBlock, KMAX == 128 ? 16 : 24) k_knn_gang(
+__global__ void __launch_bounds__(kKnnBlock, KMAX == 128 ? 16 : kGangBlocks) k_knn_gang(
     Tree T, const uint16_t *__restrict__ nids, const double *__restrict__ dirs, const double *__restrict__ q,
     const double *__restrict__ qn, int64_t nq, int k, double max_dist, double cos_t, int32_t *__restrict__ out_idx,
     double *__restrict__ out_d2, int32_t *__restrict__ out_count, int32_t *__restrict__ out_visited,
@@ -988,6 +989,14 @@ inline int tree_levels(int n) {
   return levels;
 }
 
+// Whether lanes wait for one another at heaps in global memory.  Beyond two
+// rounds of blocks the walks' number counts more than the waits (heaps and
+// nodes share L2).  k_knn_gang / k_knn, k = 200 over 270,000 points, radii of
+// 300 and of 600: 110,000 queries 3.71 / 5.65 and 5.47 / 6.91 ms, 130,000 5.41 /
+// 5.98 and 8.07 / 7.62, 200,000 7.75 / 10.42 and 11.34 / 12.57, 300,000 14.36 /
+// 13.77 and 21.62 / 19.86, 600,000 34.42 / 29.23 and 53.66 / 49.00.
+inline bool gang_in_global(int64_t nq) { return nq <= (int64_t)2 * 152 * kGangBlocks * kKnnBlock; }
+
 // Full warps with heaps of more than kGangEntries entries: k_knn_gang.  The others:
 // k_knn<KMAX, S> with S chosen by the tree's depth.
 template <int KMAX>
@@ -999,7 +1008,7 @@ void knn_kernel(cudaStream_t stream, const Tree &T, const uint16_t *nids, const 
   const int per_warp = queries_per_warp(nq, spread_warps(smem));
   const unsigned grid = knn_grid(nq, per_warp);
   if constexpr (KMAX != 32) {
-    if (per_warp == 32 && k > kGangEntries) {
+    if (per_warp == 32 && k > kGangEntries && (KMAX > 0 || gang_in_global(nq))) {
       const int depth = tree_levels(T.n);
       k_knn_gang<KMAX><<<grid, kKnnBlock, smem + (size_t)depth * kKnnBlock * sizeof(uint2), stream>>>(
           T, nids, dirs, q, qn, nq, k, max_dist, cos_t, out_idx, out_d2, out_count, out_visited, scratch, status, nq_dev,
