@@ -108,7 +108,6 @@ struct Dev {
   double *hcoef;              // 3 per node
   double *hsplit;
   int32_t *hid, *htries, *haxis, *hbase;  // hbase: a big node's first bucket
-  uint32_t *heads;            // the level's nodes' first slots, by rank
   uint32_t *hnl, *hnr;
   uint8_t *hleaf;
   double *bcost, *bpos;       // 3 per node
@@ -301,7 +300,6 @@ __global__ void k_head_setup(Dev D, int64_t level_base, int depth) {
     const int2 r = D.seg[s];
     const int64_t id = level_base + (int64_t)D.cnt[s];
     D.hid[s] = (int32_t)id;
-    D.heads[D.cnt[s]] = (uint32_t)s;
     float lo[3], hi[3];
     for (int c = 0; c < 3; ++c) {
       const unsigned long long kl = D.hkeys[s * 6 + c], kh = D.hkeys[s * 6 + 3 + c];
@@ -1190,7 +1188,6 @@ cudaError_t build_accel_tree_gpu(const std::vector<MeshJob> &jobs, int64_t min_n
   want(&D.hcoef, nn * 24);
   want(&D.hsplit, nn * 8);
   want(&D.hid, nn * 4);
-  want(&D.heads, nn * 4);
   want(&D.htries, nn * 4);
   want(&D.haxis, nn * 4);
   want(&D.hnl, nn * 4);
