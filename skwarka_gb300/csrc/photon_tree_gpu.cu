@@ -43,13 +43,15 @@ __device__ __forceinline__ uint32_t fkey(float f) {  // order-preserving bits of
 // ------------------------------------------------------------ scans --
 // Exclusive scan of n 64-bit values in place: the totals of tiles of 2,048
 // values, then every tile's scan after the totals before it, which each block
-// adds up itself (reading up to kScanTotals values costs less than a launch
-// of one block that scans them: 1.1M values took 23 us in three launches of
-// per-block scans, their totals' scan and the totals added back, 11 of it the
-// one block; the accelerator of 1.1M triangles, made and read back, 17.7 -> 16.6
-// ms with two).  Bound by its launches at the sizes of the tree builds.
+// adds up itself (1.1M values took 23 us in three launches of per-block scans,
+// their totals' scan and the totals added back, 11 of it the one block; the
+// accelerator of 1.1M triangles, made and read back, 17.7 -> 16.6 ms with two).
+// Bound by its launches at the sizes of the tree builds.
 constexpr int kScanTile = 2048, kScanPer = kScanTile / kBlock;
-// Beyond this many tiles the totals are scanned by a launch of their own.
+// Beyond this many tiles the totals are scanned by a launch of their own.  The
+// blocks' own sums grow with the square of the tiles; with / without the third
+// launch: 512 tiles 14.4 / 10.2 us, 2,048 24.6 / 20.5, 4,096 36.9 / 34.8, 8,192
+// (16.8M values) 83.6 / 80.7, 16,384 159 / 172, 32,768 302 / 406.
 constexpr int kScanTotals = 8192;
 
 // The sum over the block, in every thread.
