@@ -1,6 +1,7 @@
 """Shared fixtures.  `gpu` marks tests that need a CUDA device; everything
 else runs on CPU.  The oracle (oracle/) is the checker in these tests."""
 import os
+import subprocess
 import sys
 from pathlib import Path
 
@@ -14,6 +15,30 @@ if str(ROOT) not in sys.path:
 
 def pytest_configure(config):
     config.addinivalue_line("markers", "gpu: needs a CUDA GPU (runs on the GB300)")
+
+
+@pytest.fixture(autouse=True)
+def no_process_left(monkeypatch):
+    """Processes that a test started and did not wait for (it failed, or one of them ran out of time) end with it: on a
+    shared GPU they would go on computing."""
+    started = []
+
+    class Popen(subprocess.Popen):
+        def __init__(self, *args, **kwargs):
+            super().__init__(*args, **kwargs)
+            started.append(self)
+
+    monkeypatch.setattr(subprocess, "Popen", Popen)
+    yield
+    left = [p for p in started if p.poll() is None]
+    for p in left:
+        p.terminate()
+    for p in left:
+        try:
+            p.wait(timeout=5)
+        except subprocess.TimeoutExpired:
+            p.kill()
+            p.wait()
 
 
 @pytest.fixture(scope="session")
