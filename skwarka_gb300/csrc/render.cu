@@ -694,7 +694,8 @@ __device__ __noinline__ MediaSeq media_seq(unsigned k) {
 // comparisons, and a triangle the ray certainly misses is skipped
 // (tri_test32).  What is left in double is the ray itself, the slabs that p
 // lies on, and the triangle p lies on.
-__device__ bool own_light_leaf_occludes(const SceneDev &S, int j, D3 x, const MediaSeq &q, D3 &p_out,
+// under: tri_under of the march's rays.
+__device__ bool own_light_leaf_occludes(const SceneDev &S, int j, D3 x, const MediaSeq &q, float under, D3 &p_out,
                                         double &len_out) {
   const int g = S.light_tri[j];
   const int j0 = S.tri_vidx[3 * g], j1 = S.tri_vidx[3 * g + 1], j2 = S.tri_vidx[3 * g + 2];
@@ -764,7 +765,7 @@ __device__ bool own_light_leaf_occludes(const SceneDev &S, int j, D3 x, const Me
       return false;
   }
   const int first = __float_as_int(lb[6]), count = __float_as_int(lb[7]);
-  const float pf[3] = {(float)p.x, (float)p.y, (float)p.z}, under = tri_under(rf, S.scene_abs);
+  const float pf[3] = {(float)p.x, (float)p.y, (float)p.z};
   for (int k = 0; k < count; ++k) {
     const float4 ta = S.accel_tris[3 * (first + k)], tb = S.accel_tris[3 * (first + k) + 1],
                  tc = S.accel_tris[3 * (first + k) + 2];
@@ -893,6 +894,10 @@ __global__ void __launch_bounds__(kMediaBlock) k_media(SceneDev S, MediaArgs A, 
   const bool scatters = !black(ss);
   const int nlights = S.n_point_lights + S.n_area_lights;
   const V3 dirv = d * -1.0f;
+  // light rays start in the medium's box and have unit length
+  float box = 0.0f;
+  for (int a = 0; a < 3; ++a) box += fmaxf(fabsf(M.lo[a]), fabsf(M.hi[a]));
+  const float under = tri_under(S.scene_abs, box, 2.0f);
   double tb = t0;
   const double te = t1;
   V3 point = o + d * t0, rad = v3(0, 0, 0);
@@ -944,7 +949,7 @@ __global__ void __launch_bounds__(kMediaBlock) k_media(SceneDev S, MediaArgs A, 
         // light ray differently from the reference's double one)
         const D3 xd{__dadd_rn((double)o.x, __dmul_rn((double)d.x, tp)), __dadd_rn((double)o.y, __dmul_rn((double)d.y, tp)),
                     __dadd_rn((double)o.z, __dmul_rn((double)d.z, tp))};
-        self_occ = own_light_leaf_occludes(S, L.tri_begin + a, xd, seq, spd, lend);
+        self_occ = own_light_leaf_occludes(S, L.tri_begin + a, xd, seq, under, spd, lend);
         const V3 sp = v3((float)spd.x, (float)spd.y, (float)spd.z);
         const V3 to = sp - point;
         dist = len(to);

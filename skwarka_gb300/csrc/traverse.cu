@@ -135,8 +135,8 @@ __device__ __forceinline__ SlabRay make_slab_ray(const RayF &r, float scene_abs)
   s.fx = ox + wx;
   s.fy = oy + wy;
   s.fz = oz + wz;
-  if (ROUNDED) {  // the distances are within w / c
-    constexpr float most = c * 1.0e38f;
+  constexpr float most = c * 1.0e38f;  // the distances are within w / c
+  if (ROUNDED && !(wx + wy + wz < most)) {
     const float inf = __int_as_float(0x7f800000);
     if (!(wx < most)) s.ix = 0.0f, s.nx = -inf, s.fx = inf;
     if (!(wy < most)) s.iy = 0.0f, s.ny = -inf, s.fy = inf;
@@ -509,7 +509,9 @@ __global__ void __launch_bounds__(SKW_TRAV_BLOCK, SKW_TRAV_MINB)
     }
     __syncwarp(busy);
     if (has_post) {
-      const float under = DRAY ? tri_under(r, scene_abs) : 0.0f;
+      const float under = DRAY ? tri_under(scene_abs, fabsf(r.ox) + fabsf(r.oy) + fabsf(r.oz),
+                                           fabsf(r.dx) + fabsf(r.dy) + fabsf(r.dz))
+                               : 0.0f;
       for (uint32_t k = 0; k < post_cnt; ++k) {
         const int slot = (int)(post_a + k);
         float3 v0, v1, v2;

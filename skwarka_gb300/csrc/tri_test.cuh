@@ -26,8 +26,8 @@ namespace {
 // g / 2 times the other cross product, so that det, n1, n2 and nt are off by
 // at most 3g (1 + S1) S.  Their bounds get 8g (1 + S1) S (tri_under, from the
 // scene's largest coordinate B): the rest is for the roundings of the bounds
-// themselves, in that range too.  (200,001 closest hits over 1.1M triangles:
-// 518 us without, 525 with it.)
+// themselves, in that range too.  (200,001 closest hits over 1.1M triangles,
+// with the walk's guard for distances beyond a float: 539 us without, 556 with.)
 constexpr float kTriErr = 10.0f * 5.9604645e-8f, kTriErrD = 12.0f * 5.9604645e-8f;
 constexpr double kDblEps = 2.220446049250313e-16;
 
@@ -37,9 +37,9 @@ struct RayF {
   float ox, oy, oz, dx, dy, dz, tmin, tmax;
 };
 
-// The subnormal range's part of a double ray's bounds (above).
-__device__ __forceinline__ float tri_under(const RayF &r, float scene_abs) {
-  const float o = fabsf(r.ox) + fabsf(r.oy) + fabsf(r.oz), d = fabsf(r.dx) + fabsf(r.dy) + fabsf(r.dz);
+// The subnormal range's part of a double ray's bounds (above); o, d: the sums
+// of its origin's and direction's components' magnitudes.
+__device__ __forceinline__ float tri_under(float scene_abs, float o, float d) {
   return 1.1210388e-44f * (1.0f + 12.0f * scene_abs) * (1.0f + 15.0f * scene_abs + 2.0f * o + d);  // 8 * 2^-149
 }
 
@@ -77,15 +77,12 @@ __device__ __forceinline__ int tri_test32(const RayF &r, float3 v0, float3 v1, f
   const float A1x = ady * a2z + adz * a2y, A1y = adz * a2x + adx * a2z, A1z = adx * a2y + ady * a2x;
   const float A2x = aoy * a1z + aoz * a1y, A2y = aoz * a1x + aox * a1z, A2z = aox * a1y + aoy * a1x;
   const float D = fabsf(det);
-  float edet = kErr * (a1x * A1x + a1y * A1y + a1z * A1z) + 1e-15f * D;
-  float en1 = kErr * (aox * A1x + aoy * A1y + aoz * A1z) + 1e-15f * D;
-  float en2 = kErr * (adx * A2x + ady * A2y + adz * A2z) + 1e-15f * D;
-  float ent = kErr * (a2x * A2x + a2y * A2y + a2z * A2z);
+  const float rest = ROUNDED ? 1e-15f * D + under : 1e-15f * D;
+  const float edet = kErr * (a1x * A1x + a1y * A1y + a1z * A1z) + rest;
+  const float en1 = kErr * (aox * A1x + aoy * A1y + aoz * A1z) + rest;
+  const float en2 = kErr * (adx * A2x + ady * A2y + adz * A2z) + rest;
+  const float et0 = kErr * (a2x * A2x + a2y * A2y + a2z * A2z), ent = ROUNDED ? et0 + under : et0;
   if (ROUNDED) {
-    edet += under;
-    en1 += under;
-    en2 += under;
-    ent += under;
     // (beyond 1e37 the reciprocal would be subnormal; below 8 bounds of det,
     // 1 / det's own error would not be covered by t's bound)
     if (!(D > 8.0f * edet && D < 1e37f)) return kAmbiguous;
