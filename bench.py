@@ -174,8 +174,7 @@ def host_transfer_mode(ctx) -> str:
 def load_l2(kind: str, rays: int, seconds: float):
     """The L2 side of the roofline: L2 bytes per ray (lts__t_sectors of the
     committed ncu capture) at this run's rays per second, against the L2
-    peak of the same capture (its bytes over its duration over its
-    lts__throughput fraction)."""
+    peak of the same capture (sectors per cycle times its L2 clock)."""
     p = ROOT / "profiles" / "traffic.json"
     if not p.exists():
         return None
