@@ -346,13 +346,14 @@ __device__ __noinline__ ExactHit exact_hit(const float4 *__restrict__ tris, cons
 // Closest-hit results are skw_hit_d (the exact double t, prim, tri).
 //
 // What bounds it: the latency of the divergent walk (ncu, 1M closest hits:
-// 0.46 instructions issued per cycle and scheduler, 57 % of the stalls on node
-// loads, L1 at 74 % of its peak, DRAM at 3 %).  What the shape of the step is
+// 0.49 instructions issued per cycle and scheduler, 42 % of the stalls on node
+// loads, 11 of 32 lanes, L1 at 57 % of its peak, DRAM at 2 %).  What the shape of the step is
 // for, measured on 4,194,304 closest / 2,000,003 any hits over 1.1M triangles
 // (3.99 / 1.71 ms before): one place that pops, children loaded and tested
 // without branches, one 32-byte load per node and no spills in the step:
 // 3.47 / 1.33 ms.  200,001 double rays: 3.25 -> 0.53 ms with the float
-// decisions (87 % of the kernel was double triangle tests).
+// decisions (87 % of the kernel was double triangle tests), 0.55 with bounds that
+// hold at any scale.
 template <int CAP, bool CLOSEST, bool DRAY>
 __global__ void __launch_bounds__(SKW_TRAV_BLOCK, SKW_TRAV_MINB)
     k_trace(const float4 *__restrict__ nodes, const float4 *__restrict__ tris, const float4 *__restrict__ rays,
